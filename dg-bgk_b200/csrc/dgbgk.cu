@@ -1,8 +1,6 @@
 // C ABI of the DG-BGK sweep on B200 (sm_100a): handle management, device
 // memory, the captured two-step CUDA graph and the state transfers.
-#include <cuda.h>
 #include <cuda_runtime.h>
-#include <cudaTypedefs.h>
 
 #include <algorithm>
 #include <cmath>
@@ -55,18 +53,6 @@ template <class X> int upload(X** p, const std::vector<X>& v, cudaStream_t s) {
 template <class X> void dfree(X*& p) {
   if (p) cudaFree((void*)p);
   p = nullptr;
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  if (!fn) {
-    cudaDriverEntryPointQueryResult q;
-    void* p = nullptr;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-  }
-  return fn;
 }
 
 struct ImplBase {
@@ -166,6 +152,8 @@ template <class T, bool ONE> MomFn<T> mom_fn1(int R) {
   return R == 4 ? k_moments<T, 4, ONE> : R == 3 ? k_moments<T, 3, ONE> : R == 2 ? k_moments<T, 2, ONE> : k_moments<T, 1, ONE>;
 }
 template <class T> MomFn<T> mom_fn(int R, bool one) { return one ? mom_fn1<T, true>(R) : mom_fn1<T, false>(R); }
+// dynamic shared memory of a sweep CTA: 227 KB less its static arrays
+constexpr size_t SWEEP_SMEM_MAX = 227 * 1024 - 1024;
 template <class T> using SweepFn = void (*)(BatchArgs<T>, int, const CaseDev<T>);
 template <class T, bool ONE> SweepFn<T> sweep_fn1(int eb, int immat) {
   if (eb == 64) return immat == 1 ? k_sweep<T, 64, 1, ONE> : k_sweep<T, 64, 0, ONE>;
@@ -189,14 +177,18 @@ inline int allow_max_smem(const void* fn) {
   return 0;
 }
 
+// Tile buffers of the sweep: two where they fit, else (a wide halo) one.
+template <class T> int sweep_bufs(int eb, int max_halo) {
+  return SweepGeo<T>::smem(eb, max_halo, 2) <= SWEEP_SMEM_MAX ? 2 : 1;
+}
 // Resident sweep CTAs per SM for a tile shape (0: does not fit).
 template <class T> int sweep_per_sm(int eb, int immat, int max_halo, bool one) {
-  const size_t smem = SweepGeo<T>::smem(eb, max_halo);
-  if (smem > 227 * 1024) return 0;
+  const size_t smem = SweepGeo<T>::smem(eb, max_halo, sweep_bufs<T>(eb, max_halo));
+  if (smem > SWEEP_SMEM_MAX) return 0;
   SweepFn<T> fn = sweep_fn<T>(eb, immat, one);
   if (allow_max_smem((const void*)fn) != 0) return 0;
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, SweepGeo<T>::TPE * eb, smem) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, SweepGeo<T>::threads(eb), smem) !=
       cudaSuccess)
     return 0;
   return per_sm;
@@ -339,7 +331,8 @@ int build_launch_set(LaunchSet<T>& L, const std::vector<CaseDev<T>>& cs, int eb,
     set_error("sweep kernel does not fit on an SM with this tile");
     return DGBGK_EUNSUP;
   }
-  L.sweep_smem = SweepGeo<T>::smem(eb, max_halo);
+  L.args.sweep_bufs = sweep_bufs<T>(eb, max_halo);
+  L.sweep_smem = SweepGeo<T>::smem(eb, max_halo, L.args.sweep_bufs);
   L.sweep_grid = std::max(1, std::min(L.total_units, sps * nsm));
   return 0;
 }
@@ -390,10 +383,9 @@ int enqueue_step(const LaunchSet<T>& L, cudaStream_t st, float* ms = nullptr, co
     TRY(launch_check("k_wall", L.total_walls, WALL_THREADS, 0));
   }
   if (ms) cudaEventRecord(ev[2], st);
-  constexpr int TPE = SweepGeo<T>::TPE;
-  sweep_fn<T>(L.eb, L.immat, L.one)<<<L.sweep_grid, TPE * L.eb, L.sweep_smem, st>>>(L.args, L.total_units,
-                                                                                     L.one_case);
-  TRY(launch_check("k_sweep", L.sweep_grid, TPE * L.eb, L.sweep_smem));
+  const int snt = SweepGeo<T>::threads(L.eb);
+  sweep_fn<T>(L.eb, L.immat, L.one)<<<L.sweep_grid, snt, L.sweep_smem, st>>>(L.args, L.total_units, L.one_case);
+  TRY(launch_check("k_sweep", L.sweep_grid, snt, L.sweep_smem));
   // the specular part of ALPHA < 1 wall sides: the parallel items, then the
   // ones that wait on earlier deferred velocities
   for (const auto& c : L.spec_cases) {
@@ -573,10 +565,10 @@ template <class T> struct Impl : ImplBase {
   }
 
   int nvt() const { return (pl.V + SweepGeo<T>::VT - 1) / SweepGeo<T>::VT; }
-  // measured on B200 (channel 200x100, 24x48 velocities): FP32 sweep 0.414 ms
-  // at 128 elements per tile, 0.50 at 64; FP64 1.24 ms at 128 (one CTA of
-  // 8 warps per SM), 1.02 at 64 (three CTAs of 4 warps)
-  static int default_eb() { return sizeof(T) == 8 ? 64 : 128; }
+  // measured on B200: FP32 sweep of the 200x100 channel at 24x48 velocities
+  // 0.304 ms with 64 elements (two CTAs of 8 warps per SM), 0.312 with 128
+  // (one of 16); FP64 0.805 with 64, 0.770 with 128
+  static int default_eb() { return sizeof(T) == 8 ? 128 : 64; }
 
   int init(int tile_elems) {
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
@@ -658,31 +650,7 @@ template <class T> struct Impl : ImplBase {
     return 0;
   }
 
-  // f[b] as a [3E rows][Vp] tensor; box = one 64-byte velocity segment of
-  // BOX_ROWS rows, 64-byte swizzle (the sweep's tile layout)
-  int make_tensor_maps() {
-    auto enc = tensor_map_encoder();
-    if (!enc) {
-      set_error("cuTensorMapEncodeTiled is not available from the driver");
-      return DGBGK_ECUDA;
-    }
-    const CUtensorMapDataType dt = sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    cuuint64_t dims[2] = {(cuuint64_t)Vp, (cuuint64_t)3 * pl.E};
-    cuuint64_t strides[1] = {(cuuint64_t)Vp * sizeof(T)};
-    cuuint32_t box[2] = {(cuuint32_t)SweepGeo<T>::VT, (cuuint32_t)SweepGeo<T>::BOX_ROWS};
-    cuuint32_t estr[2] = {1, 1};
-    for (int b = 0; b < 2; ++b) {
-      CUresult r = enc(&hc.tm[b], dt, 2, f[b], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                       CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS) {
-        set_error("cuTensorMapEncodeTiled failed for the state buffer");
-        return DGBGK_ECUDA;
-      }
-    }
-    return 0;
-  }
-
-  // this case's table entry (the tensor maps are set by make_tensor_maps)
+  // this case's table entry
   void fill_case() {
     hc.f[0] = f[0];
     hc.f[1] = f[1];
@@ -751,13 +719,19 @@ template <class T> struct Impl : ImplBase {
   // Sweep tile: EB elements per CTA (TPE*EB threads) x one 64-byte velocity
   // segment; `upc` work units per resident CTA picks the tiles per unit.
   int set_tile(int tile_elems, int upc) {
-    const int eb = tile_elems > 0 ? tile_elems : default_eb();
+    int eb = tile_elems > 0 ? tile_elems : default_eb();
     if (eb != 64 && eb != 128) {
       set_error("tile_elems must be 64 or 128");
       return DGBGK_EINVAL;
     }
     if (pl.EB != eb || halo_off == nullptr) {
       build_blocks(pl, eb);
+      if (eb == 128 && SweepGeo<T>::smem(eb, pl.max_halo, 1) > SWEEP_SMEM_MAX) {
+        // a halo too wide for this tile (an element order without locality):
+        // 64 elements have at most 192 neighbours, which fit
+        eb = 64;
+        build_blocks(pl, eb);
+      }
       dfree(halo_off);
       dfree(halo_list);
       dfree(rec);
@@ -769,42 +743,35 @@ template <class T> struct Impl : ImplBase {
       std::memset((void*)r.data(), 0, r.size() * sizeof(ElemRec<T>));
       for (int e = 0; e < pl.E; ++e) {
         const auto& g = pl.geo[e];
-        int flags = g.inflow & 7, interior = 0;
+        int flags = g.inflow & 7;
         for (int k = 0; k < 3; ++k) {
-          r[e].gx[k] = (T)g.gx[k];
-          r[e].gy[k] = (T)g.gy[k];
-          r[e].mm[k] = (T)g.mm[k];
+          coef_set(r[e].gx[k], g.gx[k]);
+          coef_set(r[e].gy[k], g.gy[k]);
+          coef_set(r[e].mm[k], g.mm[k]);
           const size_t i = 3 * (size_t)e + k;
           const PlanEdge& pe = pl.edge[i];
-          r[e].edge[k].anx = (T)(pe.alen * pe.nx);
-          r[e].edge[k].any = (T)(pe.alen * pe.ny);
           // the flux source's rows: the neighbour's (its slot and local
           // nodes) across an interior side, the element's own otherwise
           const int inf = edge_info(pl, i, e % eb);
           const int slot = inf >> 8, kind = inf & 3;
-          r[e].edge[k].offp = tile_row_off(3 * slot + ((inf >> 3) & 3));
-          r[e].edge[k].offq = tile_row_off(3 * slot + ((inf >> 5) & 3));
-          if (kind == 0 || kind == 2) flags |= FLAG_FLUX0 << k;
-          if (kind == 0) ++interior;
-          const bool wall = kind == 3;
-          r[e].bside[k] = wall ? pe.bside : -1;
-          if (wall) flags |= 8 << k;
+          const bool zero = kind == 1 || kind == 3;
+          coef_set(r[e].en[k][0], -(pe.alen * pe.nx));
+          coef_set(r[e].en[k][1], -(pe.alen * pe.ny));
+          r[e].off[k][0] = zero ? 0 : tile_row(3 * slot + ((inf >> 3) & 3));
+          r[e].off[k][1] = zero ? 0 : tile_row(3 * slot + ((inf >> 5) & 3));
+          r[e].bside[k] = kind == 3 ? pe.bside : -1;
+          if (kind == 3) flags |= 8 << k;
+          if (kind == 1) flags |= FLAG_INFLOW_EDGE0 << k;
         }
-        if (interior == 3) flags |= FLAG_INTERIOR;
-        const int j = e % eb;
-        r[e].own01 = tile_row_off(3 * j) | (tile_row_off(3 * j + 1) << 16);
-        r[e].own2 = tile_row_off(3 * j + 2);
-        r[e].area = (T)g.area;
         r[e].flags = flags;
         r[e].wslot = pl.spec ? pl.wslot[e] : -1;
       }
       TRY(upload(&rec, r, st));
     }
-    if (SweepGeo<T>::smem(pl.EB, pl.max_halo) > 227 * 1024) {
+    if (SweepGeo<T>::smem(pl.EB, pl.max_halo, 1) > SWEEP_SMEM_MAX) {
       set_error("sweep tile needs more than 227 KB of shared memory");
       return DGBGK_EUNSUP;
     }
-    TRY(make_tensor_maps());
     const int sps = sweep_per_sm<T>(pl.EB, pl.immat, pl.max_halo, true);
     if (sps < 1) {
       set_error("sweep kernel does not fit on an SM with this tile");
@@ -919,9 +886,9 @@ template <class T> struct Impl : ImplBase {
     } else if (k == 3) {
       const int nt = std::max(n3, (int)pl.walls.size());
       k_shard_fin<T><<<(nt + 255) / 256, 256, 0, st>>>(C, sums1, sums2);
-      constexpr int TPE = SweepGeo<T>::TPE;
-      sweep_fn<T>(single.eb, single.immat, true)<<<single.sweep_grid, TPE * single.eb, single.sweep_smem, st>>>(
-          single.args, single.total_units, single.one_case);
+      sweep_fn<T>(single.eb, single.immat, true)<<<single.sweep_grid, SweepGeo<T>::threads(single.eb),
+                                                   single.sweep_smem, st>>>(single.args, single.total_units,
+                                                                            single.one_case);
       k_shard_respart<T><<<1, 32, 0, st>>>(C, res);
     } else if (k == 4) {
       k_shard_resid<T><<<1, 32, 0, st>>>(C, res, single.args.ctl);
@@ -1783,6 +1750,8 @@ template <class T> struct BatchImpl : BatchBase {
     for (auto* c : cs) {
       TRY(c->set_tile(e, u));
       CK(cudaStreamSynchronize(c->st));
+      // a case whose halo does not fit a 128-element tile: 64 for all
+      if (c->pl.EB != e) return configure(c->pl.EB, u);
     }
     max_halo = 0;
     long tiles = 0;

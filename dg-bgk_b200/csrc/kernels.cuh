@@ -13,19 +13,17 @@
 //   k_sweep   : the whole velocity-loop body (GTEQNF, GETFLA, GETELC,
 //               EDGFLXOPT/GETBOU, GETINC/CMMINC, ADTHEM, INFLOW;
 //               src/advnce.f90:286-377) on tiles of (element block x one
-//               64-byte velocity segment).  Persistent CTAs draw work units
+//               128-byte velocity segment).  Persistent CTAs draw work units
 //               (a block at several tiles); the block's records are staged
-//               once per unit, the tiles' f rows arrive double-buffered (the
-//               block's as 2-D TMA boxes, the halo's by cp.async), and each
-//               thread works on whole elements at 8 (FP32) or 4 (FP64)
-//               velocities.
+//               once per unit, the tiles' f rows arrive by cp.async,
+//               double-buffered, and eight lanes share an element, each at 4
+//               (FP32, packed pairs) or 2 (FP64) velocities.
 //   k_resid   : GETRES + the residual bookkeeping (src/advnce.f90:385,
 //               422-429), the convergence test and the step counter.
 // Every device-side wait on an mbarrier is bounded: on expiry the kernel
 // sets Ctrl::timeout, drains its own copies with a second bounded wait and
 // returns; the host reports DGBGK_ECUDA.
 #pragma once
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -118,7 +116,6 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 // a batch a table of many.  The work of the launch set is flattened: sweep
 // units, moment row groups and wall sides of case c are [off[c], off[c+1]).
 template <class T> struct alignas(64) CaseDev {
-  CUtensorMap tm[2];  // f[b] as [3E rows][Vp] (sweep tile boxes, 64-byte swizzle)
   T* f[2];            // state, ping-pong; Ctrl::cur is the current one
   ElemRec<T>* rec;
   const int* halo_off;
@@ -210,6 +207,7 @@ template <class T> struct BatchArgs {
   BatchCtl* ctl;
   int ncases;
   int max_halo;             // over the cases (sweep tile layout)
+  int sweep_bufs;           // sweep tile buffers, 2 or (a wide halo) 1
   int mom_stages;           // moment ring stages per warp
   unsigned mom_rowbytes;    // moment ring row size (max over the cases)
 };
@@ -507,23 +505,24 @@ __device__ __forceinline__ double node_epilogue(const CaseDev<T>& C, int node, d
     const double b2 = rho / (2 * ps);
     const double a = nd * (b2 / PI_D);
     if (sizeof(T) == 4) {
-      en.A[i] = (T)a;
-      en.ex[i] = (T)(-b2 * LOG2E_D);
-      en.ux[i] = (T)ux;
-      en.uy[i] = (T)uy;
+      coef_set(en.A[i], a);
+      coef_set(en.ex[i], -b2 * LOG2E_D);
+      coef_set(en.ux[i], -ux);
+      coef_set(en.uy[i], -uy);
     } else {
-      en.A[i] = (T)(log(a) - b2 * (ux * ux + uy * uy));
-      en.ex[i] = (T)(-b2);
-      en.ux[i] = (T)(2.0 * b2 * ux);
-      en.uy[i] = (T)(2.0 * b2 * uy);
+      coef_set(en.A[i], log(a) - b2 * (ux * ux + uy * uy));
+      coef_set(en.ex[i], -b2);
+      coef_set(en.ux[i], 2.0 * b2 * ux);
+      coef_set(en.uy[i], 2.0 * b2 * uy);
     }
   } else {
-    en.A[i] = (T)(sizeof(T) == 4 ? 0.0 : -INFINITY);
-    en.ex[i] = (T)0;
-    en.ux[i] = (T)(sizeof(T) == 4 ? ux : 0.0);
-    en.uy[i] = (T)(sizeof(T) == 4 ? uy : 0.0);
+    coef_set(en.A[i], sizeof(T) == 4 ? 0.0 : -INFINITY);
+    coef_set(en.ex[i], 0.0);
+    coef_set(en.ux[i], sizeof(T) == 4 ? -ux : 0.0);
+    coef_set(en.uy[i], sizeof(T) == 4 ? -uy : 0.0);
   }
-  en.mu[i] = (T)mu;
+  coef_set(en.mu[i], mu);
+  coef_set(en.mt[i], mu);
   C.nraw[node] = s0;
   C.disux[node] = ux;
   C.disuy[node] = uy;
@@ -748,86 +747,69 @@ __device__ __forceinline__ double step_dt(const Ctrl* c) {
   return fmin(dtb, c->dtc);
 }
 
-// Sweep tile geometry.  A tile is one 64-byte segment of velocities (16 FP32
-// or 8 FP64 values) of the three rows of every element of a block and of its
-// halo: row r = 3*slot + i (block element j: slot j; halo element h: slot
-// EB + h), 64 bytes per row, with the 16-byte chunks of a row permuted by the
-// 64-byte swizzle (chunk c of row r at 16*(c ^ ((r >> 1) & 3))).  The block's
-// rows arrive as 2-D TMA boxes that apply this swizzle, the halo rows by
-// cp.async copies that apply it by hand; with it, eight threads that each
-// read their own element's row with 16-byte vectors fall on eight distinct
-// bank groups.  A work unit is one block at `tpu` consecutive velocity
-// tiles: the block's element records and the halo's record heads are staged
-// in shared memory once per unit, the f rows once per tile (double-buffered).
+// Sweep geometry.  LPE = 8 lanes share an element, each with one 16-byte
+// vector of velocities (4 FP32 or 2 FP64), so a warp works on EPW = 4
+// elements at 32 (16) velocities and every row access -- global or shared --
+// is a whole 128-byte line.  A tile is one such velocity segment of an
+// element block and its halo: the rows of g = f - UMEAN, 128 bytes each, row
+// r = 3*slot + i (block element j: slot j; halo element h: slot EB + h) at
+// byte 128*r.  Eight lanes read a row through all 32 banks, so neither the
+// own rows nor the neighbours' rows conflict.  A work unit is one block at
+// consecutive velocity tiles: its element records, the halo's record heads
+// and the halo list are staged in shared memory once per unit.
 template <class T> struct SweepGeo {
-  static constexpr int W = 16 / (int)sizeof(T);  // values per 16-byte vector
-  static constexpr int VT = 64 / (int)sizeof(T);  // velocities per tile
-  static constexpr int NCH = 4;                   // 16-byte chunks per row segment
-  // threads per block element in the sweep, each taking NCH / TPE chunks.
-  // Two for both precisions: on the Mach 2 channel (200x100, 24x48) four
-  // threads per element made the FP32 sweep 0.42 -> 0.55 ms, and the FP64
-  // sweep (16 warps per SM but 128 registers, spilling) slower than two
-  // threads at 8 warps and 226 registers without spills
-#ifndef DGBGK_SWEEP_TPE32
-#define DGBGK_SWEEP_TPE32 2
+  static constexpr int W = 16 / (int)sizeof(T);  // velocities per lane
+  static constexpr int NP = W / 2 < 1 ? 1 : W / 2;  // pairs per lane
+  static constexpr int LPE = 8;                  // lanes per element
+  static constexpr int VT = W * LPE;             // velocities per tile
+  static constexpr int EPW = 32 / LPE;           // elements of a warp at a time
+#ifndef DGBGK_IT32_64
+#define DGBGK_IT32_64 2
 #endif
-#ifndef DGBGK_SWEEP_TPE64
-#define DGBGK_SWEEP_TPE64 2
+#ifndef DGBGK_IT32_128
+#define DGBGK_IT32_128 2
 #endif
-  static constexpr int TPE = sizeof(T) == 4 ? DGBGK_SWEEP_TPE32 : DGBGK_SWEEP_TPE64;
-  static constexpr int CPT = NCH / TPE;           // chunks per thread
-  static_assert(TPE == 2 || TPE == 4, "two or four threads per element");
-  static constexpr int BOX_ROWS = 192;            // rows of one TMA box
-  static constexpr int RW = (int)(sizeof(ElemRec<T>) / 16);                    // record words
-  static constexpr int HW = (REC_HEAD_VALUES * (int)sizeof(T) + 15) / 16;        // head words
-  static constexpr int HR = 16 * (HW | 1);  // halo head pitch (odd number of words)
-  static constexpr int TPU_MAX = 16;
-  // velocity tables staged per unit: cx, cy, NFINF (and |c|^2 for the FP64
-  // exponent)
-  static constexpr int NTAB = sizeof(T) == 8 ? 4 : 3;
-  // one tile buffer, 1024-byte aligned
-  static constexpr size_t tile_bytes(int EB, int max_halo) {
-    return ((size_t)3 * (EB + max_halo) * 64 + 1023) / 1024 * 1024;
+#ifndef DGBGK_IT64_64
+#define DGBGK_IT64_64 2
+#endif
+#ifndef DGBGK_IT64_128
+#define DGBGK_IT64_128 2
+#endif
+#ifndef DGBGK_SWEEP_REGS32
+#define DGBGK_SWEEP_REGS32 128
+#endif
+#ifndef DGBGK_SWEEP_REGS64
+#define DGBGK_SWEEP_REGS64 128
+#endif
+  // block elements per lane group: their NFO and UMEAN stay in registers
+  // between the phases (16 registers an element)
+  static constexpr int iters(int EB) {
+    return sizeof(T) == 4 ? (EB == 64 ? DGBGK_IT32_64 : DGBGK_IT32_128) : (EB == 64 ? DGBGK_IT64_64 : DGBGK_IT64_128);
   }
-  // alignment slack, two tiles, records [EB], halo heads [max_halo][HR],
-  // velocity tables [NTAB][TPU_MAX * VT], halo row list [3 * max_halo]
-  static constexpr size_t smem(int EB, int max_halo) {
-    return 1024 + 2 * tile_bytes(EB, max_halo) + (size_t)EB * sizeof(ElemRec<T>) + (size_t)max_halo * HR +
-           NTAB * (size_t)TPU_MAX * VT * sizeof(T) + ((size_t)3 * max_halo * 4 + 15) / 16 * 16;
+  static constexpr int threads(int EB) { return EB / (EPW * iters(EB)) * 32; }
+  // resident CTAs per SM the register budget is set for
+  static constexpr int min_ctas(int EB) {
+    const int c = 65536 / ((sizeof(T) == 4 ? DGBGK_SWEEP_REGS32 : DGBGK_SWEEP_REGS64) * threads(EB));
+    return c < 1 ? 1 : c;
+  }
+  static constexpr int RW = (int)(sizeof(ElemRec<T>) / 16);                // record words
+  static constexpr int HW = (REC_HEAD_VALUES * (int)sizeof(typename CoefOf<T>::type) + 15) / 16;  // head words
+  // pitches in shared memory: odd numbers of 16-byte words, so that the four
+  // records a warp reads at once fall on different banks
+  static constexpr int RP = 16 * (RW | 1), HR = 16 * (HW | 1);
+  static constexpr int TPU_MAX = 16;
+  // rows of swtab: cx, cy, NFINF (and |c|^2 for the FP64 exponent)
+  static constexpr int NTAB = sizeof(T) == 8 ? 4 : 3;
+  static constexpr unsigned tile_bytes(int EB, int max_halo) { return tile_row(3 * (EB + max_halo)); }
+  // velocity tables staged per unit: cx, cy (and |c|^2 for the FP64 exponent)
+  static constexpr int NVT = sizeof(T) == 8 ? 3 : 2;
+  // `bufs` tiles, records [EB], halo heads [max_halo], velocity tables
+  // [NVT][TPU_MAX * VT], halo list [max_halo]
+  static constexpr size_t smem(int EB, int max_halo, int bufs) {
+    return (size_t)bufs * tile_bytes(EB, max_halo) + (size_t)EB * RP + (size_t)max_halo * HR +
+           (size_t)NVT * TPU_MAX * ROW_BYTES + ((size_t)max_halo * 4 + 15) / 16 * 16;
   }
 };
-
-
-// A tensor map read from global memory (the batch's case table, written by
-// a host copy) must be acquired by the tensormap proxy before a thread uses
-// it; one fence per map and thread.  Maps passed as __grid_constant__
-// parameters need none.
-__device__ __forceinline__ void tensormap_acquire(const CUtensorMap* p) {
-  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(p) : "memory");
-}
-
-// 2-D tiled TMA load (no multicast) of one box into shared memory.
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
-          "r"(smem_u32(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
-// 2-D tiled TMA store of one box from shared memory (elements outside the
-// tensor are not written), tracked by the issuing thread's bulk groups.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, const void* src) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x),
-               "r"(y), "r"(smem_u32(src))
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// the issuing thread's bulk stores have finished reading shared memory
-__device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// ... all but the most recent one
-__device__ __forceinline__ void bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
-// ... and their writes are complete
-__device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // 16-byte asynchronous copy global -> shared through L2 only (cp.async.cg).
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -852,85 +834,118 @@ template <> __device__ __forceinline__ float nfo_exp<float>(float x, const doubl
   return p;
 }
 
-template <class T> struct Vec;
-template <> struct Vec<float> {
-  using type = float4;
-  static __device__ __forceinline__ float get(const float4& v, int k) {
-    return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
-  }
-  static __device__ __forceinline__ void set(float4& v, int k, float x) {
-    if (k == 0)
-      v.x = x;
-    else if (k == 1)
-      v.y = x;
-    else if (k == 2)
-      v.z = x;
-    else
-      v.w = x;
-  }
-};
-template <> struct Vec<double> {
-  using type = double2;
-  static __device__ __forceinline__ double get(const double2& v, int k) { return k == 0 ? v.x : v.y; }
-  static __device__ __forceinline__ void set(double2& v, int k, double x) {
-    if (k == 0)
-      v.x = x;
-    else
-      v.y = x;
-  }
-};
-template <class T> __device__ __forceinline__ typename Vec<T>::type vld(const void* p) {
-  return *reinterpret_cast<const typename Vec<T>::type*>(p);
+// Pairs of velocities: FP32 on packed instructions (one issue slot for two
+// values, each rounded as the scalar instruction would), FP64 scalar.
+template <class T> struct Pair;
+template <> struct Pair<float> { using type = float2; using vec = float4; };
+template <> struct Pair<double> { using type = double2; using vec = double2; };
+__device__ __forceinline__ float2 padd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 pmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 pdup(float a) { return make_float2(a, a); }
+__device__ __forceinline__ double2 padd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 pmul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ double2 pfma(double2 a, double2 b, double2 c) {
+  return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
 }
-template <class T> __device__ __forceinline__ void vst(void* p, const typename Vec<T>::type& v) {
-  *reinterpret_cast<typename Vec<T>::type*>(p) = v;
+__device__ __forceinline__ double2 pdup(double a) { return make_double2(a, a); }
+template <class P> __device__ __forceinline__ P pneg(P a) {
+  a.x = -a.x;
+  a.y = -a.y;
+  return a;
 }
+// a - b; FP32 as one packed fma(b, -1, a), the same rounding (negating a
+// packed operand takes two instructions)
+__device__ __forceinline__ float2 psub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ double2 psub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+// a record's coefficient as a pair and as a value
+__device__ __forceinline__ float2 pdup(const CoefF& c) { return make_float2(c.x, c.y); }
+__device__ __forceinline__ float pval(const CoefF& c) { return c.x; }
+__device__ __forceinline__ double pval(double c) { return c; }
+// the pairs of a 16-byte vector
+__device__ __forceinline__ float2 pget(const float4& v, int h) { return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y); }
+__device__ __forceinline__ double2 pget(const double2& v, int) { return v; }
+__device__ __forceinline__ void pset(float4& v, int h, float2 p) {
+  if (h) {
+    v.z = p.x;
+    v.w = p.y;
+  } else {
+    v.x = p.x;
+    v.y = p.y;
+  }
+}
+__device__ __forceinline__ void pset(double2& v, int, double2 p) { v = p; }
 
-// Phase 1 of the sweep on one 16-byte chunk of an element's three rows
-// (tile byte offsets ro[0..2]): NFO (GTEQNF, src/gteqnf.f90:35-37) and
-// UMEAN = 0.5*DTE*(div F - 1/3 sum_i MU_i (NFO_i - f_i)) with div F = sum_i
-// (N_i,x cx + N_i,y cy) f_i (GETELC, src/getelc.f90:54-83).  The rows are
-// overwritten in place with g = f - UMEAN, the value every edge flux and the
-// volume term of this element use (src/getelc.f90:87-117,
-// src/edgflxopt.f90:95-125); NFO and UMEAN are returned.  FP32: NFO =
+template <class T> __device__ __forceinline__ typename Pair<T>::vec vld(const void* p) {
+  return *reinterpret_cast<const typename Pair<T>::vec*>(p);
+}
+template <class T> __device__ __forceinline__ void vst(void* p, const typename Pair<T>::vec& v) {
+  *reinterpret_cast<typename Pair<T>::vec*>(p) = v;
+}
+// Phase 1 of the sweep on one lane's velocities of an element's three rows:
+// NFO (GTEQNF, src/gteqnf.f90:35-37) and UMEAN = 0.5*DTE*(div F -
+// 1/3 sum_i MU_i (NFO_i - f_i)) with div F = sum_i (N_i,x cx + N_i,y cy) f_i
+// (GETELC, src/getelc.f90:54-83); g = f - UMEAN, the value every edge flux
+// and the volume term of this element use (src/getelc.f90:87-117,
+// src/edgflxopt.f90:95-125), replaces f.  The staged record carries the
+// gradients times 0.5*DTE and MU times -DTE/6 (sweep_scale).  FP32: NFO =
 // A*2^(ex*|c-u|^2) with the SFU's 2^x; FP64: NFO = exp(a0 + a1*cx + a2*cy +
 // ex*|c|^2) (the exponent expanded, three FMAs; c2 = |c|^2 per velocity).
 template <class T>
-__device__ __forceinline__ void sweep_p1(const ElemRec<T>& r, const double* etab, unsigned char* tl,
-                                         const unsigned (&ro)[3], const typename Vec<T>::type& cxv,
-                                         const typename Vec<T>::type& cyv, const typename Vec<T>::type& c2v, T dth,
-                                         T dth3, typename Vec<T>::type (&q)[3], typename Vec<T>::type& u) {
-  using VO = Vec<T>;
-  constexpr int W = SweepGeo<T>::W;
-  typename VO::type f[3];
+__device__ __forceinline__ void sweep_p1(const ElemRec<T>& r, const double* etab, unsigned char* rows,
+                                         const typename Pair<T>::vec& cxv, const typename Pair<T>::vec& cyv,
+                                         const typename Pair<T>::vec& c2v, typename Pair<T>::vec (&q)[3],
+                                         typename Pair<T>::vec& u) {
+  using P = typename Pair<T>::type;
+  typename Pair<T>::vec f[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i) f[i] = vld<T>(tl + ro[i]);
+  for (int i = 0; i < 3; ++i) f[i] = vld<T>(rows + i * ROW_BYTES);
 #pragma unroll
-  for (int w = 0; w < W; ++w) {
-    const T cx = VO::get(cxv, w), cy = VO::get(cyv, w);
-    const T f0 = VO::get(f[0], w), f1 = VO::get(f[1], w), f2 = VO::get(f[2], w);
-    const T sx = r.gx[0] * f0 + r.gx[1] * f1 + r.gx[2] * f2;
-    const T sy = r.gy[0] * f0 + r.gy[1] * f1 + r.gy[2] * f2;
-    T coll = (T)0;
+  for (int h = 0; h < SweepGeo<T>::NP; ++h) {
+    const P cx = pget(cxv, h), cy = pget(cyv, h);
+    P fi[3], um;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) fi[i] = pget(f[i], h);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      T qi;
+      P qi;
       if constexpr (sizeof(T) == 8) {
-        qi = exp_tang(fma(r.ux[i], cx, fma(r.uy[i], cy, fma(r.ex[i], VO::get(c2v, w), r.A[i]))), etab);
+        const P x = pfma(pdup(r.ux[i]), cx, pfma(pdup(r.uy[i]), cy, pfma(pdup(r.ex[i]), pget(c2v, h), pdup(r.A[i]))));
+        qi.x = nfo_exp<T>(x.x, etab);
+        qi.y = nfo_exp<T>(x.y, etab);
       } else {
-        const T dx = r.ux[i] - cx, dy = r.uy[i] - cy;
-        qi = r.A[i] * nfo_exp<T>(r.ex[i] * (dx * dx + dy * dy), etab);
+        const P dx = padd(cx, pdup(r.ux[i])), dy = padd(cy, pdup(r.uy[i]));
+        const P x = pmul(pdup(r.ex[i]), pfma(dx, dx, pmul(dy, dy)));
+        qi.x = nfo_exp<T>(x.x, etab);
+        qi.y = nfo_exp<T>(x.y, etab);
+        qi = pmul(pdup(r.A[i]), qi);
       }
-      VO::set(q[i], w, qi);
-      coll += r.mu[i] * (qi - VO::get(f[i], w));
+      pset(q[i], h, qi);
+      const P t = psub(qi, fi[i]);
+      um = i == 0 ? pmul(pdup(r.mu[0]), t) : pfma(pdup(r.mu[i]), t, um);
     }
-    const T um = dth * (sx * cx + sy * cy) - dth3 * coll;
-    VO::set(u, w, um);
+    const P sx = pfma(pdup(r.gx[2]), fi[2], pfma(pdup(r.gx[1]), fi[1], pmul(pdup(r.gx[0]), fi[0])));
+    const P sy = pfma(pdup(r.gy[2]), fi[2], pfma(pdup(r.gy[1]), fi[1], pmul(pdup(r.gy[0]), fi[0])));
+    um = pfma(sx, cx, pfma(sy, cy, um));
+    pset(u, h, um);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) VO::set(f[i], w, VO::get(f[i], w) - um);
+    for (int i = 0; i < 3; ++i) pset(f[i], h, psub(fi[i], um));
   }
 #pragma unroll
-  for (int i = 0; i < 3; ++i) vst<T>(tl + ro[i], f[i]);
+  for (int i = 0; i < 3; ++i) vst<T>(rows + i * ROW_BYTES, f[i]);
+}
+
+// The step's factors of a staged record, applied to its 16-byte word k (two
+// coefficients) by the thread that copied it: 0.5*DTE to the gradients
+// (words 0 to 2), -DTE/6 to MU (words 9, 10), DTE to MT and MM (words 11 to
+// 13); the other words are left alone.
+template <class T> __device__ __forceinline__ void sweep_scale(unsigned char* word, int k, T dth, T mdt6, T dt) {
+  if (k > 13 || (k > 2 && k < 9)) return;
+  const T s = k < 3 ? dth : k < 11 ? mdt6 : dt;
+  typename Pair<T>::vec v = vld<T>(word);
+#pragma unroll
+  for (int h = 0; h < SweepGeo<T>::NP; ++h) pset(v, h, pmul(pget(v, h), pdup(s)));
+  vst<T>(word, v);
 }
 
 // max that keeps a NaN operand (max.NaN): the residual's "change the
@@ -957,50 +972,59 @@ __device__ __forceinline__ void resid_add(Ctrl* ctrl, const double* red_m, const
   atomicMax(reinterpret_cast<unsigned long long*>(&ctrl->acc_max), (unsigned long long)__double_as_longlong(mm));
 }
 
-// Persistent sweep kernel: EB block elements, TPE*EB threads.  Work units are
-// (block b, group of `tpu` velocity tiles) with b fastest, handed out in
-// order (the first by blockIdx, the rest from a device counter), so the CTAs
-// running at one moment cover neighbouring blocks at the same velocities and
-// the halo rows they read are L2 hits.  Per unit the block's element records
-// and the halo's record heads are staged in shared memory; per tile the
-// block's rows arrive as TMA boxes (completing on an mbarrier, bounded wait)
-// and the halo's rows by cp.async copies, double-buffered so the next tile's
-// rows load while this one is computed.  Per tile:
-//  * phase 1: UMEAN and g = f - UMEAN of every block and halo element; a
-//    block element's NFO and UMEAN stay in the registers of the thread that
-//    updates it;
-//  * phase 2, threads j, j+EB, .. (TPE of them) take NCH/TPE of block
-//    element j's 16-byte velocity chunks each: the volume term (src/getelc.f90:87-117), the edge fluxes gathered
-//    per element (EDGFLXOPT src/edgflxopt.f90:95-125; outflow and, with zero
-//    length, inflow and wall sides read the element itself), the wall sides'
-//    fluxes (GETBOU src/getbou.f90:142-281), GETINC/CMMINC, ADTHEM and INFLOW;
-//    the new rows stay in registers.
-// Two barriers per tile: at the top (tile k has landed; every thread is
-// done with tile k - 1, whose new rows it then writes back into that tile's
-// buffer) and after phase 1; after the second, thread 0 stores tile k - 1
-// and the next tile's copies go into its buffer once the store has read it.
-// The unit's last tile is written back and stored at the unit's end.
+// Persistent sweep kernel.  Work units are (block b, group of `tpu` velocity
+// tiles) with b fastest, handed out in order (the first by blockIdx, the
+// rest from a device counter), so the CTAs running at one moment cover
+// neighbouring blocks at the same velocities and the halo rows they read are
+// L2 hits.  Per unit the block's element records, the halo's record heads and
+// the unit's velocities are staged in shared memory; per tile
+//  * the rows of every block and halo element are copied to the tile by the
+//    lanes that will work on them (cp.async, a tile ahead: they wait for
+//    their own copies only);
+//  * phase 1: UMEAN and g = f - UMEAN, which replaces f in the tile; a block
+//    element's NFO and UMEAN stay in the registers of the lanes that update
+//    it;
+//  * phase 2, the same lanes update the element: the volume term
+//    (src/getelc.f90:87-117) and the edge fluxes gathered per element from
+//    the tile (EDGFLXOPT src/edgflxopt.f90:95-125; an outflow side reads the
+//    element itself), the wall sides' fluxes (GETBOU
+//    src/getbou.f90:142-281), GETINC/CMMINC, ADTHEM and INFLOW; the new rows
+//    go to global memory as whole lines.
+// With two tile buffers one barrier per tile is enough (between its phases:
+// a warp past it has left the previous tile, whose buffer the copies of the
+// next one overwrite); a mesh whose halo leaves room for one buffer only
+// takes a second barrier after phase 2.
 // ONE: a single case passed as a kernel parameter (its fields come from the
 // constant bank, no registers); otherwise the case table.
 // Upwinding: the own value is taken where SC = n.c > 0.  The reference takes
 // it where SC > 0 for the ISIDE(3) element and SC >= 0 for the other; the
 // two differ only at SC = 0, where the flux SC*value is zero either way.
-// Residency: FP32, two CTAs per SM (128 registers); FP64 with 64-element
-// blocks, three CTAs of 4 warps (168 registers, a few spilled: 1.02 ms per
-// sweep on the 200x100 channel at 24x48 velocities, against 1.24 ms for one
-// 8-warp CTA of 128 elements at 208 registers).
+//
+// Why this mapping.  FP32 issues 486 warp instructions per 128 (element,
+// velocity) pairs, halo included; two lanes per element at 8 velocities each,
+// 64-byte swizzled rows and scalar arithmetic took 760.  What went: half of
+// the FMA-pipe issue slots (packed pairs), the duplication of coefficients
+// (the records hold them as pairs) and the swizzle's index arithmetic, the
+// staging of the new rows through the tile, and the neighbour gather's bank
+// conflicts (2.0e7 -> 0.3e7 per launch).  200x100 channel, 24x48 velocities
+// (1.375e8 DOFs): FP32 0.394 -> 0.304 ms, FP64 0.945 -> 0.770.  Bound (FP32,
+// ncu): latency at 16 warps per SM (128 registers), issue active 0.52, stalls
+// per issue wait 1.2, short-scoreboard and barrier 0.9 each, math-pipe 0.9;
+// FMA pipe 0.41 and shared-memory wavefronts 0.62 of their peaks.  Measured
+// and not kept: one element per lane group and 16 warps per 64 elements
+// (FP32 0.372, FP64 0.817), four per group in FP64 (1.04), FP64 at 168
+// registers (0.840), coefficients duplicated in registers (0.387), f loaded
+// straight into registers at the start of phase 1 (0.387).
 template <class T, int EB, int IMMAT, bool ONE>
-__global__ void __launch_bounds__(SweepGeo<T>::TPE * EB, sizeof(T) == 4 ? 2 : (EB == 64 ? 3 : 1))
+__global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_ctas(EB))
     k_sweep(BatchArgs<T> a, int total_units, const __grid_constant__ CaseDev<T> one) {
   using G = SweepGeo<T>;
-  using VO = Vec<T>;
-  using VecT = typename VO::type;
-  constexpr int W = G::W, VT = G::VT, NCH = G::NCH, RW = G::RW, HW = G::HW, HR = G::HR;
-  constexpr int TPE = G::TPE, CPT = G::CPT;
-  constexpr int NT = TPE * EB, NW = NT / 32;
-  constexpr int NBOX = (3 * EB + G::BOX_ROWS - 1) / G::BOX_ROWS;
-  constexpr unsigned BOX_BYTES = G::BOX_ROWS * 64;
-  static_assert(EB % 16 == 0, "whole warps");
+  using P = typename Pair<T>::type;
+  using VecT = typename Pair<T>::vec;
+  constexpr int W = G::W, NP = G::NP, VT = G::VT, RW = G::RW, RP = G::RP, HW = G::HW, HR = G::HR;
+  constexpr int ITERS = G::iters(EB), EPW = G::EPW;
+  constexpr int NT = G::threads(EB), NW = NT / 32;
+  static_assert(NW * EPW * ITERS == EB, "whole warps");
   extern __shared__ __align__(128) unsigned char sm_raw[];
   // the next unit, handed from thread 0 to the CTA: two slots used in turn,
   // so thread 0 never overwrites the slot another warp may still be reading
@@ -1009,46 +1033,26 @@ __global__ void __launch_bounds__(SweepGeo<T>::TPE * EB, sizeof(T) == 4 ? 2 : (E
   // it, and the warps would then disagree on the unit and on the barriers)
   __shared__ int s_unit[2];
   __shared__ double red_m[NW], red_s[NW];
-  __shared__ uint64_t bars[2];  // TMA completion of tile buffer 0 / 1
   // FP64: the 2^(j/64) table of the NFO exp (one entry for FP32, unused)
   __shared__ double etab[sizeof(T) == 8 ? EXP_TAB : 1];
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int sub = (tid & 31) / G::LPE, l8 = tid & (G::LPE - 1);
   if (sizeof(T) == 8)
     for (int i = tid; i < EXP_TAB; i += NT) etab[i] = exp2((double)i / EXP_TAB);
-  // tile buffers 1024-byte aligned (the swizzle pattern repeats every 512 B)
-  unsigned char* const base = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
-  const size_t tile_bytes = G::tile_bytes(EB, a.max_halo);
-  ElemRec<T>* const recs = reinterpret_cast<ElemRec<T>*>(base + 2 * tile_bytes);
-  unsigned char* const hrec = reinterpret_cast<unsigned char*>(recs + EB);
-  T* const vtab = reinterpret_cast<T*>(hrec + (size_t)a.max_halo * HR);  // cx, cy, NFINF (, |c|^2)
-  constexpr int UV = G::TPU_MAX * VT;
-  int* const hrow = reinterpret_cast<int*>(vtab + G::NTAB * UV);  // f rows of the unit's halo, 3 per element
-  const int j = tid % EB, hh = tid / EB;  // block element, and which of its TPE parts
-  const T third = (T)(1.0 / 3.0);
-  if (tid == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-    fence_mbar_init();
+  const unsigned tile_bytes = G::tile_bytes(EB, a.max_halo);
+  const bool two = a.sweep_bufs > 1;
+  unsigned char* const recs = sm_raw + (two ? 2 : 1) * tile_bytes;  // pitch RP
+  unsigned char* const hrec = recs + EB * RP;                       // pitch HR
+  unsigned char* const vtab = hrec + (size_t)a.max_halo * HR;       // [NVT][TPU_MAX] rows
+  int* const hl = reinterpret_cast<int*>(vtab + G::NVT * G::TPU_MAX * ROW_BYTES);  // the halo's elements
+  const int j0 = warp * EPW + sub;  // the lane group's block elements: j0 + it*NW*EPW
+  if (tid < ROW_BYTES / 4) {  // the tiles' rows of zeros
+    reinterpret_cast<float*>(sm_raw)[tid] = 0.f;
+    if (two) reinterpret_cast<float*>(sm_raw + tile_bytes)[tid] = 0.f;
   }
-  __syncthreads();
-  uint32_t par = 0;  // bit b: parity of the next phase of bars[b]
-  bool aborted = false;
-  int abort_buf = 0;
-  // the new block rows of tile vt (written into buffer bi by every thread,
-  // each followed by a proxy fence, before a barrier) as NBOX box stores
-  // issued by thread 0; rows past 3E are not written
-  auto store = [&](const CUtensorMap* map, int vt, int bi, int y0) {
-    const unsigned char* srcb = base + (size_t)bi * tile_bytes;
-#pragma unroll
-    for (int x = 0; x < NBOX; ++x) tma_store_2d(map, vt * VT, y0 + x * G::BOX_ROWS, srcb + x * BOX_BYTES);
-    bulk_commit();
-  };
 
   int unit = blockIdx.x, c = 0, iter = 0;
-  // tiles this CTA has started: the two tile buffers are used in turn across
-  // units, so a unit's first tile goes to the buffer its predecessor's last
-  // tile did not use, whose box store was issued a tile earlier
-  int gk = 0;
+  int gk = 0;  // tiles this CTA has started
   // residual partials of the thread's values: a single case adds them to its
   // control block once per CTA (after the last unit), a batch once per unit
   double rmax = 0.0, rsq = 0.0;
@@ -1058,12 +1062,6 @@ __global__ void __launch_bounds__(SweepGeo<T>::TPE * EB, sizeof(T) == 4 ? 2 : (E
     c = ONE ? 0 : find_case(a.unit_off, a.ncases, unit);
     const CaseDev<T>& C = ONE ? one : a.cases[c];
     const bool active = !C.ctrl->done;  // the same for every thread
-    if (!ONE && active && tid == 0) {
-      tensormap_acquire(&C.tm[0]);
-      tensormap_acquire(&C.tm[1]);
-    }
-    const CUtensorMap* last_map = nullptr;
-    int last_vt = 0, last_bi = 0, last_y0 = 0;
     if (active) {
       const int lu = unit - (ONE ? 0 : a.unit_off[c]);
       const int b = lu % C.nblocks, vg = lu / C.nblocks;
@@ -1073,403 +1071,306 @@ __global__ void __launch_bounds__(SweepGeo<T>::TPE * EB, sizeof(T) == 4 ? 2 : (E
       sweep_group(C, vg, vt0, ntl);
       const int cur = C.ctrl->cur;
       const double dtd = step_dt(C.ctrl);
-      const T dt = (T)dtd, dth = (T)(0.5 * dtd), dth3 = (T)(0.5 * dtd / 3.0);
-      const int* __restrict__ hlist = C.halo_list + h0;
-
-      // unit prologue, all of it asynchronous (the first tile's barrier
-      // publishes it): tile 0's block rows as TMA boxes (thread 0, once the
-      // buffer's last box store has read it) and its halo rows by cp.async,
-      // row numbers from the halo list; the block's element records, the
-      // halo's record heads and the unit's slices of the velocity tables
-      // (cp.async, in one group with the halo rows); the halo row list of
-      // the later tiles
-      {
-        const int bi0 = gk & 1;
-        unsigned char* dst = base + (size_t)bi0 * tile_bytes;
-        if (tid == 0) {
-          bulk_wait_read1();  // the newest store reads the other buffer
-          fence_proxy_async_smem();
-          mbar_expect_tx(&bars[bi0], NBOX * BOX_BYTES);
+      const T dt = (T)dtd;
+      const T* __restrict__ fo = C.f[cur];
+      T* __restrict__ fnw = C.f[cur ^ 1];
+      const unsigned pitch = (unsigned)C.Vp * (unsigned)sizeof(T);
+      unsigned own[ITERS];  // first rows of the lane group's elements
 #pragma unroll
-          for (int x = 0; x < NBOX; ++x)
-            tma_load_2d(dst + x * BOX_BYTES, &C.tm[cur], vt0 * VT, 3 * e0 + x * G::BOX_ROWS, &bars[bi0]);
-        }
-        const T* srcf = C.f[cur] + (size_t)vt0 * VT;
-        for (int w = tid; w < nh * 12; w += NT) {
-          const int row = w >> 2, cq = w & 3, h = row / 3;
-          cp_async16(dst + (tile_row_off(3 * EB + row) ^ (16u * cq)),
-                     srcf + (size_t)(hlist[h] * 3 + (row - 3 * h)) * C.Vp + cq * W);
-        }
+      for (int it = 0; it < ITERS; ++it) own[it] = 3u * (unsigned)(e0 + min(j0 + it * NW * EPW, nb - 1));
+      // Copies of tile vt's rows into a buffer by the lanes that will work on
+      // them in phase 1 (so a lane waits for its own copies only): the lane
+      // group's block elements (past the end of the mesh the last one again)
+      // and its share of the halo.
+      auto issue = [&](int vt, unsigned char* buf, const int* list) {
+        const unsigned char* src = reinterpret_cast<const unsigned char*>(fo + (size_t)vt * VT + l8 * W);
+        auto copy3 = [&](int slot, unsigned row) {
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+            cp_async16(buf + tile_row(3 * slot + i) + 16 * l8, src + (unsigned long long)(row + i) * pitch);
+        };
+#pragma unroll
+        for (int it = 0; it < ITERS; ++it) copy3(j0 + it * NW * EPW, own[it]);
+#pragma unroll 1
+        for (int h = j0; h < nh; h += NW * EPW) copy3(EB + h, 3u * (unsigned)list[h]);
+        cp_async_commit();
+      };
+      // unit prologue, all of it asynchronous: the block's element records,
+      // the halo's record heads and the unit's velocities, then the first
+      // tile's rows; the records are scaled by the step's factors as they
+      // land, by the threads that copied them
+      {
+        const int* __restrict__ hlist = C.halo_list + h0;
         const uint4* src = reinterpret_cast<const uint4*>(C.rec + e0);
-        for (int w = tid; w < nb * RW; w += NT) cp_async16(reinterpret_cast<uint4*>(recs) + w, src + w);
+        for (int w = tid; w < nb * RW; w += NT) cp_async16(recs + w / RW * RP + 16 * (w % RW), src + w);
         for (int w = tid; w < nh * HW; w += NT) {
           const int s = w / HW, k = w - s * HW;
           cp_async16(hrec + (size_t)s * HR + 16 * k, reinterpret_cast<const uint4*>(C.rec + hlist[s]) + k);
         }
-        // table t's values [vt0*VT, (vt0 + ntl)*VT) to vtab + t*UV, 16 bytes a copy
-        constexpr int TW = VT * (int)sizeof(T) / 16;  // 16-byte words of one tile's values
-        const int nw = ntl * TW;
-        for (int w = tid; w < G::NTAB * nw; w += NT) {
-          const int t = w / nw, x = w - t * nw;
-          cp_async16(reinterpret_cast<uint4*>(vtab + t * UV) + x,
-                     reinterpret_cast<const uint4*>(C.swtab + (size_t)t * C.Vp + (size_t)vt0 * VT) + x);
+        for (int w = tid; w < G::NVT * ntl * G::LPE; w += NT) {
+          const int t = w / (ntl * G::LPE), x = w - t * ntl * G::LPE;
+          cp_async16(vtab + t * G::TPU_MAX * ROW_BYTES + 16 * x,
+                     C.swtab + (size_t)(t == 2 ? 3 : t) * C.Vp + (size_t)vt0 * VT + (size_t)x * W);
         }
         cp_async_commit();
-        for (int s = tid; s < 3 * nh; s += NT) {
-          const int h = s / 3;
-          hrow[s] = hlist[h] * 3 + (s - 3 * h);
-        }
-      }
-      // copies of tile vt (k >= 1) into buffer bi: the block's rows (3*e0 ..)
-      // as NBOX TMA boxes issued by thread 0 once the buffer's last box store
-      // has read it (rows past 3E read as zeros), the halo rows (tile rows
-      // 3*EB ..) by cp.async, four threads per 64-byte row
-      auto issue = [&](int vt, int bi) {
-        unsigned char* dst = base + (size_t)bi * tile_bytes;
-        const T* src = C.f[cur] + (size_t)vt * VT;
-        for (int w = tid; w < nh * 12; w += NT) {
-          const int row = w >> 2, cq = w & 3;
-          cp_async16(dst + (tile_row_off(3 * EB + row) ^ (16u * cq)), src + (size_t)hrow[row] * C.Vp + cq * W);
-        }
-        if (tid == 0) {
-          bulk_wait_read0();
-          fence_proxy_async_smem();  // the buffer's previous generic accesses
-          mbar_expect_tx(&bars[bi], NBOX * BOX_BYTES);
-#pragma unroll
-          for (int x = 0; x < NBOX; ++x)
-            tma_load_2d(dst + x * BOX_BYTES, &C.tm[cur], vt * VT, 3 * e0 + x * G::BOX_ROWS, &bars[bi]);
-        }
-      };
-      const unsigned hx = 16u * CPT * hh;  // the thread's first chunk, as an offset XOR
-      // block element j's own rows at the thread's first chunk
-      unsigned own[3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) own[i] = tile_row_off(3 * j + i) ^ hx;
-      // the new rows of the previous tile, written back after the next
-      // tile's first barrier
-      VecT outv[CPT][3];
-      auto put_rows = [&](unsigned char* t) {
-        if (j < nb) {
-#pragma unroll
-          for (int cc = 0; cc < CPT; ++cc)
-#pragma unroll
-            for (int i = 0; i < 3; ++i) vst<T>(t + (own[i] ^ (16u * cc)), outv[cc][i]);
-        }
-        fence_proxy_async_smem();
-      };
-
-      for (int k = 0; k < ntl; ++k, ++gk) {
-        const int bi = gk & 1;
-        unsigned char* const tl = base + (size_t)bi * tile_bytes;
-        // thread 0 waits for the boxes (the others wait in the barrier, not
-        // spinning); every thread waits for its own halo copies
-        const uint32_t ph = (par >> bi) & 1u;
-        const bool ok = tid != 0 || mbar_wait_bounded(&bars[bi], ph);
-        par ^= 1u << bi;
-        cp_async_wait<0>();
-        // tile k has landed (or the wait expired), and every thread has
-        // written and fenced its new rows of tile k - 1
-        if (__syncthreads_or(ok ? 0 : 1)) {
-          aborted = true;
-          abort_buf = bi;
-          break;
-        }
-        if (tid != 0) mbar_try_wait(&bars[bi], ph);  // completed: acquires the box data
-        // every thread is past its phase-2 reads of tile k - 1: its new rows
-        // replace the block rows in its buffer, for the box store
-        if (k > 0) put_rows(base + (size_t)(bi ^ 1) * tile_bytes);
-        const int vb0 = (vt0 + k) * VT;
-        const T* vx = vtab + k * VT;
-        const T* vy = vtab + UV + k * VT;
-        const T* vn = vtab + 2 * UV + k * VT;
-        const T* vc2 = vtab + (G::NTAB - 1) * UV + k * VT;  // |c|^2 (FP64; unused in FP32)
-
-        // ---- phase 1: block element j (chunks CPT*hh ..), then the halo
-        // chunk by chunk
-        VecT qr[CPT][3], ur[CPT];
-        if (j < nb) {
-          const ElemRec<T>& r = recs[j];
-#pragma unroll
-          for (int cc = 0; cc < CPT; ++cc) {
-            const int cq = CPT * hh + cc;
-            const unsigned ro[3] = {own[0] ^ (16u * cc), own[1] ^ (16u * cc), own[2] ^ (16u * cc)};
-            sweep_p1<T>(r, etab, tl, ro, vld<T>(vx + cq * W), vld<T>(vy + cq * W), vld<T>(vc2 + cq * W), dth, dth3,
-                        qr[cc], ur[cc]);
-          }
-        }
-        for (int w = tid; w < nh * NCH; w += NT) {
-          const int hs = w >> 2, cq = w & 3;
-          const ElemRec<T>& r = *reinterpret_cast<const ElemRec<T>*>(hrec + (size_t)hs * HR);
-          const int r0 = 3 * (EB + hs);
-          const unsigned ro[3] = {tile_row_off(r0) ^ (16u * cq), tile_row_off(r0 + 1) ^ (16u * cq),
-                                  tile_row_off(r0 + 2) ^ (16u * cq)};
-          VecT qd[3], ud;
-          sweep_p1<T>(r, etab, tl, ro, vld<T>(vx + cq * W), vld<T>(vy + cq * W), vld<T>(vc2 + cq * W), dth, dth3, qd,
-                      ud);
+        issue(vt0, sm_raw + (two ? (gk & 1) * tile_bytes : 0), hlist);
+        for (int s = tid; s < nh; s += NT) hl[s] = hlist[s];
+        cp_async_wait<1>();
+        const T dth = (T)(0.5 * dtd), mdt6 = (T)(-0.5 * dtd / 3.0);
+        for (int w = tid; w < nb * RW; w += NT)
+          sweep_scale<T>(recs + w / RW * RP + 16 * (w % RW), w % RW, dth, mdt6, dt);
+        for (int w = tid; w < nh * HW; w += NT) {
+          const int s = w / HW, k = w - s * HW;
+          sweep_scale<T>(hrec + (size_t)s * HR + 16 * k, k, dth, mdt6, dt);
         }
         __syncthreads();
-        // tile k - 1's new rows are in place: store them, then load tile k + 1
-        // into that buffer once the store has read it
-        if (tid == 0 && k > 0) store(&C.tm[cur ^ 1], vt0 + k - 1, bi ^ 1, 3 * e0);
-        if (k + 1 < ntl) {
-          issue(vt0 + k + 1, bi ^ 1);
-          cp_async_commit();
-        }
+      }
 
-        // ---- phase 2: the update of block element j, chunks CPT*hh ..
-        // CPT*hh + CPT - 1 (row offsets own[], srcp[], srcq[] are at chunk
-        // CPT*hh; chunk CPT*hh + cc of the same row is at offset ^ 16*cc)
-        T rmt = (T)0, sqt = (T)0;
-        if (j < nb) {
-          const ElemRec<T>& r = recs[j];
-          // per edge: the flux source's rows, AL*n where the edge carries
-          // the element-centric flux (zero on inflow and wall sides, whose
-          // flux the wall path adds); MU*DTE, MM*DTE
-          const int flags = r.flags;
-          unsigned srcp[3], srcq[3];
-          T anx[3], any[3], mudt[3], mmdt[3], cmx[3], cmn[3];
+      for (int k = 0; k < ntl; ++k, ++gk) {
+        unsigned char* const tl8 = sm_raw + (two ? (gk & 1) * tile_bytes : 0) + 16 * l8;
+        const int v0 = (vt0 + k) * VT + l8 * W;  // the lane's first velocity
+        const unsigned char* vt = vtab + k * ROW_BYTES + 16 * l8;
+        const VecT cxv = vld<T>(vt), cyv = vld<T>(vt + G::TPU_MAX * ROW_BYTES),
+                   c2v = vld<T>(vt + (G::NVT - 1) * G::TPU_MAX * ROW_BYTES);  // |c|^2 (FP64)
+        cp_async_wait<0>();
+
+        // ---- phase 1: the lane group's block elements and its share of
+        // the halo
+        VecT q[ITERS][3], u[ITERS];
 #pragma unroll
-          for (int k2 = 0; k2 < 3; ++k2) {
-            srcp[k2] = r.edge[k2].offp ^ hx;
-            srcq[k2] = r.edge[k2].offq ^ hx;
-            const bool fl = (flags & (FLAG_FLUX0 << k2)) != 0;
-            anx[k2] = fl ? r.edge[k2].anx : (T)0;
-            any[k2] = fl ? r.edge[k2].any : (T)0;
-          }
+        for (int it = 0; it < ITERS; ++it) {
+          const int j = j0 + it * NW * EPW;
+          sweep_p1<T>(*reinterpret_cast<const ElemRec<T>*>(recs + min(j, nb - 1) * RP), etab, tl8 + tile_row(3 * j), cxv, cyv, c2v, q[it], u[it]);
+        }
+#pragma unroll 1
+        for (int h = j0; h < nh; h += NW * EPW) {
+          VecT qh[3], uh;
+          sweep_p1<T>(*reinterpret_cast<const ElemRec<T>*>(hrec + (size_t)h * HR), etab,
+                      tl8 + tile_row(3 * (EB + h)), cxv, cyv, c2v, qh, uh);
+        }
+        __syncthreads();
+        if (two && k + 1 < ntl) issue(vt0 + k + 1, sm_raw + ((gk + 1) & 1) * tile_bytes, hl);
+
+        // ---- phase 2: the update of the lane group's block elements
+        const bool whole = (vt0 + k + 1) * VT <= C.V;  // no velocity of the tile past V
+        T rmt = (T)0;
+        P sqt = pdup((T)0);
+#pragma unroll
+        for (int it = 0; it < ITERS; ++it) {
+          const int j = j0 + it * NW * EPW;
+          const bool live = j < nb;  // past the end of the mesh: nothing is written
+          const ElemRec<T>& r = *reinterpret_cast<const ElemRec<T>*>(recs + min(j, nb - 1) * RP);
+          const int flags = r.flags;
+          P rhs[3][NP], sgm[NP], g[3][NP];
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
-            mudt[i] = r.mu[i] * dt;
-            mmdt[i] = r.mm[i] * dt;
-            if (IMMAT == 0) {
-              cmx[i] = C.cmax[3 * (e0 + j) + i];
-              cmn[i] = C.cmin[3 * (e0 + j) + i];
-            }
+            const VecT gv = vld<T>(tl8 + tile_row(3 * j + i));
+#pragma unroll
+            for (int h = 0; h < NP; ++h) g[i][h] = pget(gv, h);
           }
 #pragma unroll
-          for (int cc = 0; cc < CPT; ++cc) {
-            const int cq = CPT * hh + cc;
-            const unsigned cx16 = 16u * cc;
-            const int vb = vb0 + cq * W;
-            VecT(&out)[3] = outv[cc];
-            if (vb >= C.V) {  // all past V: the padding stays zero
+          for (int h = 0; h < NP; ++h) sgm[h] = padd(padd(g[0][h], g[1][h]), g[2][h]);
+          // Edge fluxes (EDGFLXOPT, src/edgflxopt.f90:95-125): RHS_p -=
+          // AL*SC*(2 u_p + u_q), RHS_q -= AL*SC*(u_p + 2 u_q), (u_p, u_q)
+          // the element's own values where AL*SC > 0, the source's otherwise.
+          // The node opposite the edge takes GETELC's volume term RHS_i =
+          // AREA/3 (N_i,x cx + N_i,y cy) sum(g) (src/getelc.f90:87-117): for
+          // P1, AREA/3 grad N_i = -(EL/6) n of that edge.  -AL*SC is formed,
+          // so that every term is one fused multiply-add.
 #pragma unroll
-              for (int i = 0; i < 3; ++i) out[i] = VecT{};
-              continue;
-            }
-            const VecT cxv = vld<T>(vx + cq * W), cyv = vld<T>(vy + cq * W);
-            VecT g[3];
+          for (int k2 = 0; k2 < 3; ++k2) {
+            const int p = k2, qn = (k2 + 1) % 3, op = (k2 + 2) % 3;
+            const VecT gpv = vld<T>(tl8 + r.off[k2][0]), gqv = vld<T>(tl8 + r.off[k2][1]);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) g[i] = vld<T>(tl + (own[i] ^ cx16));
-            // GETELC second half, the volume term RHS_i = AREA/3 (N_i,x cx +
-            // N_i,y cy) sum(g) (src/getelc.f90:87-117).  For P1,
-            // AREA/3 grad N_i = -(EL/6) n of the edge opposite node i, so an
-            // element whose three sides are interior (AL*n of every edge at
-            // hand) takes RHS_i = -AL*c.n(edge (i+1) mod 3) * sum(g), added
-            // in the edge loop below (sgm = sum(g)); the others use the
-            // gradients, with RHS_3 = -(RHS_1 + RHS_2) from the gradients
-            // summing to zero (sgm = 0)
-            T rhs[3][W], sgm[W];
-            if (flags & FLAG_INTERIOR) {
-#pragma unroll
-              for (int w = 0; w < W; ++w) {
-                sgm[w] = VO::get(g[0], w) + VO::get(g[1], w) + VO::get(g[2], w);
-                rhs[0][w] = rhs[1][w] = rhs[2][w] = (T)0;
-              }
-            } else {
-              const T area3 = r.area * third;
-#pragma unroll
-              for (int w = 0; w < W; ++w) {
-                const T cx = VO::get(cxv, w), cy = VO::get(cyv, w);
-                const T s3 = (VO::get(g[0], w) + VO::get(g[1], w) + VO::get(g[2], w)) * area3;
-                rhs[0][w] = (r.gx[0] * cx + r.gy[0] * cy) * s3;
-                rhs[1][w] = (r.gx[1] * cx + r.gy[1] * cy) * s3;
-                rhs[2][w] = -(rhs[0][w] + rhs[1][w]);
-                sgm[w] = (T)0;
+            for (int h = 0; h < NP; ++h) {
+              const P ms = pfma(pdup(r.en[k2][0]), pget(cxv, h), pmul(pdup(r.en[k2][1]), pget(cyv, h)));  // -AL*SC
+              const P gp = pget(gpv, h), gq = pget(gqv, h);
+              P up, uq;
+              up.x = ms.x < (T)0 ? g[p][h].x : gp.x;
+              up.y = ms.y < (T)0 ? g[p][h].y : gp.y;
+              uq.x = ms.x < (T)0 ? g[qn][h].x : gq.x;
+              uq.y = ms.y < (T)0 ? g[qn][h].y : gq.y;
+              const P fp = pfma(pdup((T)2), up, uq), fq = pfma(pdup((T)2), uq, up);
+              if (k2 == 0) {
+                rhs[p][h] = pmul(ms, fp);
+                rhs[qn][h] = pmul(ms, fq);
+                rhs[op][h] = pmul(ms, sgm[h]);
+              } else {
+                rhs[p][h] = pfma(ms, fp, rhs[p][h]);
+                rhs[qn][h] = pfma(ms, fq, rhs[qn][h]);
+                rhs[op][h] = pfma(ms, sgm[h], rhs[op][h]);
               }
             }
-            // edge fluxes (EDGFLXOPT, src/edgflxopt.f90:95-125): RHS_p -=
-            // AL*SC*(2 u_p + u_q), RHS_q -= AL*SC*(u_p + 2 u_q), (u_p, u_q)
-            // the element's own values where AL*SC > 0, the source's
-            // otherwise; AL*SC is zero on sides without the element-centric
-            // flux.  The node opposite the edge takes the volume term.
+          }
+          // GETINC / CMMINC, ADTHEM (f >= 0), INFLOW and the residual.  An
+          // element away from walls and inflow at velocities below V takes
+          // the plain form; dmask (ALPHA < 1): bit 3*w + i marks node i at
+          // velocity v0 + w as deferred (its update gets the specular part in
+          // k_wspec).
+          unsigned dmask = 0u;
+          P sq = pdup((T)0);
+          VecT out[3];
+          auto finish = [&](auto plain) {
+            constexpr bool PLAIN = decltype(plain)::value;
 #pragma unroll
-            for (int k2 = 0; k2 < 3; ++k2) {
-              const int p = k2, qn = (k2 + 1) % 3, op = (k2 + 2) % 3;
-              const VecT gp = vld<T>(tl + (srcp[k2] ^ cx16)), gq = vld<T>(tl + (srcq[k2] ^ cx16));
-#pragma unroll
-              for (int w = 0; w < W; ++w) {
-                const T as = anx[k2] * VO::get(cxv, w) + any[k2] * VO::get(cyv, w);
-                const bool mine = as > (T)0;
-                const T up = mine ? VO::get(g[p], w) : VO::get(gp, w);
-                const T uq = mine ? VO::get(g[qn], w) : VO::get(gq, w);
-                rhs[p][w] -= as * ((T)2 * up + uq);
-                rhs[qn][w] -= as * (up + (T)2 * uq);
-                rhs[op][w] -= as * sgm[w];
+            for (int i = 0; i < 3; ++i) {
+              const bool counts = PLAIN || !(flags & (1 << i));  // not reset by INFLOW
+              T cmx = (T)0, cmn = (T)0;
+              if (IMMAT == 0) {
+                cmx = C.cmax[3 * (e0 + min(j, nb - 1)) + i];
+                cmn = C.cmin[3 * (e0 + min(j, nb - 1)) + i];
               }
-            }
-            // ALPHA < 1: bit 3*w + i marks node i at velocity vb + w as
-            // deferred (its update gets the specular part in k_wspec)
-            unsigned dmask = 0u;
-            if (flags & 0x38) {
-              // wall sides; molecules leaving the wall (src/getbou.f90:189-255)
-              // carry the diffuse part ALPHA*ETA*Mw here, the specular part
-              // (1-ALPHA)*Rf in k_wspec
-              const bool spec = C.spec != 0;
 #pragma unroll
-              for (int k2 = 0; k2 < 3; ++k2) {
-                if (!(flags & (8 << k2))) continue;
-                const int p = k2, qn = (k2 + 1) % 3;
-                const int bs = r.bside[k2];
-                const T twr = (T)2 * C.rgas * C.bTw[bs];
-                const T uwx = C.bUw[2 * bs], uwy = C.bUw[2 * bs + 1], eta = C.bEta[bs];
-                const T wnx = r.edge[k2].anx, wny = r.edge[k2].any;  // AL*n of the wall side
-                // with the specular part, the wall branch is taken where the
-                // host's FP64 TEST < 0 (the items of k_wspec are built from it)
-                const int* rfi = spec ? C.rf_i + (size_t)C.rside[bs] * C.V * 2 : nullptr;
-#pragma unroll
-                for (int w = 0; w < W; ++w) {
-                  const T cx = VO::get(cxv, w), cy = VO::get(cyv, w);
-                  const T asw = wnx * cx + wny * cy;  // AL * (n.c), the sign of TEST
-                  const bool own = spec ? !(vb + w < C.V && rfi[2 * (vb + w)] >= 0) : asw >= (T)0;
-                  T up, uq;
-                  if (own) {
-                    up = VO::get(g[p], w);
-                    uq = VO::get(g[qn], w);
-                  } else {
-                    T mw;
-                    if (uwx == (T)0 && uwy == (T)0) {
-                      const T spd = sqrt(cx * cx + cy * cy);
-                      mw = dexp<T>(-(spd * spd) / twr);
-                    } else {
-                      const T dx = cx - uwx, dy = cy - uwy;
-                      mw = dexp<T>(-(dx * dx + dy * dy) / twr);
-                    }
-                    up = uq = C.alpha * (mw * eta);
-                    if (spec) dmask |= ((1u << p) | (1u << qn)) << (3 * w);
-                  }
-                  rhs[p][w] -= asw * ((T)2 * up + uq);
-                  rhs[qn][w] -= asw * (up + (T)2 * uq);
+              for (int h = 0; h < NP; ++h) {
+                const P f = padd(g[i][h], pget(u[it], h));
+                const P cdt = pmul(pdup(r.mt[i]), psub(pget(q[it][i], h), f));  // COLL*DTE
+                const P d = pfma(pdup(r.mm[i]), rhs[i][h], cdt);
+                P rr, ch, fn = padd(f, d);
+                if (IMMAT == 1) {
+                  rr.x = fabs(d.x);
+                  rr.y = fabs(d.y);
+                } else {
+                  rr.x = fmax((rhs[i][h].x >= (T)0 ? cmx : cmn) * (rhs[i][h].x * dt) + cdt.x, (T)0);
+                  rr.y = fmax((rhs[i][h].y >= (T)0 ? cmx : cmn) * (rhs[i][h].y * dt) + cdt.y, (T)0);
                 }
-              }
-            }
-            // GETINC / CMMINC, ADTHEM (f >= 0), INFLOW; the padding past V
-            // stays zero
-            // defer: some node of this chunk waits for the specular part
-            // (only wall elements with ALPHA < 1; the other variant has no
-            // per-value test)
-            auto finish = [&](auto full, auto defer) {
-#pragma unroll
-              for (int w = 0; w < W; ++w) {
-                const bool live = decltype(full)::value || vb + w < C.V;
-                const T u = VO::get(ur[cc], w);
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                  const T f = VO::get(g[i], w) + u;
-                  const T qmf = VO::get(qr[cc][i], w) - f;
-                  T d, rr, x = (T)0, cdt = (T)0;
-                  if (IMMAT == 1) {
-                    d = mmdt[i] * rhs[i][w] + mudt[i] * qmf;
-                    rr = fabs(d);
-                  } else {
-                    x = rhs[i][w] * dt;
-                    cdt = mudt[i] * qmf;
-                    d = r.mm[i] * x + cdt;
-                    rr = ((x >= (T)0) ? cmx[i] : cmn[i]) * x + cdt;
-                    rr = rr > (T)0 ? rr : (T)0;
-                  }
-                  // L2 residual: the change the unknown receives (-f where
-                  // the clip applies, i.e. where d < -f; none at
-                  // inflow-reset nodes); a non-finite d or f reaches the sum
-                  T ch;
-                  if constexpr (sizeof(T) == 4)
-                    ch = fmax_nan(d, -f);
-                  else
-                    ch = (f + d < (T)0) ? -f : d;
-                  T fn = fmax(f + d, (T)0);
-                  if (live) {
-                    if (decltype(defer)::value && ((dmask >> (3 * w + i)) & 1u)) {
+                // L2 residual: the change the unknown receives (-f where
+                // the clip applies, i.e. where d < -f; none at inflow-reset
+                // nodes); a non-finite d or f reaches the sum
+                if constexpr (sizeof(T) == 4) {
+                  ch.x = fmax_nan(d.x, -f.x);
+                  ch.y = fmax_nan(d.y, -f.y);
+                } else {
+                  ch.x = fn.x < (T)0 ? -f.x : d.x;
+                  ch.y = fn.y < (T)0 ? -f.y : d.y;
+                }
+                fn.x = fmax(fn.x, (T)0);
+                fn.y = fmax(fn.y, (T)0);
+                if constexpr (PLAIN) {
+                  rmt = fmax(rmt, fmax(rr.x, rr.y));
+                  sq = pfma(ch, ch, sq);
+                } else {
+                  auto value = [&](int w, T dd, T rrr, T chh, T xx, T cc, T& ff, T& s) {
+                    if (v0 + w >= C.V) {
+                      ff = (T)0;
+                      return;
+                    }
+                    if ((dmask >> (3 * w + i)) & 1u) {
                       // deferred: k_wspec adds the specular part, clips and
                       // counts the residual
-                      const size_t o = ((size_t)r.wslot * 3 + i) * C.Vp + vb + w;
-                      if (IMMAT == 1) {
-                        C.wd[o] = d;
-                      } else {
-                        C.wd[o] = x;
-                        C.wd[(size_t)C.n_spec_slots * 3 * C.Vp + o] = cdt;
+                      if (live) {
+                        const size_t o = ((size_t)r.wslot * 3 + i) * C.Vp + v0 + w;
+                        if (IMMAT == 1) {
+                          C.wd[o] = dd;
+                        } else {
+                          C.wd[o] = xx * dt;
+                          C.wd[(size_t)C.n_spec_slots * 3 * C.Vp + o] = cc;
+                        }
                       }
                     } else {
-                      rmt = fmax(rmt, rr);
-                      if (!(flags & (1 << i))) sqt += ch * ch;
+                      rmt = fmax(rmt, rrr);
+                      if (counts) s += chh * chh;
                     }
-                  } else {
-                    fn = (T)0;
-                  }
-                  VO::set(out[i], w, fn);
+                  };
+                  value(2 * h, d.x, rr.x, ch.x, rhs[i][h].x, cdt.x, fn.x, sq.x);
+                  value(2 * h + 1, d.y, rr.y, ch.y, rhs[i][h].y, cdt.y, fn.y, sq.y);
                 }
+                pset(out[i], h, fn);
               }
-            };
-            if (dmask != 0u) {
-              if (vb + W <= C.V)
-                finish(std::true_type(), std::true_type());
-              else
-                finish(std::false_type(), std::true_type());
-            } else {
-              if (vb + W <= C.V)
-                finish(std::true_type(), std::false_type());
-              else
-                finish(std::false_type(), std::false_type());
             }
+          };
+          if (whole && (flags & 0x1ff) == 0) {
+            finish(std::true_type());
+          } else {
+            // Wall sides: molecules leaving the wall (src/getbou.f90:189-255)
+            // carry the diffuse part ALPHA*ETA*Mw here, the specular part
+            // (1-ALPHA)*Rf in k_wspec; inflow sides: no flux.  The edge loop
+            // has added the element's own values where AL*SC > 0 and nothing
+            // elsewhere: the difference is added.
+            const bool spec = C.spec != 0;
+#pragma unroll
+            for (int k2 = 0; k2 < 3; ++k2) {
+              const bool inflow = (flags & (FLAG_INFLOW_EDGE0 << k2)) != 0;
+              if (!inflow && !(flags & (8 << k2))) continue;
+              const int p = k2, qn = (k2 + 1) % 3;
+              const int bs = inflow ? 0 : r.bside[k2];
+              const T twr = (T)2 * C.rgas * C.bTw[bs];
+              const T uwx = C.bUw[2 * bs], uwy = C.bUw[2 * bs + 1], eta = C.bEta[bs];
+              const T wnx = pval(r.en[k2][0]), wny = pval(r.en[k2][1]);  // -AL*n of the side
+              // with the specular part, the wall branch is taken where the
+              // host's FP64 TEST < 0 (the items of k_wspec are built from it)
+              const int* rfi = spec && !inflow ? C.rf_i + (size_t)C.rside[bs] * C.V * 2 : nullptr;
+              auto wall = [&](int w, T cx, T cy, T gp, T gq, T& rp, T& rq) {
+                const T ms = wnx * cx + wny * cy;  // -AL*SC, as in the edge loop
+                const bool mine = rfi ? !(v0 + w < C.V && rfi[2 * (v0 + w)] >= 0) : ms <= (T)0;
+                T up = gp, uq = gq;
+                if (inflow) {
+                  up = uq = (T)0;
+                } else if (!mine) {
+                  T mw;
+                  if (uwx == (T)0 && uwy == (T)0) {
+                    const T spd = sqrt(cx * cx + cy * cy);
+                    mw = dexp<T>(-(spd * spd) / twr);
+                  } else {
+                    const T dx = cx - uwx, dy = cy - uwy;
+                    mw = dexp<T>(-(dx * dx + dy * dy) / twr);
+                  }
+                  up = uq = C.alpha * (mw * eta);
+                  if (spec) dmask |= ((1u << p) | (1u << qn)) << (3 * w);
+                }
+                if (ms < (T)0) {
+                  up -= gp;
+                  uq -= gq;
+                }
+                rp += ms * ((T)2 * up + uq);
+                rq += ms * (up + (T)2 * uq);
+              };
+#pragma unroll
+              for (int h = 0; h < NP; ++h) {
+                const P cx = pget(cxv, h), cy = pget(cyv, h);
+                wall(2 * h, cx.x, cy.x, g[p][h].x, g[qn][h].x, rhs[p][h].x, rhs[qn][h].x);
+                wall(2 * h + 1, cx.y, cy.y, g[p][h].y, g[qn][h].y, rhs[p][h].y, rhs[qn][h].y);
+              }
+            }
+            finish(std::false_type());
             if (flags & 7) {
-              const VecT nf = vld<T>(vn + cq * W);  // zero past V
+              const VecT nf = vld<T>(C.nfinf + v0);  // zero past V
 #pragma unroll
               for (int i = 0; i < 3; ++i)
                 if (flags & (1 << i)) out[i] = nf;
             }
           }
+          if (live) {
+            sqt = padd(sqt, sq);
+            unsigned char* dst = reinterpret_cast<unsigned char*>(fnw + v0);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) vst<T>(dst + (unsigned long long)(own[it] + i) * pitch, out[i]);
+          }
         }
         rmax = fmax(rmax, (double)rmt);
-        rsq += (double)sqt;
-      }
-      if (aborted) {
-        // a bounded wait expired (the vote made every thread leave the tile
-        // loop together): drain this CTA's copies in flight, bounded, and
-        // report through the case's control block
-        if (tid == 0) {
-          C.ctrl->timeout = 1;
-          mbar_wait_bounded(&bars[abort_buf], ((par >> abort_buf) & 1u) ^ 1u);
-          bulk_wait0();
+        rsq += (double)sqt.x + (double)sqt.y;
+        if (!two && k + 1 < ntl) {
+          __syncthreads();
+          issue(vt0 + k + 1, sm_raw, hl);
         }
-        return;
       }
       // a batch: the unit's residual, per warp
       if (!ONE) {
         rmax = warp_max(rmax);
         rsq = warp_sum(rsq);
         if ((tid & 31) == 0) {
-          red_m[tid >> 5] = rmax;
-          red_s[tid >> 5] = rsq;
+          red_m[warp] = rmax;
+          red_s[warp] = rsq;
         }
         rmax = rsq = 0.0;
       }
-      last_map = &C.tm[cur ^ 1];
-      last_vt = vt0 + ntl - 1;
-      last_bi = (gk - 1) & 1;
-      last_y0 = 3 * e0;
-      // the last tile's new rows, once every thread is past its reads
-      __syncthreads();
-      put_rows(base + (size_t)last_bi * tile_bytes);
     }
-    // every thread is past phase 2 of the unit's last tile and has written
-    // its rows: store the last tile and (a batch) add the unit's residual to
-    // its case (the sum of squares can differ in its last bits between runs:
-    // the order of the atomics varies); the records, tables and halo list
-    // may be replaced
+    // every thread is past phase 2 of the unit's last tile: (a batch) add the
+    // unit's residual to its case (the sum of squares can differ in its last
+    // bits between runs: the order of the atomics varies); the records and
+    // the halo list may be replaced
     if (tid == 0) s_unit[iter & 1] = next;
     __syncthreads();
-    if (tid == 0 && last_map) {
-      store(last_map, last_vt, last_bi, last_y0);
-      if (!ONE) resid_add<NW>(C.ctrl, red_m, red_s);
-    }
+    if (!ONE && active && tid == 0) resid_add<NW>(C.ctrl, red_m, red_s);
     unit = s_unit[iter & 1];
     ++iter;
     if (tid == 0 && unit < total_units) next = (int)gridDim.x + atomicAdd(&a.ctl->sweep_next, 1);
@@ -1480,13 +1381,12 @@ __global__ void __launch_bounds__(SweepGeo<T>::TPE * EB, sizeof(T) == 4 ? 2 : (E
     rmax = warp_max(rmax);
     rsq = warp_sum(rsq);
     if ((tid & 31) == 0) {
-      red_m[tid >> 5] = rmax;
-      red_s[tid >> 5] = rsq;
+      red_m[warp] = rmax;
+      red_s[warp] = rsq;
     }
     __syncthreads();
     if (tid == 0) resid_add<NW>(one.ctrl, red_m, red_s);
   }
-  if (tid == 0) bulk_wait0();  // the last box stores are complete before the CTA exits
 }
 
 // ------------------------------------------------ specular wall part ----
@@ -1532,7 +1432,7 @@ template <class T> __global__ void __launch_bounds__(256) k_wspec(const __grid_c
       const int p = k, q = (k + 1) % 3;
       const T dp = om * ((zd2 * F(p, i1) + zd1 * F(p, i2)) / (zd1 + zd2));
       const T dq = om * ((zd2 * F(q, i1) + zd1 * F(q, i2)) / (zd1 + zd2));
-      const T as = r.edge[k].anx * cx + r.edge[k].any * cy;  // AL * (n.c)
+      const T as = -(pval(r.en[k][0]) * cx + pval(r.en[k][1]) * cy);  // AL * (n.c)
       drhs[p] -= as * ((T)2 * dp + dq);
       drhs[q] -= as * (dp + (T)2 * dq);
       mask |= (1u << p) | (1u << q);
@@ -1543,12 +1443,12 @@ template <class T> __global__ void __launch_bounds__(256) k_wspec(const __grid_c
       const size_t od = ((size_t)s * 3 + i) * C.Vp + v;
       T d, rr;
       if (C.immat == 1) {
-        d = C.wd[od] + (r.mm[i] * dt) * drhs[i];
+        d = C.wd[od] + (pval(r.mm[i]) * dt) * drhs[i];
         rr = fabs(d);
       } else {
         // CMMINC (src/cmminc.f90:22-41) on the whole RHS*DTE
         const T x = C.wd[od] + dt * drhs[i], cdt = C.wd[(size_t)C.n_spec_slots * 3 * C.Vp + od];
-        d = r.mm[i] * x + cdt;
+        d = pval(r.mm[i]) * x + cdt;
         rr = ((x >= (T)0) ? C.cmax[3 * (size_t)e + i] : C.cmin[3 * (size_t)e + i]) * x + cdt;
         rr = rr > (T)0 ? rr : (T)0;
       }

@@ -16,62 +16,77 @@
 
 namespace dgbgk {
 
-// Per element and local edge k (from local node k to node (k+1) mod 3).
-// The sweep forms every edge flux from an upwind "source" row set: the
-// neighbour across an interior side, the element itself on an outflow side
-// (the upwind value of an outflow side is always the element's own) and, as a
-// placeholder, on inflow sides (no flux) and wall sides (whose flux the wall
-// path adds).  The source's two rows (its local nodes at my points k and
-// k+1) are given as their byte offsets in the sweep tile at velocity chunk 0
-// (tile_row_off below); chunk c of the same row is at offset ^ 16*c.
-template <class T> struct alignas(16) ElemEdge {
-  T anx, any;      // AL times the outward unit normal; AL = EL/6 (interior) or RSIDO(3)/6 (boundary)
-  unsigned offp;   // tile offset of the source's row at point k
-  unsigned offq;   // ... at point k+1
-};
+// A row of a sweep tile in bytes: one velocity segment of a DG node.  The
+// first row of a tile holds zeros, row r = 3*slot + i comes after it.
+constexpr int ROW_BYTES = 128;
+constexpr unsigned tile_row(int r) { return (unsigned)(r + 1) * ROW_BYTES; }
 
-// Byte offset of 16-byte chunk 0 of row r in a sweep tile (64-byte rows
-// with the 64-byte swizzle: chunk c of row r at 16*(c ^ ((r >> 1) & 3)),
-// i.e. at tile_row_off(r) ^ 16*c).
+// A coefficient of an element record.  FP32: the value twice, the operand of
+// a packed instruction on two velocities as it is loaded (duplicating in
+// registers took one ALU instruction per coefficient and use); FP64: the
+// value.
+struct alignas(8) CoefF {
+  float x, y;
+};
+template <class T> struct CoefOf;
+template <> struct CoefOf<float> {
+  using type = CoefF;
+};
+template <> struct CoefOf<double> {
+  using type = double;
+};
 #if defined(__CUDACC__)
 __host__ __device__
 #endif
-inline unsigned tile_row_off(int r) { return (unsigned)(r * 64 + 16 * ((r >> 1) & 3)); }
+inline void coef_set(CoefF& c, double v) { c.x = c.y = (float)v; }
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+inline void coef_set(double& c, double v) { c = v; }
 
 // Everything the sweep needs about one element, in one 16-byte-aligned
 // record.  The leading part (shape-function gradients and the GTEQNF /
-// COMPMU parameters of the three DG nodes, 21 values) is all a halo element
-// needs; the moment kernel rewrites the node parameters every step.
+// COMPMU parameters of the three DG nodes, 21 coefficients) is all a halo
+// element needs; the moment kernel rewrites the node parameters every step.
+//
+// Per local edge k (from local node k to node (k+1) mod 3) the sweep forms
+// the flux from an upwind "source" row set: the neighbour across an interior
+// side, the element itself on an outflow side (the upwind value of an outflow
+// side is always the element's own) and the tile's row of zeros on wall
+// sides (the wall's own flux is added by a separate path) and on inflow sides
+// (no flux; the part the element's own values add is taken out by the same
+// path).  The source's two rows (its local nodes at my points k and k+1) are
+// given as their byte offsets in the sweep tile (tile_row).
 template <class T> struct alignas(16) ElemRec {
-  T gx[3], gy[3];  // shape-function gradients GEOME(1:3), GEOME(4:6)
+  using C = typename CoefOf<T>::type;
+  C gx[3], gy[3];  // shape-function gradients GEOME(1:3), GEOME(4:6)
   // GTEQNF's Maxwellian NFO (src/gteqnf.f90:26-40) at node i and velocity c,
   // with A = DISND*BETA2/PI and u = (DISUX, DISUY):
-  //  FP32: NFO = A * 2^(ex*|c-u|^2), ex = -BETA2*log2(e): A, ex, ux, uy;
+  //  FP32: NFO = A * 2^(ex*|c-u|^2), ex = -BETA2*log2(e): A, ex, and -u in
+  //        ux, uy;
   //  FP64: NFO = exp(a0 + a1*cx + a2*cy + ex*|c|^2), the exponent expanded:
   //        A holds a0 = ln(A) - BETA2*|u|^2, ux a1 = 2*BETA2*ux, uy a2 =
   //        2*BETA2*uy, ex = -BETA2 (a0 = -inf where A = 0).
   // (NFO = 0 where DISPS < 1e-20, src/gteqnf.f90:32.)
-  T A[3];
-  T ex[3];
-  T ux[3];
-  T uy[3];
-  T mu[3];   // collision frequency MU (src/compmu.f90:90-92)
-  T area;    // 0.5 * GEOME(7)   (src/getelc.f90:44)
-  T mm[3];   // MMAT (IMMAT = 1) or CMMAT row sums (IMMAT = 0)
+  C A[3];
+  C ex[3];
+  C ux[3];
+  C uy[3];
+  C mu[3];     // collision frequency MU (src/compmu.f90:90-92)
+  C pad;
+  C mt[3];     // MU again, for the update of the element's own values
+  C mm[3];     // MMAT (IMMAT = 1) or CMMAT row sums (IMMAT = 0)
+  C en[3][2];  // per edge -AL times the outward unit normal, AL = EL/6 (interior) or RSIDO(3)/6 (boundary)
+  unsigned off[3][2];  // per edge: tile offsets of the source's rows at points k and k+1
   int bside[3];  // boundary side index of each wall edge (kind 3), else -1
-  ElemEdge<T> edge[3];
   int flags;  // bits [0,3): DG node i sits on an inflow-side node (INFLOW);
-              // bits [3,6): edge k is a wall side; bits [6,9): edge k carries
-              // the element-centric flux (interior or outflow side); bit 9:
-              // all three edges are interior sides
+              // bits [3,6): edge k is a wall side; bits [6,9): edge k is an
+              // inflow side
   int wslot;  // wall element slot (ALPHA < 1: the deferred updates), else -1
-  unsigned own01;  // tile offsets (chunk 0) of the element's own rows 0 and 1 (16 bits each)
-  unsigned own2;   // ... and row 2
 };
-constexpr int FLAG_FLUX0 = 1 << 6;      // FLAG_FLUX0 << k: edge k carries the element-centric flux
-constexpr int FLAG_INTERIOR = 1 << 9;  // all three edges interior
-static_assert(sizeof(ElemRec<float>) == 176 && sizeof(ElemRec<double>) == 336, "record layout");
-// values of the leading part a halo element needs (gx .. mu)
+constexpr int FLAG_INFLOW_EDGE0 = 1 << 6;  // FLAG_INFLOW_EDGE0 << k: edge k is an inflow side
+static_assert(sizeof(ElemRec<float>) == 320 && sizeof(ElemRec<double>) == 320, "record layout");
+// coefficients of the leading part a halo element needs (gx .. mu)
 constexpr int REC_HEAD_VALUES = 21;
 
 // One type-4 wall side for the wall-flux kernel (FLUCON2).
