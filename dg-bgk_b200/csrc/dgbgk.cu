@@ -227,6 +227,21 @@ template <class T> void set_groups(CaseDev<T>& k, int nvt, int t, bool halve) {
   k.ngrp = k.nreg + m;
 }
 
+// Tiles per sweep work unit of a case alone on `grid` resident CTAs: three
+// units per CTA, rounded up, in equal groups (and set_groups' tail).  Fewer
+// leave CTAs without work behind the blocks with walls, whose tiles take up to
+// twice as long; more pay the unit prologue (about a third of a tile) more
+// often.  Measured, FP32 sweep in us at 1, 2, 3, 4, 6, 8 tiles a unit: 100x100
+// channel at 16x32 velocities (16.9 tiles per CTA) 102, 90, 87, 85, 84, 91;
+// 93x47 at 20x20, ALPHA 0.9 (6.0) 58, 55, 57, 60, 64, 69; 61x37 at 11x37
+// (3.1) 37, 38, 45, 38, 49, 55; 200x100 at 24x48 (75.6) 404, 338, 319, 309,
+// 299, 295, and 290 at 12.
+inline int tiles_per_unit_alone(long total_tiles, int grid, int nvt) {
+  const int t = (int)std::min<long>(16, (total_tiles + 3L * grid - 1) / (3L * grid));
+  const int ng = (nvt + t - 1) / t;
+  return (nvt + ng - 1) / ng;
+}
+
 // Uploads the case table and picks the launch shapes.  Moments: per-warp
 // rings of R-row stages; picks (R, warps per CTA, ring stages) with the most
 // resident warps per SM (shared memory and registers), then the most rows in
@@ -300,7 +315,9 @@ int build_launch_set(LaunchSet<T>& L, const std::vector<CaseDev<T>>& cs, int eb,
   }
   CK(cudaMemcpyAsync(L.d_cases, cs.data(), n * sizeof(CaseDev<T>), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(L.d_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-  CK(cudaMemsetAsync(L.d_ctl, 0, sizeof(BatchCtl), st));
+  BatchCtl ctl{};
+  for (int j = 0; j < EXP_TAB; ++j) ctl.etab[j] = std::exp2((double)j / EXP_TAB);
+  CK(cudaMemcpyAsync(L.d_ctl, &ctl, sizeof(BatchCtl), cudaMemcpyHostToDevice, st));
   L.n = n;
   L.one = one;
   L.one_case = one ? cs[0] : CaseDev<T>{};
@@ -469,13 +486,14 @@ template <class T> struct Impl : ImplBase {
   // device arrays
   T* f[2] = {nullptr, nullptr};
   ElemRec<T>* rec = nullptr;
-  int *halo_off = nullptr, *halo_list = nullptr;
+  int* halo = nullptr;  // [nblocks][hp]
+  int hp = 0;
   T *cmax = nullptr, *cmin = nullptr;
   T* tabs = nullptr;  // moment tables [MOM_TABS][Vp]
   double *nraw = nullptr, *disux = nullptr, *disuy = nullptr, *disps = nullptr, *mu = nullptr;
   T* swtab = nullptr;  // [NTAB][Vp] the sweep's velocity tables (cx, cy, NFINF, FP64: |c|^2)
   double *cxD = nullptr, *cyD = nullptr, *wjf = nullptr;
-  T *bTw = nullptr, *bUw = nullptr, *bEta = nullptr;
+  T* bwall = nullptr;  // [B][4] wall records
   double* bEtaD = nullptr;
   WallSide* walls = nullptr;
   int *node_off = nullptr, *node_dg = nullptr;
@@ -491,6 +509,7 @@ template <class T> struct Impl : ImplBase {
   int *rside = nullptr, *rf_i = nullptr, *welem = nullptr, *spec_par = nullptr, *spec_seq_off = nullptr,
       *spec_seq = nullptr;
   T *rf_z = nullptr, *wd = nullptr;
+  unsigned* rf_bits = nullptr;
   // extrapolation snapshots [snap_cap][3E*Vp] (slots 0 .. snap_n - 1 taken)
   // and the Gram / coefficient buffers
   T* snaps = nullptr;
@@ -515,8 +534,7 @@ template <class T> struct Impl : ImplBase {
     dfree(f[1]);
     dfree(rec);
     dfree(tabs);
-    dfree(halo_off);
-    dfree(halo_list);
+    dfree(halo);
     dfree(cmax);
     dfree(cmin);
     dfree(nraw);
@@ -528,9 +546,7 @@ template <class T> struct Impl : ImplBase {
     dfree(cxD);
     dfree(cyD);
     dfree(wjf);
-    dfree(bTw);
-    dfree(bUw);
-    dfree(bEta);
+    dfree(bwall);
     dfree(bEtaD);
     dfree(walls);
     dfree(node_off);
@@ -543,6 +559,7 @@ template <class T> struct Impl : ImplBase {
     dfree(rside);
     dfree(rf_i);
     dfree(rf_z);
+    dfree(rf_bits);
     dfree(welem);
     dfree(wd);
     dfree(spec_par);
@@ -613,11 +630,15 @@ template <class T> struct Impl : ImplBase {
       tb[4 * (size_t)Vp + v] = (T)(pl.wjf[v] * pl.cy[v]);
     }
     TRY(upload(&tabs, tb, st));
-    std::vector<T> tw(pl.bTw.begin(), pl.bTw.end()), uw(pl.bUw.begin(), pl.bUw.end()),
-        z(std::max(pl.B, 1), (T)0);
-    TRY(upload(&bTw, tw, st));
-    TRY(upload(&bUw, uw, st));
-    TRY(upload(&bEta, z, st));
+    // wall records: velocity, exponent coefficient -1/(2 R T_w) (FP32 with
+    // log2(e), for the SFU's 2^x), ALPHA*ETA (the wall kernel's)
+    std::vector<T> wl(4 * (size_t)std::max(pl.B, 1), (T)0);
+    for (int b = 0; b < pl.B; ++b) {
+      wl[4 * (size_t)b] = (T)pl.bUw[2 * b];
+      wl[4 * (size_t)b + 1] = (T)pl.bUw[2 * b + 1];
+      wl[4 * (size_t)b + 2] = (T)(-(sizeof(T) == 4 ? LOG2E_D : 1.0) / (2.0 * pl.rgas * pl.bTw[b]));
+    }
+    TRY(upload(&bwall, wl, st));
     std::vector<double> zd(std::max(pl.B, 1), 0.0);
     TRY(upload(&bEtaD, zd, st));
     TRY(upload(&walls, pl.walls, st));
@@ -630,6 +651,13 @@ template <class T> struct Impl : ImplBase {
       TRY(upload(&rside, pl.rside, st));
       TRY(upload(&rf_i, pl.rf_i, st));
       TRY(upload(&rf_z, rz, st));
+      const size_t nw = (size_t)Vp / 32;
+      std::vector<unsigned> bits(std::max<size_t>(pl.B * nw, 1), 0u);
+      for (int b = 0; b < pl.B; ++b)
+        if (pl.rside[b] >= 0)
+          for (int v = 0; v < pl.V; ++v)
+            if (pl.rf_i[((size_t)pl.rside[b] * pl.V + v) * 2] >= 0) bits[b * nw + v / 32] |= 1u << (v % 32);
+      TRY(upload(&rf_bits, bits, st));
       TRY(upload(&welem, pl.welem, st));
       // deferred wall values: IMMAT = 1 DELUN without the specular part;
       // IMMAT = 0 RHS*DTE and COLL*DTE (two halves), whose CMMINC residual
@@ -645,7 +673,7 @@ template <class T> struct Impl : ImplBase {
     std::memset(hctrl, 0, 3 * sizeof(Ctrl));
     CK(cudaMemcpyAsync(ctrl, hctrl, sizeof(Ctrl), cudaMemcpyHostToDevice, st));
     TRY(ensure_hist(1024));
-    TRY(set_tile(tile_elems, 8));
+    TRY(set_tile(tile_elems));
     CK(cudaStreamSynchronize(st));
     return 0;
   }
@@ -655,16 +683,14 @@ template <class T> struct Impl : ImplBase {
     hc.f[0] = f[0];
     hc.f[1] = f[1];
     hc.rec = rec;
-    hc.halo_off = halo_off;
-    hc.halo_list = halo_list;
+    hc.halo = halo;
+    hc.hp = hp;
     hc.swtab = swtab;
     hc.cx = swtab;
     hc.cy = swtab + Vp;
     hc.nfinf = swtab + 2 * (size_t)Vp;
     hc.tabs = tabs;
-    hc.bTw = bTw;
-    hc.bUw = bUw;
-    hc.bEta = bEta;
+    hc.bwall = bwall;
     hc.bEtaD = bEtaD;
     hc.cxD = cxD;
     hc.cyD = cyD;
@@ -684,7 +710,6 @@ template <class T> struct Impl : ImplBase {
     hc.MM = pl.M / 6.022e26;
     hc.sigt = 3.1416 * pl.d * pl.d;
     hc.alpha = (T)pl.alpha;
-    hc.rgas = (T)pl.rgas;
     hc.E = pl.E;
     hc.V = pl.V;
     hc.Vp = Vp;
@@ -700,6 +725,8 @@ template <class T> struct Impl : ImplBase {
     hc.rside = rside;
     hc.rf_i = rf_i;
     hc.rf_z = rf_z;
+    hc.rf_bits = rf_bits;
+    hc.rf_words = Vp / 32;
     hc.welem = welem;
     hc.wd = wd;
     hc.spec_par = spec_par;
@@ -716,15 +743,14 @@ template <class T> struct Impl : ImplBase {
     return 0;
   }
 
-  // Sweep tile: EB elements per CTA (TPE*EB threads) x one 64-byte velocity
-  // segment; `upc` work units per resident CTA picks the tiles per unit.
-  int set_tile(int tile_elems, int upc) {
+  // Sweep tile: EB elements per CTA x one 128-byte velocity segment.
+  int set_tile(int tile_elems) {
     int eb = tile_elems > 0 ? tile_elems : default_eb();
     if (eb != 64 && eb != 128) {
       set_error("tile_elems must be 64 or 128");
       return DGBGK_EINVAL;
     }
-    if (pl.EB != eb || halo_off == nullptr) {
+    if (pl.EB != eb || halo == nullptr) {
       build_blocks(pl, eb);
       if (eb == 128 && SweepGeo<T>::smem(eb, pl.max_halo, 1) > SWEEP_SMEM_MAX) {
         // a halo too wide for this tile (an element order without locality):
@@ -732,11 +758,16 @@ template <class T> struct Impl : ImplBase {
         eb = 64;
         build_blocks(pl, eb);
       }
-      dfree(halo_off);
-      dfree(halo_list);
+      dfree(halo);
       dfree(rec);
-      TRY(upload(&halo_off, pl.halo_off, st));
-      TRY(upload(&halo_list, pl.halo_list, st));
+      hp = std::max(pl.max_halo, 1) + 1;
+      std::vector<int> hal((size_t)pl.nblocks * hp, 0);
+      for (int b = 0; b < pl.nblocks; ++b) {
+        hal[(size_t)b * hp] = pl.halo_off[b + 1] - pl.halo_off[b];
+        std::copy(pl.halo_list.begin() + pl.halo_off[b], pl.halo_list.begin() + pl.halo_off[b + 1],
+                  hal.begin() + (size_t)b * hp + 1);
+      }
+      TRY(upload(&halo, hal, st));
       // element records: geometry, mass matrix and edges (the node
       // parameters are filled by the moment kernel before every sweep)
       std::vector<ElemRec<T>> r(pl.E);
@@ -777,7 +808,7 @@ template <class T> struct Impl : ImplBase {
       set_error("sweep kernel does not fit on an SM with this tile");
       return DGBGK_EUNSUP;
     }
-    tpu = tiles_per_unit((long)pl.nblocks * nvt(), sps * nsm, upc, nvt());
+    tpu = tiles_per_unit_alone((long)pl.nblocks * nvt(), sps * nsm, nvt());
     return refresh();
   }
 
@@ -790,7 +821,7 @@ template <class T> struct Impl : ImplBase {
     TRY(dalloc(&hist_l2, n));
     TRY(dalloc(&hist_dt, n));
     hist_cap = n;
-    if (halo_off) TRY(refresh());
+    if (halo) TRY(refresh());
     return 0;
   }
 
@@ -1748,7 +1779,7 @@ template <class T> struct BatchImpl : BatchBase {
   // from the whole batch's work (about u units per resident CTA).
   int configure(int e, int u) {
     for (auto* c : cs) {
-      TRY(c->set_tile(e, u));
+      TRY(c->set_tile(e));
       CK(cudaStreamSynchronize(c->st));
       // a case whose halo does not fit a 128-element tile: 64 for all
       if (c->pl.EB != e) return configure(c->pl.EB, u);

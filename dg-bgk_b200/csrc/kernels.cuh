@@ -38,23 +38,6 @@ constexpr double TINY_D = 1e-20;
 constexpr double LOG2E_D = 1.4426950408889634;  // log2(e)
 constexpr unsigned WAIT_TRIES = 1u << 22;  // x ~256 ns sleep: ~1 s
 
-// e^x in FP32 for the FP32 sweep: t = x*log2(e) is formed with its rounding
-// error recovered by an FMA (t_lo = fma(x, L, -t) + x*(log2(e) - L)), 2^t
-// comes from the SFU's ex2.approx and the low part enters to first order,
-// 2^t_lo ~ 1 + t_lo*ln2.  Relative error ~2.5e-7 (the SFU's 2^-22 bound).
-// Arguments here are finite and <= 0 (x = -BETA2*|c-u|^2).
-__device__ __forceinline__ float exp_sfu(float x) {
-  const float L = 1.44269502163f, Llo = 1.92596303e-8f;
-  const float t = x * L;
-  const float tl = fmaf(x, L, -t) + x * Llo;
-  float p;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p) : "f"(t));
-  return fmaf(p, tl * 0.693147181f, p);
-}
-template <class T> __device__ __forceinline__ T dexp(T x);
-template <> __device__ __forceinline__ double dexp<double>(double x) { return exp(x); }
-template <> __device__ __forceinline__ float dexp<float>(float x) { return exp_sfu(x); }
-
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -118,16 +101,15 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 template <class T> struct alignas(64) CaseDev {
   T* f[2];            // state, ping-pong; Ctrl::cur is the current one
   ElemRec<T>* rec;
-  const int* halo_off;
-  const int* halo_list;
+  const int* halo;  // [nblocks][hp]: the block's halo count and its halo elements
+  int hp;           // pitch: at least one more than the largest halo
   const T* swtab;  // [NTAB][Vp] sweep tables cx, cy, NFINF (, |c|^2), zero past V
   const T* cx;     // rows 0, 1, 2 of swtab
   const T* cy;
   const T* nfinf;
   const T* tabs;   // [MOM_TABS][Vp] moment tables: cx, cy, w = WEIGHT*JAC*FRAC, w*cx, w*cy; zero past V
-  const T* bTw;    // per boundary side: wall temperature, wall velocity (x, y), ETA
-  const T* bUw;
-  T* bEta;
+  T* bwall;        // per boundary side [4]: wall velocity (x, y), the wall Maxwellian's exponent coefficient
+                   // -1/(2 R T_w) (FP32: times log2(e)), ALPHA*ETA (written by the wall kernel)
   double* bEtaD;
   const double* cxD;  // [V] FP64 velocity tables for FLUCON2
   const double* cyD;
@@ -145,7 +127,7 @@ template <class T> struct alignas(64) CaseDev {
   double* hist_dt;
   Ctrl* ctrl;
   double MM, sigt;  // M/NA, PI*d*d
-  T alpha, rgas;
+  T alpha;
   int E, V, Vp, nblocks, nvt;
   int tpu, nreg, ngrp, halve;  // velocity-tile groups of the sweep's units (sweep_group)
   int nwall;          // FLUCON2 wall sides
@@ -157,6 +139,8 @@ template <class T> struct alignas(64) CaseDev {
   const int* rside;         // [B] reflection-table row, -1 off the walls
   const int* rf_i;          // [rows][V][2] mirrored grid velocities I1, I2; -1 where TEST >= 0
   const T* rf_z;            // [rows][V][2] ZD1, ZD2
+  const unsigned* rf_bits;  // [B][rf_words] bit v: rf_i >= 0 there
+  int rf_words;             // Vp/32
   const int* welem;         // [slots] wall elements (plan order)
   T* wd;                    // deferred values: IMMAT = 1 [slots][3][Vp] DELUN without the specular part;
                             // IMMAT = 0 [2][slots][3][Vp] RHS*DTE without it, COLL*DTE
@@ -735,16 +719,19 @@ template <class T> __global__ void __launch_bounds__(WALL_THREADS) k_wall(BatchA
     for (int k = 0; k < WALL_THREADS / 32; ++k) t += part[k];
     const double eta = t / ws.sumbottom;
     C.bEtaD[ws.bside] = eta;
-    C.bEta[ws.bside] = (T)eta;
+    C.bwall[4 * (size_t)ws.bside + 3] = (T)((double)C.alpha * eta);
   }
 }
 
 // -------------------------------------------------------------- sweep ----
 // DTE = min(CSAFE/maxMU, DTEc)  (src/alotim2.f90:10-15, src/advnce.f90:258-262)
 __device__ __forceinline__ double step_dt(const Ctrl* c) {
-  const double mx = c->maxmu;
+  const double mx = c->maxmu, dtc = c->dtc;
+  // well inside the collision limit the Courant limit is the smaller one: no
+  // division in front of the kernel's first unit
+  if (mx > 0.0 && mx * dtc < 0.899 && dtc < 1000000.0) return dtc;
   const double dtb = (mx > 0.0) ? 0.9 * (1.0 / mx) : 1000000.0;
-  return fmin(dtb, c->dtc);
+  return fmin(dtb, dtc);
 }
 
 // Sweep geometry.  LPE = 8 lanes share an element, each with one 16-byte
@@ -935,13 +922,12 @@ __device__ __forceinline__ void sweep_p1(const ElemRec<T>& r, const double* etab
   for (int i = 0; i < 3; ++i) vst<T>(rows + i * ROW_BYTES, f[i]);
 }
 
-// The step's factors of a staged record, applied to its 16-byte word k (two
-// coefficients) by the thread that copied it: 0.5*DTE to the gradients
-// (words 0 to 2), -DTE/6 to MU (words 9, 10), DTE to MT and MM (words 11 to
-// 13); the other words are left alone.
-template <class T> __device__ __forceinline__ void sweep_scale(unsigned char* word, int k, T dth, T mdt6, T dt) {
-  if (k > 13 || (k > 2 && k < 9)) return;
-  const T s = k < 3 ? dth : k < 11 ? mdt6 : dt;
+// The step's factors of a staged record, applied to its 16-byte words (two
+// coefficients) by the lane that copied them: 0.5*DTE to the gradients (words
+// 0 to 2), -DTE/6 to MU (words 9, 10), DTE to MT and MM (words 11 to 13); the
+// other words are left alone.
+__device__ __forceinline__ bool sweep_scaled(int word) { return word < 3 || (word >= 9 && word < 14); }
+template <class T> __device__ __forceinline__ void sweep_scale(unsigned char* word, T s) {
   typename Pair<T>::vec v = vld<T>(word);
 #pragma unroll
   for (int h = 0; h < SweepGeo<T>::NP; ++h) pset(v, h, pmul(pget(v, h), pdup(s)));
@@ -1035,10 +1021,9 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
   __shared__ double red_m[NW], red_s[NW];
   // FP64: the 2^(j/64) table of the NFO exp (one entry for FP32, unused)
   __shared__ double etab[sizeof(T) == 8 ? EXP_TAB : 1];
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int sub = (tid & 31) / G::LPE, l8 = tid & (G::LPE - 1);
-  if (sizeof(T) == 8)
-    for (int i = tid; i < EXP_TAB; i += NT) etab[i] = exp2((double)i / EXP_TAB);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int sub = lane / G::LPE, l8 = tid & (G::LPE - 1);
+  if (sizeof(T) == 8 && tid < EXP_TAB) etab[tid] = a.ctl->etab[tid];
   const unsigned tile_bytes = G::tile_bytes(EB, a.max_halo);
   const bool two = a.sweep_bufs > 1;
   unsigned char* const recs = sm_raw + (two ? 2 : 1) * tile_bytes;  // pitch RP
@@ -1056,21 +1041,40 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
   // residual partials of the thread's values: a single case adds them to its
   // control block once per CTA (after the last unit), a batch once per unit
   double rmax = 0.0, rsq = 0.0;
+  // a single case's control values, the same for every unit
+  int cur = 0;
+  double dtd = 0.0;
+  bool active = false;
+  auto control = [&](const Ctrl* ctl) {
+    active = !ctl->done;
+    cur = ctl->cur;
+    dtd = step_dt(ctl);
+  };
+  if (ONE) control(one.ctrl);
   // the unit after this one, drawn ahead so the atomic's latency is hidden
   int next = (tid == 0 && unit < total_units) ? (int)gridDim.x + atomicAdd(&a.ctl->sweep_next, 1) : 0;
   while (unit < total_units) {
     c = ONE ? 0 : find_case(a.unit_off, a.ncases, unit);
     const CaseDev<T>& C = ONE ? one : a.cases[c];
-    const bool active = !C.ctrl->done;  // the same for every thread
+    if (!ONE) control(C.ctrl);  // the same for every thread
     if (active) {
       const int lu = unit - (ONE ? 0 : a.unit_off[c]);
       const int b = lu % C.nblocks, vg = lu / C.nblocks;
       const int e0 = b * EB, nb = min(EB, C.E - e0);
-      const int h0 = C.halo_off[b], nh = C.halo_off[b + 1] - h0;
+      // the halo: its count, and the first entries each thread needs before
+      // the count is there (two loads in flight instead of one after the
+      // other; entries past the count are valid element numbers)
+      const int* __restrict__ hrow = C.halo + (size_t)b * C.hp;
+      const int nh = hrow[0];
+      constexpr int NHW = NT / 16;  // half-warps
+      constexpr int PRE_H = 2, PRE_R = 2;
+      int idh[PRE_H], idr[PRE_R];
+#pragma unroll
+      for (int x = 0; x < PRE_H; ++x) idh[x] = hrow[min(1 + (tid >> 4) + x * NHW, C.hp - 1)];
+#pragma unroll
+      for (int x = 0; x < PRE_R; ++x) idr[x] = hrow[min(1 + j0 + x * NW * EPW, C.hp - 1)];
       int vt0, ntl;
       sweep_group(C, vg, vt0, ntl);
-      const int cur = C.ctrl->cur;
-      const double dtd = step_dt(C.ctrl);
       const T dt = (T)dtd;
       const T* __restrict__ fo = C.f[cur];
       T* __restrict__ fnw = C.f[cur ^ 1];
@@ -1082,7 +1086,8 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
       // them in phase 1 (so a lane waits for its own copies only): the lane
       // group's block elements (past the end of the mesh the last one again)
       // and its share of the halo.
-      auto issue = [&](int vt, unsigned char* buf, const int* list) {
+      auto issue = [&](int vt, unsigned char* buf, auto first) {
+        constexpr bool FIRST = decltype(first)::value;  // the unit's first tile: hl is not there yet
         const unsigned char* src = reinterpret_cast<const unsigned char*>(fo + (size_t)vt * VT + l8 * W);
         auto copy3 = [&](int slot, unsigned row) {
 #pragma unroll
@@ -1091,21 +1096,35 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
         };
 #pragma unroll
         for (int it = 0; it < ITERS; ++it) copy3(j0 + it * NW * EPW, own[it]);
+        if constexpr (FIRST) {
+#pragma unroll
+          for (int x = 0; x < PRE_R; ++x)
+            if (j0 + x * NW * EPW < nh) copy3(EB + j0 + x * NW * EPW, 3u * (unsigned)idr[x]);
+        }
 #pragma unroll 1
-        for (int h = j0; h < nh; h += NW * EPW) copy3(EB + h, 3u * (unsigned)list[h]);
+        for (int h = j0 + (FIRST ? PRE_R : 0) * NW * EPW; h < nh; h += NW * EPW)
+          copy3(EB + h, 3u * (unsigned)(FIRST ? hrow[1 + h] : hl[h]));
         cp_async_commit();
       };
-      // unit prologue, all of it asynchronous: the block's element records,
-      // the halo's record heads and the unit's velocities, then the first
-      // tile's rows; the records are scaled by the step's factors as they
-      // land, by the threads that copied them
+      // unit prologue, all of it asynchronous: the block's element records
+      // (a warp per record, a lane per word), the halo's record heads (a
+      // half-warp each) and the unit's velocities, then the first tile's
+      // rows; the records are scaled by the step's factors as they land, by
+      // the lanes that copied them
       {
-        const int* __restrict__ hlist = C.halo_list + h0;
         const uint4* src = reinterpret_cast<const uint4*>(C.rec + e0);
-        for (int w = tid; w < nb * RW; w += NT) cp_async16(recs + w / RW * RP + 16 * (w % RW), src + w);
-        for (int w = tid; w < nh * HW; w += NT) {
-          const int s = w / HW, k = w - s * HW;
-          cp_async16(hrec + (size_t)s * HR + 16 * k, reinterpret_cast<const uint4*>(C.rec + hlist[s]) + k);
+        if (lane < RW)
+#pragma unroll 4
+          for (int j = warp; j < nb; j += NW) cp_async16(recs + j * RP + 16 * lane, src + j * RW + lane);
+        const int hw = tid & 15, hs = tid >> 4;
+        if (hw < HW) {
+#pragma unroll
+          for (int x = 0; x < PRE_H; ++x)
+            if (hs + x * NHW < nh)
+              cp_async16(hrec + (hs + x * NHW) * HR + 16 * hw, reinterpret_cast<const uint4*>(C.rec + idh[x]) + hw);
+#pragma unroll 1
+          for (int s = hs + PRE_H * NHW; s < nh; s += NHW)
+            cp_async16(hrec + s * HR + 16 * hw, reinterpret_cast<const uint4*>(C.rec + hrow[1 + s]) + hw);
         }
         for (int w = tid; w < G::NVT * ntl * G::LPE; w += NT) {
           const int t = w / (ntl * G::LPE), x = w - t * ntl * G::LPE;
@@ -1113,17 +1132,27 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
                      C.swtab + (size_t)(t == 2 ? 3 : t) * C.Vp + (size_t)vt0 * VT + (size_t)x * W);
         }
         cp_async_commit();
-        issue(vt0, sm_raw + (two ? (gk & 1) * tile_bytes : 0), hlist);
-        for (int s = tid; s < nh; s += NT) hl[s] = hlist[s];
+        issue(vt0, sm_raw + (two ? (gk & 1) * tile_bytes : 0), std::true_type());
+        for (int s = tid; s < nh; s += NT) hl[s] = hrow[1 + s];
         cp_async_wait<1>();
         const T dth = (T)(0.5 * dtd), mdt6 = (T)(-0.5 * dtd / 3.0);
-        for (int w = tid; w < nb * RW; w += NT)
-          sweep_scale<T>(recs + w / RW * RP + 16 * (w % RW), w % RW, dth, mdt6, dt);
-        for (int w = tid; w < nh * HW; w += NT) {
-          const int s = w / HW, k = w - s * HW;
-          sweep_scale<T>(hrec + (size_t)s * HR + 16 * k, k, dth, mdt6, dt);
+        if (sweep_scaled(lane)) {
+          const T sc = lane < 3 ? dth : lane < 11 ? mdt6 : dt;
+#pragma unroll 4
+          for (int j = warp; j < nb; j += NW) sweep_scale<T>(recs + j * RP + 16 * lane, sc);
+        }
+        if (hw < HW && sweep_scaled(hw)) {
+          const T sc = hw < 3 ? dth : mdt6;
+          for (int s = hs; s < nh; s += NHW) sweep_scale<T>(hrec + s * HR + 16 * hw, sc);
         }
         __syncthreads();
+        // the wall records of the lane group's elements into L1
+        if (l8 < 3)
+#pragma unroll
+          for (int it = 0; it < ITERS; ++it) {
+            const int bs = reinterpret_cast<const ElemRec<T>*>(recs + min(j0 + it * NW * EPW, nb - 1) * RP)->bside[l8];
+            if (bs >= 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(C.bwall + 4 * (size_t)bs));
+          }
       }
 
       for (int k = 0; k < ntl; ++k, ++gk) {
@@ -1149,7 +1178,7 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
                       tl8 + tile_row(3 * (EB + h)), cxv, cyv, c2v, qh, uh);
         }
         __syncthreads();
-        if (two && k + 1 < ntl) issue(vt0 + k + 1, sm_raw + ((gk + 1) & 1) * tile_bytes, hl);
+        if (two && k + 1 < ntl) issue(vt0 + k + 1, sm_raw + ((gk + 1) & 1) * tile_bytes, std::false_type());
 
         // ---- phase 2: the update of the lane group's block elements
         const bool whole = (vt0 + k + 1) * VT <= C.V;  // no velocity of the tile past V
@@ -1202,19 +1231,81 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
               }
             }
           }
-          // GETINC / CMMINC, ADTHEM (f >= 0), INFLOW and the residual.  An
-          // element away from walls and inflow at velocities below V takes
-          // the plain form; dmask (ALPHA < 1): bit 3*w + i marks node i at
-          // velocity v0 + w as deferred (its update gets the specular part in
-          // k_wspec).
+          // ALPHA < 1: bit 3*w + i marks node i at velocity v0 + w as deferred
+          // (its update gets the specular part in k_wspec)
           unsigned dmask = 0u;
+          if (flags & 0x1f8) {
+            // Wall sides: molecules leaving the wall (src/getbou.f90:189-255)
+            // carry the diffuse part ALPHA*ETA*Mw here, the specular part
+            // (1-ALPHA)*Rf in k_wspec; inflow sides: no flux.  The edge loop
+            // has added the element's own values where AL*SC > 0 and nothing
+            // elsewhere: the difference is added.
+            const bool spec = C.spec != 0;
+            // one edge at a time by its number, so that lanes whose wall is a
+            // different local edge go together (and the code is there once)
+            for (int em = ((flags >> 3) | (flags >> 6)) & 7; em != 0; em &= em - 1) {
+              const int k2 = __ffs(em) - 1;
+              const bool inflow = (flags & (FLAG_INFLOW_EDGE0 << k2)) != 0;
+              const T wnx = pval(r.en[k2][0]), wny = pval(r.en[k2][1]);  // -AL*n of the side
+              const int bs = inflow ? 0 : r.bside[k2];
+              const VecT* wr = reinterpret_cast<const VecT*>(C.bwall + 4 * (size_t)bs);
+              T w4[4];
+              if constexpr (sizeof(T) == 4) {
+                const VecT a4 = wr[0];
+                w4[0] = a4.x, w4[1] = a4.y, w4[2] = a4.z, w4[3] = a4.w;
+              } else {
+                const VecT a2 = wr[0], b2 = wr[1];
+                w4[0] = a2.x, w4[1] = a2.y, w4[2] = b2.x, w4[3] = b2.y;
+              }
+              // with the specular part, the wall branch is taken where the
+              // host's FP64 TEST < 0 (the items of k_wspec are built from
+              // it): one bit per velocity
+              const bool sp = spec && !inflow;
+              const unsigned tb = sp ? C.rf_bits[(size_t)bs * C.rf_words + (v0 >> 5)] >> (v0 & 31) : 0u;
+              const unsigned nodes = k2 == 0 ? 3u : k2 == 1 ? 6u : 5u;
+              auto wall = [&](int w, T cx, T cy, T gp, T gq, T& rp, T& rq) {
+                const T ms = wnx * cx + wny * cy;  // -AL*SC, as in the edge loop
+                const bool mine = sp ? !((tb >> w) & 1u) : ms <= (T)0;
+                T up = gp, uq = gq;
+                if (inflow) {
+                  up = uq = (T)0;
+                } else if (!mine) {
+                  const T dx = cx - w4[0], dy = cy - w4[1];
+                  up = uq = w4[3] * nfo_exp<T>(w4[2] * (dx * dx + dy * dy), etab);
+                  if (sp) dmask |= nodes << (3 * w);
+                }
+                if (ms < (T)0) {
+                  up -= gp;
+                  uq -= gq;
+                }
+                rp = ms * ((T)2 * up + uq);
+                rq = ms * (up + (T)2 * uq);
+              };
+#pragma unroll
+              for (int h = 0; h < NP; ++h) {
+                const P cx = pget(cxv, h), cy = pget(cyv, h);
+                const P gp = k2 == 0 ? g[0][h] : k2 == 1 ? g[1][h] : g[2][h];
+                const P gq = k2 == 0 ? g[1][h] : k2 == 1 ? g[2][h] : g[0][h];
+                P rp, rq;
+                wall(2 * h, cx.x, cy.x, gp.x, gq.x, rp.x, rq.x);
+                wall(2 * h + 1, cx.y, cy.y, gp.y, gq.y, rp.y, rq.y);
+                const P z = pdup((T)0);
+                rhs[0][h] = padd(rhs[0][h], k2 == 0 ? rp : k2 == 2 ? rq : z);
+                rhs[1][h] = padd(rhs[1][h], k2 == 1 ? rp : k2 == 0 ? rq : z);
+                rhs[2][h] = padd(rhs[2][h], k2 == 2 ? rp : k2 == 1 ? rq : z);
+              }
+            }
+          }
+          // GETINC / CMMINC, ADTHEM (f >= 0), INFLOW and the residual.  Plain:
+          // every value of the lane is updated and counted; otherwise those
+          // past V (which stay zero), of nodes INFLOW resets and deferred
+          // ones are left out of the residual.
           P sq = pdup((T)0);
           VecT out[3];
           auto finish = [&](auto plain) {
             constexpr bool PLAIN = decltype(plain)::value;
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-              const bool counts = PLAIN || !(flags & (1 << i));  // not reset by INFLOW
               T cmx = (T)0, cmn = (T)0;
               if (IMMAT == 0) {
                 cmx = C.cmax[3 * (e0 + min(j, nb - 1)) + i];
@@ -1245,92 +1336,32 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
                 }
                 fn.x = fmax(fn.x, (T)0);
                 fn.y = fmax(fn.y, (T)0);
-                if constexpr (PLAIN) {
-                  rmt = fmax(rmt, fmax(rr.x, rr.y));
-                  sq = pfma(ch, ch, sq);
-                } else {
-                  auto value = [&](int w, T dd, T rrr, T chh, T xx, T cc, T& ff, T& s) {
-                    if (v0 + w >= C.V) {
-                      ff = (T)0;
-                      return;
-                    }
-                    if ((dmask >> (3 * w + i)) & 1u) {
-                      // deferred: k_wspec adds the specular part, clips and
-                      // counts the residual
-                      if (live) {
-                        const size_t o = ((size_t)r.wslot * 3 + i) * C.Vp + v0 + w;
-                        if (IMMAT == 1) {
-                          C.wd[o] = dd;
-                        } else {
-                          C.wd[o] = xx * dt;
-                          C.wd[(size_t)C.n_spec_slots * 3 * C.Vp + o] = cc;
-                        }
-                      }
-                    } else {
-                      rmt = fmax(rmt, rrr);
-                      if (counts) s += chh * chh;
+                if constexpr (!PLAIN) {
+                  auto value = [&](int w, T dd, T xx, T cc, T& rrr, T& chh, T& ff) {
+                    const bool past = v0 + w >= C.V, def = ((dmask >> (3 * w + i)) & 1u) != 0 && !past;
+                    if (past) ff = (T)0;
+                    if (past || def) rrr = (T)0;
+                    if (past || def || (flags & (1 << i))) chh = (T)0;
+                    if (def && live) {
+                      // k_wspec adds the specular part, clips and counts the
+                      // residual
+                      const size_t o = ((size_t)r.wslot * 3 + i) * C.Vp + v0 + w;
+                      C.wd[o] = IMMAT == 1 ? dd : xx * dt;
+                      if (IMMAT == 0) C.wd[(size_t)C.n_spec_slots * 3 * C.Vp + o] = cc;
                     }
                   };
-                  value(2 * h, d.x, rr.x, ch.x, rhs[i][h].x, cdt.x, fn.x, sq.x);
-                  value(2 * h + 1, d.y, rr.y, ch.y, rhs[i][h].y, cdt.y, fn.y, sq.y);
+                  value(2 * h, d.x, rhs[i][h].x, cdt.x, rr.x, ch.x, fn.x);
+                  value(2 * h + 1, d.y, rhs[i][h].y, cdt.y, rr.y, ch.y, fn.y);
                 }
+                rmt = fmax(rmt, fmax(rr.x, rr.y));
+                sq = pfma(ch, ch, sq);
                 pset(out[i], h, fn);
               }
             }
           };
-          if (whole && (flags & 0x1ff) == 0) {
+          if (whole && (flags & 7) == 0 && dmask == 0u) {
             finish(std::true_type());
           } else {
-            // Wall sides: molecules leaving the wall (src/getbou.f90:189-255)
-            // carry the diffuse part ALPHA*ETA*Mw here, the specular part
-            // (1-ALPHA)*Rf in k_wspec; inflow sides: no flux.  The edge loop
-            // has added the element's own values where AL*SC > 0 and nothing
-            // elsewhere: the difference is added.
-            const bool spec = C.spec != 0;
-#pragma unroll
-            for (int k2 = 0; k2 < 3; ++k2) {
-              const bool inflow = (flags & (FLAG_INFLOW_EDGE0 << k2)) != 0;
-              if (!inflow && !(flags & (8 << k2))) continue;
-              const int p = k2, qn = (k2 + 1) % 3;
-              const int bs = inflow ? 0 : r.bside[k2];
-              const T twr = (T)2 * C.rgas * C.bTw[bs];
-              const T uwx = C.bUw[2 * bs], uwy = C.bUw[2 * bs + 1], eta = C.bEta[bs];
-              const T wnx = pval(r.en[k2][0]), wny = pval(r.en[k2][1]);  // -AL*n of the side
-              // with the specular part, the wall branch is taken where the
-              // host's FP64 TEST < 0 (the items of k_wspec are built from it)
-              const int* rfi = spec && !inflow ? C.rf_i + (size_t)C.rside[bs] * C.V * 2 : nullptr;
-              auto wall = [&](int w, T cx, T cy, T gp, T gq, T& rp, T& rq) {
-                const T ms = wnx * cx + wny * cy;  // -AL*SC, as in the edge loop
-                const bool mine = rfi ? !(v0 + w < C.V && rfi[2 * (v0 + w)] >= 0) : ms <= (T)0;
-                T up = gp, uq = gq;
-                if (inflow) {
-                  up = uq = (T)0;
-                } else if (!mine) {
-                  T mw;
-                  if (uwx == (T)0 && uwy == (T)0) {
-                    const T spd = sqrt(cx * cx + cy * cy);
-                    mw = dexp<T>(-(spd * spd) / twr);
-                  } else {
-                    const T dx = cx - uwx, dy = cy - uwy;
-                    mw = dexp<T>(-(dx * dx + dy * dy) / twr);
-                  }
-                  up = uq = C.alpha * (mw * eta);
-                  if (spec) dmask |= ((1u << p) | (1u << qn)) << (3 * w);
-                }
-                if (ms < (T)0) {
-                  up -= gp;
-                  uq -= gq;
-                }
-                rp += ms * ((T)2 * up + uq);
-                rq += ms * (up + (T)2 * uq);
-              };
-#pragma unroll
-              for (int h = 0; h < NP; ++h) {
-                const P cx = pget(cxv, h), cy = pget(cyv, h);
-                wall(2 * h, cx.x, cy.x, g[p][h].x, g[qn][h].x, rhs[p][h].x, rhs[qn][h].x);
-                wall(2 * h + 1, cx.y, cy.y, g[p][h].y, g[qn][h].y, rhs[p][h].y, rhs[qn][h].y);
-              }
-            }
             finish(std::false_type());
             if (flags & 7) {
               const VecT nf = vld<T>(C.nfinf + v0);  // zero past V
@@ -1350,7 +1381,7 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
         rsq += (double)sqt.x + (double)sqt.y;
         if (!two && k + 1 < ntl) {
           __syncthreads();
-          issue(vt0 + k + 1, sm_raw, hl);
+          issue(vt0 + k + 1, sm_raw, std::false_type());
         }
       }
       // a batch: the unit's residual, per warp
@@ -1615,7 +1646,7 @@ __global__ void __launch_bounds__(256) k_shard_fin(const __grid_constant__ CaseD
     const WallSide ws = C.walls[t];
     const double eta = sums2[2 * n3 + t] / ws.sumbottom;
     C.bEtaD[ws.bside] = eta;
-    C.bEta[ws.bside] = (T)eta;
+    C.bwall[4 * (size_t)ws.bside + 3] = (T)((double)C.alpha * eta);
   }
   const double m = warp_max(mu);
   if ((threadIdx.x & 31) == 0 && m > 0.0)

@@ -14,6 +14,8 @@
 #pragma once
 #include <cstdint>
 
+#include "exp_tang.h"
+
 namespace dgbgk {
 
 // A row of a sweep tile in bytes: one velocity segment of a DG node.  The
@@ -128,6 +130,7 @@ struct Ctrl {
 struct BatchCtl {
   int sweep_next;  // sweep work units handed out beyond the first wave (reset by k_resid)
   int pad[15];
+  double etab[EXP_TAB];  // 2^(j/64) of the FP64 sweep's exp
 };
 
 }  // namespace dgbgk
