@@ -223,8 +223,8 @@ __device__ __forceinline__ double sqrt_newton(double x) {
   const float xf = (float)x;
   if (!(xf > 0.f)) return 0.0;
   const double y0 = (double)rsqrt_sfu(xf);
-  const double y1 = y0 * (1.5 - 0.5 * x * y0 * y0);
-  return x * y1;
+  const double t = x * y0;  // sqrt(x) to the seed's accuracy
+  return t * fma(-0.5 * y0, t, 1.5);
 }
 // FP32 sqrt from the SFU (sqrt.approx: relative error ~2^-23; sqrt(0) = 0)
 __device__ __forceinline__ float sqrt_fast(float x) {
@@ -265,9 +265,10 @@ template <> struct RowMath<double> {
       const double dx0 = c.x - ux, dy0 = d.x - uy, dx1 = c.y - ux, dy1 = d.y - uy;
       const double q0 = dx0 * dx0 + dy0 * dy0, q1 = dx1 * dx1 + dy1 * dy1;
       const double a0 = w.x * x.x, a1 = w.y * x.y;
-      sp = fma(0.5 * q0, a0, fma(0.5 * q1, a1, sp));                // src/macros.f90:144-148
+      sp = fma(q0, a0, fma(q1, a1, sp));                            // src/macros.f90:144-148, times 2
       sc = fma(sqrt_newton(q0), a0, fma(sqrt_newton(q1), a1, sc));  // src/compmu.f90:71-74
     }
+    sp *= 0.5;  // (sp starts at zero)
   }
 };
 
@@ -384,14 +385,14 @@ template <> struct ElemMath<float> {
   }
   // pass 2 on packed pairs (c - u as c + (-u))
   static __device__ __forceinline__ void pass2(const float* rows, unsigned pitch, const float* tb, int Vp, int nq,
-                                               int lane, const double (&u)[3][2], double (&s)[3][2]) {
+                                               int lane, const float (&u)[3][2], double (&s)[3][2]) {
     const float4* cx = reinterpret_cast<const float4*>(tb);
     const float4* cy = reinterpret_cast<const float4*>(tb + Vp);
     const float4* wj = reinterpret_cast<const float4*>(tb + 2 * Vp);
     float2 nu[3][2], t[3][2];
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-      const float ux = (float)u[r][0], uy = (float)u[r][1];
+      const float ux = u[r][0], uy = u[r][1];
       nu[r][0] = make_float2(-ux, -ux);
       nu[r][1] = make_float2(-uy, -uy);
       t[r][0] = t[r][1] = make_float2(0.f, 0.f);
@@ -462,10 +463,12 @@ template <> struct ElemMath<double> {
         const double dx0 = c.x - u[r][0], dy0 = d.x - u[r][1], dx1 = c.y - u[r][0], dy1 = d.y - u[r][1];
         const double q0 = dx0 * dx0 + dy0 * dy0, q1 = dx1 * dx1 + dy1 * dy1;
         const double a0 = w.x * x.x, a1 = w.y * x.y;
-        s[r][0] = fma(0.5 * q0, a0, fma(0.5 * q1, a1, s[r][0]));                // src/macros.f90:144-148
+        s[r][0] = fma(q0, a0, fma(q1, a1, s[r][0]));                            // src/macros.f90:144-148, times 2
         s[r][1] = fma(sqrt_newton(q0), a0, fma(sqrt_newton(q1), a1, s[r][1]));  // src/compmu.f90:71-74
       }
     }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) s[r][0] *= 0.5;
   }
 };
 
@@ -521,6 +524,24 @@ template <int L> __device__ __forceinline__ double group_sum(double v) {
 #pragma unroll
   for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+
+// Sums over the warp of K values for each of three rows, row 0's left in
+// lanes 0 to 7, row 1's in 8 to 15, row 2's in 16 to 31: the first two levels
+// of the butterfly hand rows to lane groups, so each of the other three
+// levels moves K values and not 3K (6K exchanges instead of 15K).
+template <int K> __device__ __forceinline__ void row_sums(const double (&v)[3][K], int lane, double (&t)[K]) {
+  const bool hi = (lane & 16) != 0, second = (lane & 24) == 8;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const double x = (hi ? v[2][k] : v[0][k]) + __shfl_xor_sync(0xffffffffu, hi ? v[0][k] : v[2][k], 16);
+    const double y = v[1][k] + __shfl_xor_sync(0xffffffffu, v[1][k], 16);
+    t[k] = (second ? y : x) + __shfl_xor_sync(0xffffffffu, hi || second ? x : y, 8);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < K; ++k) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
 }
 
 // Moment kernel: persistent warps over the flattened row groups of all the
@@ -588,6 +609,20 @@ __global__ void __launch_bounds__(ONE ? 640 : 512, 1)
                 (unsigned long long)__double_as_longlong(m));
     mumax = 0.0;
   };
+  // The lanes of a row's group all hold its sums; lane `kept` of the group
+  // keeps them, and once every lane has a node the per-node epilogue (FP64
+  // divisions, a logarithm, the stores) runs for all of them at once.  A node
+  // at a time it was a third of the warp's instructions.
+  constexpr int KEEP = ELEM ? 8 : L;
+  int kept = 0, knode = -1;
+  double k0 = 0, kux = 0, kuy = 0, ksp = 0, ksc = 0;
+  auto flush_nodes = [&]() {
+    if (knode >= 0)
+      mumax = fmax(mumax, node_epilogue(ONE ? one : a.cases[mu_case], knode, k0, kux, kuy, k0 >= TINY_D ? k0 : 0.0,
+                                        ksp, ksc));
+    knode = -1;
+    kept = 0;
+  };
   int c = 0;
   for (int g = gw; g < total_groups; g += stride) {
     c = ONE ? 0 : find_case(a.grp_off, a.ncases, g);  // warp-uniform
@@ -602,6 +637,7 @@ __global__ void __launch_bounds__(ONE ? 640 : 512, 1)
     parity ^= 1u << s;
     const CaseDev<T>& C = ONE ? one : a.cases[c];
     if (c != mu_case) {
+      flush_nodes();
       flush_mu();
       mu_case = c;
     }
@@ -612,37 +648,30 @@ __global__ void __launch_bounds__(ONE ? 640 : 512, 1)
     // this lane's node and its sums: s0 = n, ux, uy (MACROS pass 1), sp, sc
     // (pass 2: pressure and COMPMU's mean relative speed)
     int node;
-    double s0, ux, uy, nd, sp, sc;
+    double s0, ux, uy, sp, sc;
     if constexpr (ELEM) {
       const T* rows = reinterpret_cast<const T*>(ring + (size_t)s * stage_bytes);
-      double m1[3][3], u[3][2], m2[3][2];
+      double m1[3][3], t1[3], m2[3][2], t2[2];
       ElemMath<T>::template pass1<ONE>(rows, C.rowbytes, tb, C.Vp, nql, lane, m1);
+      row_sums<3>(m1, lane, t1);
+      s0 = t1[0];
+      ux = uy = 0.0;
+      if (s0 >= TINY_D) {  // src/macros.f90:126-134
+        const double inv = 1.0 / s0;
+        ux = t1[1] * inv;
+        uy = t1[2] * inv;
+      }
+      T u[3][2];
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) m1[r][k] = group_sum<32>(m1[r][k]);
-        u[r][0] = u[r][1] = 0.0;
-        if (m1[r][0] >= TINY_D) {  // src/macros.f90:126-134
-          const double inv = 1.0 / m1[r][0];
-          u[r][0] = m1[r][1] * inv;
-          u[r][1] = m1[r][2] * inv;
-        }
+        u[r][0] = __shfl_sync(0xffffffffu, (T)ux, 8 * r);
+        u[r][1] = __shfl_sync(0xffffffffu, (T)uy, 8 * r);
       }
       ElemMath<T>::pass2(rows, C.rowbytes, tb, C.Vp, nql, lane, u, m2);
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        m2[r][0] = group_sum<32>(m2[r][0]);
-        m2[r][1] = group_sum<32>(m2[r][1]);
-      }
-      // lanes 0, 1, 2 write rows 0, 1, 2
-      const int r = lane < 3 ? lane : 0;
-      node = node0 + r;
-      s0 = r == 0 ? m1[0][0] : r == 1 ? m1[1][0] : m1[2][0];
-      ux = r == 0 ? u[0][0] : r == 1 ? u[1][0] : u[2][0];
-      uy = r == 0 ? u[0][1] : r == 1 ? u[1][1] : u[2][1];
-      sp = r == 0 ? m2[0][0] : r == 1 ? m2[1][0] : m2[2][0];
-      sc = r == 0 ? m2[0][1] : r == 1 ? m2[1][1] : m2[2][1];
-      nd = s0 >= TINY_D ? s0 : 0.0;
+      row_sums<2>(m2, lane, t2);
+      sp = t2[0];
+      sc = t2[1];
+      node = lane < 24 ? node0 + (lane >> 3) : 3 * C.E;  // lanes 16 to 23: row 2
     } else {
       node = node0 + grp;
       const T* row = reinterpret_cast<const T*>(ring + (size_t)s * stage_bytes + (size_t)grp * C.rowbytes);
@@ -653,9 +682,8 @@ __global__ void __launch_bounds__(ONE ? 640 : 512, 1)
       s0 = group_sum<L>(s0);
       s1 = group_sum<L>(s1);
       s2 = group_sum<L>(s2);
-      nd = ux = uy = 0;
+      ux = uy = 0;
       if (s0 >= TINY_D) {  // src/macros.f90:126-134
-        nd = s0;
         const double inv = 1.0 / s0;
         ux = s1 * inv;
         uy = s2 * inv;
@@ -665,7 +693,6 @@ __global__ void __launch_bounds__(ONE ? 640 : 512, 1)
       sp = group_sum<L>(sp);
       sc = group_sum<L>(sc);
     }
-    const bool live = live0 && node < 3 * C.E;
     __syncwarp();
     // the rows are consumed: refill this stage with the group nstage ahead
     if (lane == 0) {
@@ -675,7 +702,15 @@ __global__ void __launch_bounds__(ONE ? 640 : 512, 1)
         fill(s, nxt);
       }
     }
-    if ((ELEM ? lane < 3 : sub == 0) && live) mumax = fmax(mumax, node_epilogue(C, node, s0, ux, uy, nd, sp, sc));
+    if ((lane & (KEEP - 1)) == kept && live0 && node < 3 * C.E) {
+      knode = node;
+      k0 = s0;
+      kux = ux;
+      kuy = uy;
+      ksp = sp;
+      ksc = sc;
+    }
+    if (++kept == KEEP) flush_nodes();
     s = (s + 1 == nstage) ? 0 : s + 1;
   }
   if (aborted) {
@@ -685,6 +720,7 @@ __global__ void __launch_bounds__(ONE ? 640 : 512, 1)
     }
     return;
   }
+  flush_nodes();
   flush_mu();
 }
 
