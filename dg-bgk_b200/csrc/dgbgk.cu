@@ -264,27 +264,30 @@ int build_launch_set(LaunchSet<T>& L, const std::vector<CaseDev<T>>& cs, int eb,
   const size_t cap = 227 * 1024;
   long best = -1;
   for (int R : {4, 3, 2, 1})
-    for (int w : {20, 16, 15, 14, 13, 12, 10, 8, 6, 5, 4, 3, 2, 1})
+    for (int w : {20, 16, 15, 14, 13, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2, 1})
       for (int sg : {3, 2, 1}) {
         if (force_rows > 0 && R != force_rows) continue;
-        const size_t tbytes = one ? (mom_tables(R) * (size_t)cs[0].Vp * sizeof(T) + 127) / 128 * 128 : 0;
-        if (w > 16 && !one) continue;  // 640 threads: the single-case kernel only
-        const size_t bytes = 128 * (((size_t)w * sg * 8 + 127) / 128) + tbytes + (size_t)w * sg * R * maxrow;
+        const size_t tbytes = one ? (mom_tables<T>(R) * (size_t)cs[0].Vp * sizeof(T) + 127) / 128 * 128 : 0;
+        const int nt = w * 32;  // threads
+        if (nt > (one ? 640 : 512)) continue;
+        const size_t bytes =
+            128 * (((size_t)w * sg * 8 + 127) / 128) + tbytes + (size_t)w * sg * R * maxrow;
         if (bytes > cap) continue;
         // resident CTAs per SM (shared memory and registers)
         const void* mfn = (const void*)mom_fn<T>(R, one);
         int blocks = 0;
         TRY(allow_max_smem(mfn));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, mfn, w * 32, bytes));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, mfn, nt, bytes));
         blocks = std::min(blocks, 4);
         if (blocks < 1) continue;
         long score = ((long)blocks * w * 1024 + (long)blocks * w * (sg - 1) * R) * 8 + (8 - R);
-        // FP32: the element mode (R = 3: three rows per warp step sharing
-        // the velocity tables) first, while it keeps 8 or more warps per SM
-        // (measured on the 200x100 channel at 24x48 velocities: 0.158 ms,
-        // against 0.191 with one row per warp step; FP64 loses occupancy
-        // with it: 0.387 against 0.325)
-        if (R == 3 && force_rows == 0) score = (sizeof(T) == 4 && blocks * w >= 8) ? score + (1L << 40) : -1;
+        // the element mode (R = 3: three rows per warp step sharing the
+        // velocity tables) first, while it keeps 8 or more warps per SM.
+        // Measured: FP32, 24x48 velocities (15 warps), 0.158 ms against
+        // 0.191 with one row per warp step; FP64, 16x32 velocities (15
+        // warps), 0.078 against 0.095; FP64, 24x48 (7 warps), 0.387 against
+        // 0.325
+        if (R == 3 && force_rows == 0) score = blocks * nt >= 256 ? score + (1L << 40) : -1;
         if (score > best) {
           best = score;
           L.mom_rows = R;

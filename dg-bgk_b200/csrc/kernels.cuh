@@ -181,7 +181,7 @@ template <class T> __device__ __forceinline__ void sweep_group(const CaseDev<T>&
 // single case (tables in shared memory) rows 2 to 4 in its first pass and 0
 // to 2 in its second, of a batch (tables through L1) the first three.
 constexpr int MOM_TABS = 5;
-__host__ __device__ constexpr int mom_tables(int R) { return R == 3 ? 5 : 3; }
+template <class T> __host__ __device__ constexpr int mom_tables(int R) { return R == 3 && sizeof(T) == 4 ? 5 : 3; }
 
 template <class T> struct BatchArgs {
   const CaseDev<T>* cases;  // [ncases]
@@ -326,82 +326,80 @@ template <> struct RowMath<float> {
 // partials, summed in FP64 across the warp; FP64 storage: FP64 throughout.
 template <class T> struct ElemMath;
 
+// body(o) for the byte offsets o = 16*q of a lane's vectors, two at a time
+// (half the address arithmetic: FP32 0.128 -> 0.124 ms on the 200x100 channel)
+template <class F> __device__ __forceinline__ void for_vectors(int lane, int nq, F body) {
+  int q = lane;
+  for (; q + 32 < nq; q += 64) {
+    body(16 * q);
+    body(16 * q + 512);
+  }
+  if (q < nq) body(16 * q);
+}
+template <class V> __device__ __forceinline__ V at(const unsigned char* p, int o) {
+  return *reinterpret_cast<const V*>(p + o);
+}
+
 template <> struct ElemMath<float> {
   // Each sum runs as two partial sums, the even and the odd values of a
   // vector (shorter dependent chains: 0.1535 -> 0.1508 ms on the 200x100
-  // channel; four partials were slower).  Where the two partial sums take
-  // the same operations, they are the halves of one packed pair
-  // (fma/add/mul.rn.f32x2: one instruction for two values; the same bits
-  // as two scalar chains; 0.1527 -> 0.1456 ms).
+  // channel; four partials were slower), the halves of one packed pair
+  // (fma/add/mul.rn.f32x2: one instruction for two values; 0.1527 ->
+  // 0.1456 ms).
   // pass 1.  TAB: from the tables w, w*cx, w*cy (three FMAs per value;
   // tables in shared memory); otherwise from w, cx, cy (w*f, then three
   // sums; the tables the second pass reads too, through L1)
   template <bool TAB>
-  static __device__ __forceinline__ void pass1(const float* rows, unsigned pitch, const float* tb, int Vp, int nq,
-                                               int lane, double (&s)[3][3]) {
-    const float4* wj = reinterpret_cast<const float4*>(tb + 2 * Vp);
-    const float4* wx = reinterpret_cast<const float4*>(tb + (TAB ? 3 : 0) * Vp);
-    const float4* wy = reinterpret_cast<const float4*>(tb + (TAB ? 4 : 1) * Vp);
-    if constexpr (TAB) {
-      float2 t[3][3];
+  static __device__ __forceinline__ void pass1(const unsigned char* rows, unsigned pitch, const float* tb, int Vp,
+                                               int nq, int lane, double (&s)[3][3]) {
+    const unsigned char* wj = reinterpret_cast<const unsigned char*>(tb + 2 * Vp);
+    const unsigned char* wx = reinterpret_cast<const unsigned char*>(tb + (TAB ? 3 : 0) * Vp);
+    const unsigned char* wy = reinterpret_cast<const unsigned char*>(tb + (TAB ? 4 : 1) * Vp);
+    float2 t[3][3];
 #pragma unroll
-      for (int r = 0; r < 3; ++r)
+    for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) t[r][k] = make_float2(0.f, 0.f);
-      for (int q = lane; q < nq; q += 32) {
-        const float4 w = wj[q], c = wx[q], d = wy[q];
+      for (int k = 0; k < 3; ++k) t[r][k] = make_float2(0.f, 0.f);
+    for_vectors(lane, nq, [&](int o) {
+      const float4 w = at<float4>(wj, o), c = at<float4>(wx, o), d = at<float4>(wy, o);
 #pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          const float4 x =
-              reinterpret_cast<const float4*>(reinterpret_cast<const unsigned char*>(rows) + r * pitch)[q];
+      for (int r = 0; r < 3; ++r) {
+        const float4 x = at<float4>(rows + r * pitch, o);
+        if constexpr (TAB) {
           t[r][0] = __ffma2_rn(lo2(w), lo2(x), __ffma2_rn(hi2(w), hi2(x), t[r][0]));
           t[r][1] = __ffma2_rn(lo2(c), lo2(x), __ffma2_rn(hi2(c), hi2(x), t[r][1]));
           t[r][2] = __ffma2_rn(lo2(d), lo2(x), __ffma2_rn(hi2(d), hi2(x), t[r][2]));
+        } else {
+          const float2 al = __fmul2_rn(lo2(w), lo2(x)), ah = __fmul2_rn(hi2(w), hi2(x));
+          t[r][0] = __fadd2_rn(t[r][0], __fadd2_rn(al, ah));
+          t[r][1] = __ffma2_rn(lo2(c), al, __ffma2_rn(hi2(c), ah, t[r][1]));
+          t[r][2] = __ffma2_rn(lo2(d), al, __ffma2_rn(hi2(d), ah, t[r][2]));
         }
       }
+    });
 #pragma unroll
-      for (int r = 0; r < 3; ++r)
+    for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) s[r][k] = (double)t[r][k].x + (double)t[r][k].y;
-    } else {
-      float t[3][3] = {};
-      for (int q = lane; q < nq; q += 32) {
-        const float4 w = wj[q], c = wx[q], d = wy[q];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          const float4 x =
-              reinterpret_cast<const float4*>(reinterpret_cast<const unsigned char*>(rows) + r * pitch)[q];
-          const float a0 = w.x * x.x, a1 = w.y * x.y, a2 = w.z * x.z, a3 = w.w * x.w;
-          t[r][0] += (a0 + a1) + (a2 + a3);
-          t[r][1] = fmaf(c.x, a0, fmaf(c.y, a1, fmaf(c.z, a2, fmaf(c.w, a3, t[r][1]))));
-          t[r][2] = fmaf(d.x, a0, fmaf(d.y, a1, fmaf(d.z, a2, fmaf(d.w, a3, t[r][2]))));
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) s[r][k] = (double)t[r][k];
-    }
+      for (int k = 0; k < 3; ++k) s[r][k] = (double)t[r][k].x + (double)t[r][k].y;
   }
   // pass 2 on packed pairs (c - u as c + (-u))
-  static __device__ __forceinline__ void pass2(const float* rows, unsigned pitch, const float* tb, int Vp, int nq,
-                                               int lane, const float (&u)[3][2], double (&s)[3][2]) {
-    const float4* cx = reinterpret_cast<const float4*>(tb);
-    const float4* cy = reinterpret_cast<const float4*>(tb + Vp);
-    const float4* wj = reinterpret_cast<const float4*>(tb + 2 * Vp);
+  static __device__ __forceinline__ void pass2(const unsigned char* rows, unsigned pitch, const float* tb, int Vp,
+                                               int nq, int lane, const float (&u)[3][2], double (&s)[3][2]) {
+    const unsigned char* cx = reinterpret_cast<const unsigned char*>(tb);
+    const unsigned char* cy = reinterpret_cast<const unsigned char*>(tb + Vp);
+    const unsigned char* wj = reinterpret_cast<const unsigned char*>(tb + 2 * Vp);
     float2 nu[3][2], t[3][2];
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-      const float ux = u[r][0], uy = u[r][1];
-      nu[r][0] = make_float2(-ux, -ux);
-      nu[r][1] = make_float2(-uy, -uy);
+      nu[r][0] = make_float2(-u[r][0], -u[r][0]);
+      nu[r][1] = make_float2(-u[r][1], -u[r][1]);
       t[r][0] = t[r][1] = make_float2(0.f, 0.f);
     }
-    for (int q = lane; q < nq; q += 32) {
-      const float4 c = cx[q], d = cy[q], w = wj[q];
+    for_vectors(lane, nq, [&](int o) {
+      const float4 c = at<float4>(cx, o), d = at<float4>(cy, o), w = at<float4>(wj, o);
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-        const float4 x = reinterpret_cast<const float4*>(reinterpret_cast<const unsigned char*>(rows) + r * pitch)[q];
+        const float4 x = at<float4>(rows + r * pitch, o);
         const float2 el = __fadd2_rn(lo2(c), nu[r][0]), eh = __fadd2_rn(hi2(c), nu[r][0]);
         const float2 gl = __fadd2_rn(lo2(d), nu[r][1]), gh = __fadd2_rn(hi2(d), nu[r][1]);
         const float2 ql = __ffma2_rn(el, el, __fmul2_rn(gl, gl)), qh = __ffma2_rn(eh, eh, __fmul2_rn(gh, gh));
@@ -411,7 +409,7 @@ template <> struct ElemMath<float> {
         const float2 sh = make_float2(sqrt_fast(qh.x), sqrt_fast(qh.y));
         t[r][1] = __ffma2_rn(sl, al, __ffma2_rn(sh, ah, t[r][1]));  // src/compmu.f90:71-74
       }
-    }
+    });
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
       s[r][0] = 0.5 * ((double)t[r][0].x + (double)t[r][0].y);
@@ -421,52 +419,46 @@ template <> struct ElemMath<float> {
 };
 
 template <> struct ElemMath<double> {
-  // pass 1, TAB as for FP32
+  // (from w, cx, cy: the products' tables would take the room of a stage)
   template <bool TAB>
-  static __device__ __forceinline__ void pass1(const double* rows, unsigned pitch, const double* tb, int Vp, int nq,
-                                               int lane, double (&s)[3][3]) {
-    const double2* wj = reinterpret_cast<const double2*>(tb + 2 * Vp);
-    const double2* wx = reinterpret_cast<const double2*>(tb + (TAB ? 3 : 0) * Vp);
-    const double2* wy = reinterpret_cast<const double2*>(tb + (TAB ? 4 : 1) * Vp);
+  static __device__ __forceinline__ void pass1(const unsigned char* rows, unsigned pitch, const double* tb, int Vp,
+                                               int nq, int lane, double (&s)[3][3]) {
+    const unsigned char* cx = reinterpret_cast<const unsigned char*>(tb);
+    const unsigned char* cy = reinterpret_cast<const unsigned char*>(tb + Vp);
+    const unsigned char* wj = reinterpret_cast<const unsigned char*>(tb + 2 * Vp);
 #pragma unroll
     for (int r = 0; r < 3; ++r) s[r][0] = s[r][1] = s[r][2] = 0.0;
-    for (int q = lane; q < nq; q += 32) {
-      const double2 w = wj[q], c = wx[q], d = wy[q];
+    for_vectors(lane, nq, [&](int o) {
+      const double2 w = at<double2>(wj, o), c = at<double2>(cx, o), d = at<double2>(cy, o);
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-        const double2 x = reinterpret_cast<const double2*>(reinterpret_cast<const unsigned char*>(rows) + r * pitch)[q];
-        if constexpr (TAB) {
-          s[r][0] = fma(w.x, x.x, fma(w.y, x.y, s[r][0]));
-          s[r][1] = fma(c.x, x.x, fma(c.y, x.y, s[r][1]));
-          s[r][2] = fma(d.x, x.x, fma(d.y, x.y, s[r][2]));
-        } else {
-          const double a0 = w.x * x.x, a1 = w.y * x.y;
-          s[r][0] += a0 + a1;
-          s[r][1] = fma(c.x, a0, fma(c.y, a1, s[r][1]));
-          s[r][2] = fma(d.x, a0, fma(d.y, a1, s[r][2]));
-        }
+        const double2 x = at<double2>(rows + r * pitch, o);
+        const double a0 = w.x * x.x, a1 = w.y * x.y;
+        s[r][0] += a0 + a1;
+        s[r][1] = fma(c.x, a0, fma(c.y, a1, s[r][1]));
+        s[r][2] = fma(d.x, a0, fma(d.y, a1, s[r][2]));
       }
-    }
+    });
   }
-  static __device__ __forceinline__ void pass2(const double* rows, unsigned pitch, const double* tb, int Vp, int nq,
-                                               int lane, const double (&u)[3][2], double (&s)[3][2]) {
-    const double2* cx = reinterpret_cast<const double2*>(tb);
-    const double2* cy = reinterpret_cast<const double2*>(tb + Vp);
-    const double2* wj = reinterpret_cast<const double2*>(tb + 2 * Vp);
+  static __device__ __forceinline__ void pass2(const unsigned char* rows, unsigned pitch, const double* tb, int Vp,
+                                               int nq, int lane, const double (&u)[3][2], double (&s)[3][2]) {
+    const unsigned char* cx = reinterpret_cast<const unsigned char*>(tb);
+    const unsigned char* cy = reinterpret_cast<const unsigned char*>(tb + Vp);
+    const unsigned char* wj = reinterpret_cast<const unsigned char*>(tb + 2 * Vp);
 #pragma unroll
     for (int r = 0; r < 3; ++r) s[r][0] = s[r][1] = 0.0;
-    for (int q = lane; q < nq; q += 32) {
-      const double2 c = cx[q], d = cy[q], w = wj[q];
+    for_vectors(lane, nq, [&](int o) {
+      const double2 c = at<double2>(cx, o), d = at<double2>(cy, o), w = at<double2>(wj, o);
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
-        const double2 x = reinterpret_cast<const double2*>(reinterpret_cast<const unsigned char*>(rows) + r * pitch)[q];
+        const double2 x = at<double2>(rows + r * pitch, o);
         const double dx0 = c.x - u[r][0], dy0 = d.x - u[r][1], dx1 = c.y - u[r][0], dy1 = d.y - u[r][1];
-        const double q0 = dx0 * dx0 + dy0 * dy0, q1 = dx1 * dx1 + dy1 * dy1;
+        const double q0v = dx0 * dx0 + dy0 * dy0, q1v = dx1 * dx1 + dy1 * dy1;
         const double a0 = w.x * x.x, a1 = w.y * x.y;
-        s[r][0] = fma(q0, a0, fma(q1, a1, s[r][0]));                            // src/macros.f90:144-148, times 2
-        s[r][1] = fma(sqrt_newton(q0), a0, fma(sqrt_newton(q1), a1, s[r][1]));  // src/compmu.f90:71-74
+        s[r][0] = fma(q0v, a0, fma(q1v, a1, s[r][0]));                            // src/macros.f90:144-148, times 2
+        s[r][1] = fma(sqrt_newton(q0v), a0, fma(sqrt_newton(q1v), a1, s[r][1]));  // src/compmu.f90:71-74
       }
-    }
+    });
 #pragma unroll
     for (int r = 0; r < 3; ++r) s[r][0] *= 0.5;
   }
@@ -565,15 +557,18 @@ __global__ void __launch_bounds__(ONE ? 640 : 512, 1)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int grp = ELEM ? 0 : lane / L, sub = lane % L;
   const int nstage = a.mom_stages;
-  // layout: [barriers][tables [3][Vp] (ONE)][rings: warp, stage, R rows]
+  // layout: [barriers][tables [mom_tables][Vp] (ONE)][rings: warp, stage, R rows]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm_raw) + warp * nstage;
   T* tb1 = reinterpret_cast<T*>(sm_raw + 128 * (((size_t)nwarp * nstage * 8 + 127) / 128));
-  constexpr int NTB = mom_tables(R);  // tables staged for a single case
+  constexpr int NTB = mom_tables<T>(R);  // tables staged for a single case
   const size_t tbytes = ONE ? (NTB * (size_t)one.Vp * sizeof(T) + 127) / 128 * 128 : 0;
   const size_t stage_bytes = (size_t)R * a.mom_rowbytes;
   unsigned char* ring = reinterpret_cast<unsigned char*>(tb1) + tbytes + (size_t)warp * nstage * stage_bytes;
-  if (ONE)
-    for (int i = threadIdx.x; i < NTB * one.Vp; i += blockDim.x) tb1[i] = one.tabs[i];
+  if (ONE) {
+    const uint4* src = reinterpret_cast<const uint4*>(one.tabs);
+    for (int i = threadIdx.x; i < (int)(NTB * one.Vp * sizeof(T) / 16); i += blockDim.x)
+      reinterpret_cast<uint4*>(tb1)[i] = src[i];
+  }
   const int gw = blockIdx.x * nwarp + warp, stride = gridDim.x * nwarp;
   if (lane == 0) {
     for (int s = 0; s < nstage; ++s) mbar_init(&bars[s], 1);
@@ -650,9 +645,9 @@ __global__ void __launch_bounds__(ONE ? 640 : 512, 1)
     int node;
     double s0, ux, uy, sp, sc;
     if constexpr (ELEM) {
-      const T* rows = reinterpret_cast<const T*>(ring + (size_t)s * stage_bytes);
+      const unsigned char* rows = ring + (size_t)s * stage_bytes;
       double m1[3][3], t1[3], m2[3][2], t2[2];
-      ElemMath<T>::template pass1<ONE>(rows, C.rowbytes, tb, C.Vp, nql, lane, m1);
+      ElemMath<T>::template pass1<ONE && sizeof(T) == 4>(rows, C.rowbytes, tb, C.Vp, nql, lane, m1);
       row_sums<3>(m1, lane, t1);
       s0 = t1[0];
       ux = uy = 0.0;
