@@ -5,9 +5,12 @@
 // keeps W and W^T in BF16 and every activation and gradient in both
 // layouts:
 //   forward   H_{l+1} = tanh(H_l W_l^T + b_l)       A = H_l,   B = W_l
-//   output    P = H_L W_L^T + b_L                    (FP32)
-//   loss      dP = 2 (P - T) / (B n_out)             (BF16, both layouts)
+//   output    P = H_L W_L^T + b_L                    (FP32; a forward call)
+//   loss      dP = 2 (P - T) / (B n_out)             (BF16, both layouts; the
+//             output layer's epilogue in a training step, P is not stored)
 //   dW_l      = dZ_{l+1}^T H_l                        A = dZ^T,  B = H_l^T
+//             (a training step: Adam in its epilogue, the gradient is not
+//             stored)
 //   dZ_l      = (dZ_{l+1} W_l) (1 - H_l^2)            A = dZ,    B = W_l^T
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -84,19 +87,27 @@ int bf16_map(CUtensorMap* m, const void* p, int rows, int cols, int box_rows) {
   return 0;
 }
 
-// One planned GEMM: its operand maps and epilogue.
+// One planned GEMM: its operand maps, tile and epilogue.
 struct Gemm {
   CUtensorMap ta, tb;
   GemmArgs g;
-  int bn;
+  int bn, epi;
 };
 
-int plan_gemm(Gemm& G, const __nv_bfloat16* A, const __nv_bfloat16* B, int M, int N, int K, GemmArgs g) {
-  if (M % BM || K % BK || N % 64) {
+// Tile widths: 32 columns where 64 would leave SMs without a tile (the hidden
+// layers, and the output layer's dZ, whose K is n_out), 64 otherwise.  The
+// narrow tile's ring takes most of an SM: its CTAs are few, and what they
+// need is loads in flight.  dZ of 128 x 512 with K = 32768: 175 us with four
+// CTAs of 128 x 128 tiles, 75 with 16 of 128 x 32.
+constexpr int STAGES32 = 5, STAGES64 = 2, STAGES_ADAM = 2;
+
+int plan_gemm(Gemm& G, const __nv_bfloat16* A, const __nv_bfloat16* B, int M, int N, int K, int epi, GemmArgs g) {
+  if (M % BM || N % 64 || (K % (2 * BK) && !(K == BK && epi == EPI_TANH))) {
     set_error("MLP GEMM shape not a multiple of the tile");
     return DGBGK_EINVAL;
   }
-  G.bn = (N % 128 == 0) ? 128 : 64;
+  G.epi = epi;
+  G.bn = epi != EPI_ADAM && epi != EPI_F32 && (long)(M / BM) * (N / 64) < 148 ? 32 : 64;
   MTRY(bf16_map(&G.ta, A, M, K, BM));
   MTRY(bf16_map(&G.tb, B, N, K, G.bn));
   G.g = g;
@@ -106,98 +117,76 @@ int plan_gemm(Gemm& G, const __nv_bfloat16* A, const __nv_bfloat16* B, int M, in
   return 0;
 }
 
-int allow_smem(const void* fn, size_t bytes) {
-  MCK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return 0;
-}
-
-int run_gemm(const Gemm& G, cudaStream_t st) {
-  dim3 grid(G.g.N / G.bn, G.g.M / BM);
-  if (G.bn == 128) {
-    MTRY(allow_smem((const void*)k_gemm<128>, Smem<128>::TOTAL));
-    k_gemm<128><<<grid, 128, Smem<128>::TOTAL, st>>>(G.ta, G.tb, G.g);
-  } else {
-    MTRY(allow_smem((const void*)k_gemm<64>, Smem<64>::TOTAL));
-    k_gemm<64><<<grid, 128, Smem<64>::TOTAL, st>>>(G.ta, G.tb, G.g);
-  }
+template <int BN, int STAGES, int SUB, int EPI> int launch_gemm(const Gemm& G, const GemmArgs& g, cudaStream_t st) {
+  auto fn = k_gemm<BN, STAGES, SUB, EPI>;
+  constexpr int bytes = Smem<BN, STAGES, SUB, EPI>::TOTAL;
+  MCK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  fn<<<dim3(g.N / BN, g.M / BM), 128, bytes, st>>>(G.ta, G.tb, g);
   MCK(cudaGetLastError());
   return 0;
 }
+// two K-blocks of 64 a stage; the input layer's forward has one in all
+template <int EPI> int launch_gemm(const Gemm& G, const GemmArgs& g, cudaStream_t st) {
+  if (EPI == EPI_TANH && g.K == BK)
+    return G.bn == 32 ? launch_gemm<32, 1, 1, EPI_TANH>(G, g, st) : launch_gemm<64, 1, 1, EPI_TANH>(G, g, st);
+  return G.bn == 32 ? launch_gemm<32, STAGES32, 2, EPI>(G, g, st) : launch_gemm<64, STAGES64, 2, EPI>(G, g, st);
+}
+int run_gemm(const Gemm& G, const GemmArgs& g, cudaStream_t st) {
+  switch (G.epi) {
+    case EPI_TANH: return launch_gemm<EPI_TANH>(G, g, st);
+    case EPI_LINEAR: return launch_gemm<EPI_LINEAR>(G, g, st);
+    case EPI_DTANH: return launch_gemm<EPI_DTANH>(G, g, st);
+    case EPI_LOSS: return launch_gemm<EPI_LOSS>(G, g, st);
+    default: return launch_gemm<64, STAGES64, 2, EPI_F32>(G, g, st);
+  }
+}
+int run_gemm(const Gemm& G, cudaStream_t st) { return run_gemm(G, G.g, st); }
 
 // ----------------------------------------------------------- small kernels
-// minibatch: rows idx[r] of the set -> X0 (BF16, padded to KPAD, both
-// layouts) and T (FP32)
-__global__ void k_gather(const float* __restrict__ xs, const float* __restrict__ ts, const int* __restrict__ idx,
-                         int n_in, int n_out, int B, __nv_bfloat16* x0, __nv_bfloat16* x0T, float* t) {
-  const int r = blockIdx.x;
-  const int s = idx[r];
-  for (int c = threadIdx.x; c < KPAD; c += blockDim.x) {
-    const float v = c < n_in ? xs[(size_t)s * n_in + c] : 0.f;
-    x0[(size_t)r * KPAD + c] = __float2bfloat16_rn(v);
-    x0T[(size_t)c * B + r] = __float2bfloat16_rn(v);
-  }
-  for (int c = threadIdx.x; c < n_out; c += blockDim.x) t[(size_t)r * n_out + c] = ts[(size_t)s * n_out + c];
+// minibatch inputs: rows idx[r] of the set -> X0 (BF16, padded to KPAD, both
+// layouts)
+__global__ void k_gather(const float* __restrict__ xs, const int* __restrict__ idx, int n_in, int B,
+                         __nv_bfloat16* x0, __nv_bfloat16* x0T) {
+  const int r = blockIdx.x * blockDim.y + threadIdx.y, c = threadIdx.x;
+  const __nv_bfloat16 v = __float2bfloat16_rn(c < n_in ? xs[(size_t)idx[r] * n_in + c] : 0.f);
+  x0[(size_t)r * KPAD + c] = v;
+  x0T[(size_t)c * B + r] = v;
 }
 
-// MSE loss and its gradient: dP = 2 (P - T) / (B n_out) in both layouts;
-// the loss sum goes to loss[0] (FP64 atomics of per-block sums)
-__global__ void k_loss(const float* __restrict__ p, const float* __restrict__ t, int B, int n_out,
-                       __nv_bfloat16* dp, __nv_bfloat16* dpT, double* loss) {
-  const size_t n = (size_t)B * n_out;
-  const float scale = 2.f / (float)n;
-  double acc = 0.0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const float d = p[i] - t[i];
-    acc += (double)d * d;
-    const int r = (int)(i / n_out), c = (int)(i - (size_t)r * n_out);
-    const __nv_bfloat16 g = __float2bfloat16_rn(scale * d);
-    dp[i] = g;
-    dpT[(size_t)c * B + r] = g;
-  }
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  __shared__ double red[32];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-    atomicAdd(loss, s / (double)n);
-  }
+// bias gradient: the sum over the batch of G[.., j], from G^T [N][B], by a warp
+__device__ __forceinline__ float bias_grad(const __nv_bfloat16* __restrict__ row, int B, int lane) {
+  float s = 0.f;
+  for (int r = lane; r < B; r += 32) s += __bfloat162float(row[r]);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
 }
-
-// bias gradient: db[j] = sum over the batch of G[.., j], from G^T [N][B]
 __global__ void k_bias_grad(const __nv_bfloat16* __restrict__ gT, int N, int B, float* db) {
   const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (j >= N) return;
-  float s = 0.f;
-  for (int r = lane; r < B; r += 32) s += __bfloat162float(gT[(size_t)j * B + r]);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  const float s = bias_grad(gT + (size_t)j * B, B, lane);
   if (lane == 0) db[j] = s;
 }
-
-// Adam on FP32 masters; refreshes the BF16 copies W [out][in] and W^T
-// [in][out].  Padded input columns (c >= in_live) stay zero.
-__global__ void k_adam(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v, const float* __restrict__ g,
-                       int rows, int cols, int in_live, float lr, float b1, float b2, float eps, float c1, float c2,
-                       __nv_bfloat16* wb, __nv_bfloat16* wbT) {
-  const size_t n = (size_t)rows * cols;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int r = (int)(i / cols), c = (int)(i - (size_t)r * cols);
-    float x = w[i];
-    if (c < in_live) {
-      const float gi = g[i];
-      const float mi = b1 * m[i] + (1.f - b1) * gi;
-      const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-      m[i] = mi;
-      v[i] = vi;
-      x -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-      w[i] = x;
-    }
-    if (wb) {
-      const __nv_bfloat16 xb = __float2bfloat16_rn(x);
-      wb[i] = xb;
-      wbT[(size_t)c * rows + r] = xb;
-    }
+// the biases' gradients and Adam steps of up to BIAS_LAYERS layers
+constexpr int BIAS_LAYERS = 8;
+struct BiasArgs {
+  const __nv_bfloat16* gT[BIAS_LAYERS];
+  float *b[BIAS_LAYERS], *m[BIAS_LAYERS], *v[BIAS_LAYERS];
+  int end[BIAS_LAYERS];  // running sum of the layers' widths
+  int n, B;
+};
+__global__ void k_bias_adam(const __grid_constant__ BiasArgs a, const __grid_constant__ GemmArgs p) {
+  int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (j >= a.end[a.n - 1]) return;
+  int l = 0;
+  while (j >= a.end[l]) ++l;
+  if (l > 0) j -= a.end[l - 1];
+  const float g = bias_grad(a.gT[l] + (size_t)j * a.B, a.B, lane);
+  if (lane == 0) {
+    float m = a.m[l][j], v = a.v[l][j];
+    a.b[l][j] = adam_step(a.b[l][j], m, v, g, p);
+    a.m[l][j] = m;
+    a.v[l][j] = v;
   }
 }
 
@@ -241,7 +230,7 @@ struct dgbgk_mlp {
   std::vector<Layer> L;                  // depth + 1 layers
   std::vector<__nv_bfloat16*> H, HT;     // activations 0..depth (0 = input), [B][in] and [in][B]
   std::vector<__nv_bfloat16*> G, GT;     // dZ of layers 1..depth, and dP (index depth+1)
-  float *P = nullptr, *T = nullptr;
+  float* P = nullptr;
   double* loss = nullptr;                // one slot per training step (slot 0 otherwise)
   int loss_cap = 1;
   int* err = nullptr;
@@ -252,7 +241,8 @@ struct dgbgk_mlp {
   float *xin = nullptr, *tin = nullptr;  // staging of one host batch
   int* iin = nullptr;
   long long adam_t = 0;
-  std::vector<Gemm> fwd, bwd_dw, bwd_dx;
+  std::vector<Gemm> fwd, bwd_dw, bwd_dx, adam_dw;
+  Gemm out_loss;  // the output layer with the loss in its epilogue
 
   ~dgbgk_mlp() {
     cudaSetDevice(device);
@@ -265,7 +255,7 @@ struct dgbgk_mlp {
     for (auto* p : HT) mfree(p);
     for (auto* p : G) mfree(p);
     for (auto* p : GT) mfree(p);
-    mfree(P), mfree(T), mfree(loss), mfree(err), mfree(xs), mfree(ts), mfree(idx);
+    mfree(P), mfree(loss), mfree(err), mfree(xs), mfree(ts), mfree(idx);
     mfree(xin), mfree(tin), mfree(iin);
     if (st) cudaStreamDestroy(st);
   }
@@ -316,7 +306,6 @@ struct dgbgk_mlp {
       MTRY(mall(&GT[l], (size_t)B * c));
     }
     MTRY(mall(&P, (size_t)B * n_out));
-    MTRY(mall(&T, (size_t)B * n_out));
     MTRY(mall(&loss, 1));
     MTRY(mall(&err, 1));
     MTRY(mall(&xin, (size_t)B * n_in));
@@ -344,35 +333,44 @@ struct dgbgk_mlp {
     fwd.assign(nl, Gemm{});
     bwd_dw.assign(nl, Gemm{});
     bwd_dx.assign(nl, Gemm{});
+    adam_dw.assign(nl, Gemm{});
     for (int l = 0; l < nl; ++l) {
       Layer& y = L[l];
       GemmArgs g{};
       g.err = err;
       g.bias = y.b;
       if (l < depth) {
-        g.epi = EPI_TANH;
         g.out_bf = H[l + 1];
         g.out_bfT = HT[l + 1];
+        MTRY(plan_gemm(fwd[l], H[l], y.wb, B, y.out, y.in, EPI_TANH, g));
       } else {
-        g.epi = EPI_LINEAR;
         g.out_f = P;
+        MTRY(plan_gemm(fwd[l], H[l], y.wb, B, y.out, y.in, EPI_LINEAR, g));
+        g.out_bf = G[nl];
+        g.out_bfT = GT[nl];
+        g.scale = 2.f / (float)((size_t)B * n_out);
+        MTRY(plan_gemm(out_loss, H[l], y.wb, B, y.out, y.in, EPI_LOSS, g));
       }
-      MTRY(plan_gemm(fwd[l], H[l], y.wb, B, y.out, y.in, g));
       // dW_l = G_{l+1}^T H_l: [out][in], K = B
       GemmArgs gw{};
       gw.err = err;
-      gw.epi = EPI_F32;
       gw.out_f = y.gw;
-      MTRY(plan_gemm(bwd_dw[l], GT[l + 1], HT[l], y.out, y.in, B, gw));
+      MTRY(plan_gemm(bwd_dw[l], GT[l + 1], HT[l], y.out, y.in, B, EPI_F32, gw));
+      gw.w = y.w;
+      gw.m = y.mw;
+      gw.v = y.vw;
+      gw.out_bf = y.wb;
+      gw.out_bfT = y.wbT;
+      gw.live = y.in_live;
+      MTRY(plan_gemm(adam_dw[l], GT[l + 1], HT[l], y.out, y.in, B, EPI_ADAM, gw));
       // G_l = (G_{l+1} W_l) (1 - H_l^2): [B][in], K = out (not for the input layer)
       if (l > 0) {
         GemmArgs gx{};
         gx.err = err;
-        gx.epi = EPI_DTANH;
         gx.aux = H[l];
         gx.out_bf = G[l];
         gx.out_bfT = GT[l];
-        MTRY(plan_gemm(bwd_dx[l], G[l + 1], y.wbT, B, y.in, y.out, gx));
+        MTRY(plan_gemm(bwd_dx[l], G[l + 1], y.wbT, B, y.in, y.out, EPI_DTANH, gx));
       }
     }
     return 0;
@@ -383,11 +381,20 @@ struct dgbgk_mlp {
     return 0;
   }
 
-  // loss (into *lslot) and all gradients of the current minibatch (in H[0], T)
-  int backward(double* lslot) {
+  // forward, and the loss (into *lslot) and its gradient at the output, of
+  // the minibatch whose inputs are in H[0] and whose targets are rows id of t
+  int forward_loss(const float* t, const int* id, double* lslot) {
     MCK(cudaMemsetAsync(lslot, 0, sizeof(double), st));
-    k_loss<<<592, 256, 0, st>>>(P, T, B, n_out, G[depth + 1], GT[depth + 1], lslot);
-    MCK(cudaGetLastError());
+    for (int l = 0; l < depth; ++l) MTRY(run_gemm(fwd[l], st));
+    GemmArgs g = out_loss.g;
+    g.ts = t;
+    g.idx = id;
+    g.loss = lslot;
+    return run_gemm(out_loss, g, st);
+  }
+
+  // all gradients of the minibatch
+  int backward() {
     for (int l = depth; l >= 0; --l) {
       MTRY(run_gemm(bwd_dw[l], st));
       k_bias_grad<<<(L[l].out + 7) / 8, 256, 0, st>>>(GT[l + 1], L[l].out, B, L[l].gb);
@@ -397,15 +404,59 @@ struct dgbgk_mlp {
     return 0;
   }
 
-  int adam(float lr) {
+  // the same with an Adam step on every layer: every dZ, which needs the old
+  // weights, before the weights' updates
+  int backward_adam(float lr) {
     ++adam_t;
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    const float c1 = 1.f - std::pow(b1, (float)adam_t), c2 = 1.f - std::pow(b2, (float)adam_t);
-    for (auto& y : L) {
-      k_adam<<<592, 256, 0, st>>>(y.w, y.mw, y.vw, y.gw, y.out, y.in, y.in_live, lr, b1, b2, eps, c1, c2, y.wb, y.wbT);
-      k_adam<<<8, 256, 0, st>>>(y.b, y.mb, y.vb, y.gb, 1, y.out, y.out, lr, b1, b2, eps, c1, c2, nullptr, nullptr);
+    GemmArgs p{};
+    p.lr = lr;
+    p.b1 = 0.9f;
+    p.b2 = 0.999f;
+    p.eps = 1e-8f;
+    p.c1 = 1.f - std::pow(p.b1, (float)adam_t);
+    p.c2 = 1.f - std::pow(p.b2, (float)adam_t);
+    for (int l = depth; l > 0; --l) MTRY(run_gemm(bwd_dx[l], st));
+    constexpr int bytes = Smem<64, STAGES_ADAM, 1, EPI_ADAM>::TOTAL;
+    MCK(cudaFuncSetAttribute((const void*)k_gemm_adam<64, STAGES_ADAM, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             bytes));
+    for (int l1 = depth; l1 >= 0; l1 -= GROUP) {
+      GroupArgs a{};
+      int tiles = 0;
+      for (int l = l1; l >= 0 && l > l1 - GROUP; --l, ++a.n) {
+        a.ta[a.n] = adam_dw[l].ta;
+        a.tb[a.n] = adam_dw[l].tb;
+        GemmArgs& g = a.g[a.n] = adam_dw[l].g;
+        g.lr = p.lr;
+        g.b1 = p.b1;
+        g.b2 = p.b2;
+        g.eps = p.eps;
+        g.c1 = p.c1;
+        g.c2 = p.c2;
+        a.end[a.n] = tiles += (g.M / BM) * (g.N / 64);
+      }
+      k_gemm_adam<64, STAGES_ADAM, 1><<<tiles, 128, bytes, st>>>(a);
       MCK(cudaGetLastError());
     }
+    for (int l0 = 0; l0 <= depth; l0 += BIAS_LAYERS) {
+      BiasArgs a{};
+      a.B = B;
+      int rows = 0;
+      for (int l = l0; l <= depth && l < l0 + BIAS_LAYERS; ++l, ++a.n) {
+        a.gT[a.n] = GT[l + 1];
+        a.b[a.n] = L[l].b;
+        a.m[a.n] = L[l].mb;
+        a.v[a.n] = L[l].vb;
+        a.end[a.n] = rows += L[l].out;
+      }
+      k_bias_adam<<<(rows + 7) / 8, 256, 0, st>>>(a, p);
+      MCK(cudaGetLastError());
+    }
+    return 0;
+  }
+
+  int gather(const float* x, const int* id) {
+    k_gather<<<B / 4, dim3(KPAD, 4), 0, st>>>(x, id, n_in, B, H[0], HT[0]);
+    MCK(cudaGetLastError());
     return 0;
   }
 
@@ -424,15 +475,10 @@ struct dgbgk_mlp {
   // buffers; rows past n repeat nothing meaningful (their inputs are zero
   // and their outputs are not read back)
   int load_batch_host(const float* x, const float* t, int n) {
-    if (n < B) {
-      MCK(cudaMemsetAsync(xin, 0, (size_t)B * n_in * 4, st));
-      MCK(cudaMemsetAsync(tin, 0, (size_t)B * n_out * 4, st));
-    }
+    if (n < B) MCK(cudaMemsetAsync(xin, 0, (size_t)B * n_in * 4, st));
     MCK(cudaMemcpyAsync(xin, x, (size_t)n * n_in * 4, cudaMemcpyHostToDevice, st));
     if (t) MCK(cudaMemcpyAsync(tin, t, (size_t)n * n_out * 4, cudaMemcpyHostToDevice, st));
-    k_gather<<<B, 128, 0, st>>>(xin, tin, iin, n_in, n_out, B, H[0], HT[0], T);
-    MCK(cudaGetLastError());
-    return 0;
+    return gather(xin, iin);
   }
 };
 
@@ -531,8 +577,8 @@ int dgbgk_mlp_gradient(dgbgk_mlp* m, const float* x, const float* t, int n, doub
   if (!m || !x || !t || n != m->B) return set_error("dgbgk_mlp_gradient: n must equal the batch size"), DGBGK_EINVAL;
   MCK(cudaSetDevice(m->device));
   MTRY(m->load_batch_host(x, t, n));
-  MTRY(m->forward());
-  MTRY(m->backward(m->loss));
+  MTRY(m->forward_loss(m->tin, m->iin, m->loss));
+  MTRY(m->backward());
   MTRY(m->check_err());
   if (loss) MCK(cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->st));
   if (grad) {
@@ -599,12 +645,10 @@ int dgbgk_mlp_train(dgbgk_mlp* m, int iters, float lr, unsigned long long seed, 
   }
   MCK(cudaMemcpyAsync(m->idx, id.data(), id.size() * sizeof(int), cudaMemcpyHostToDevice, m->st));
   for (int it = 0; it < iters; ++it) {
-    k_gather<<<B, 128, 0, m->st>>>(m->xs, m->ts, m->idx + (size_t)it * B, m->n_in, m->n_out, B, m->H[0], m->HT[0],
-                                    m->T);
-    MCK(cudaGetLastError());
-    MTRY(m->forward());
-    MTRY(m->backward(m->loss + it));
-    MTRY(m->adam(lr));
+    const int* id = m->idx + (size_t)it * B;
+    MTRY(m->gather(m->xs, id));
+    MTRY(m->forward_loss(m->ts, id, m->loss + it));
+    MTRY(m->backward_adam(lr));
   }
   MTRY(m->check_err());
   if (loss_hist) {

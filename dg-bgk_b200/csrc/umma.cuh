@@ -27,7 +27,6 @@ namespace umma {
 
 constexpr int BM = 128;        // tile rows (MMA M)
 constexpr int BK = 64;         // K-block: 64 BF16 = one 128-byte swizzle row
-constexpr int STAGES = 4;
 constexpr unsigned WAIT_TRIES = 1u << 22;
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -124,44 +123,95 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 
 // Epilogue modes
 enum Epi : int {
-  EPI_TANH = 0,      // Y = tanh(C + bias): Y (BF16, [M][N]) and Y^T (BF16, [N][M])
-  EPI_LINEAR = 1,    // Y = C + bias: FP32 [M][N]
-  EPI_DTANH = 2,     // G = C * (1 - y^2), y = aux (BF16 [M][N]): G (BF16 [M][N]) and G^T (BF16 [N][M])
-  EPI_F32 = 3,       // C: FP32 [M][N]
+  EPI_TANH = 0,    // Y = tanh(C + bias): Y (BF16, [M][N]) and Y^T (BF16, [N][M])
+  EPI_LINEAR = 1,  // Y = C + bias: FP32 [M][N]
+  EPI_DTANH = 2,   // G = C * (1 - y^2), y = aux (BF16 [M][N]): G (BF16 [M][N]) and G^T (BF16 [N][M])
+  EPI_F32 = 3,     // C: FP32 [M][N]
+  EPI_LOSS = 4,    // d = C + bias - t: G = scale*d (BF16 [M][N]) and G^T, the sum of d^2/(M N) added to *loss
+  EPI_ADAM = 5,    // C is the gradient of the weights w [M][N]: an Adam step on them and their BF16 copies
 };
 
 struct GemmArgs {
-  const float* bias;        // [N] (EPI_TANH, EPI_LINEAR)
-  const __nv_bfloat16* aux; // [M][N] (EPI_DTANH)
-  __nv_bfloat16* out_bf;    // [M][N]
-  __nv_bfloat16* out_bfT;   // [N][M]
-  float* out_f;             // [M][N]
-  int* err;                 // set when a bounded wait expired
+  const float* bias;         // [N] (EPI_TANH, EPI_LINEAR, EPI_LOSS)
+  const __nv_bfloat16* aux;  // [M][N] (EPI_DTANH)
+  __nv_bfloat16* out_bf;     // [M][N]
+  __nv_bfloat16* out_bfT;    // [N][M]
+  float* out_f;              // [M][N]
+  // EPI_LOSS: row r's targets are ts[idx[r]*N ..]
+  const float* ts;
+  const int* idx;
+  double* loss;
+  float scale;
+  // EPI_ADAM (out_bf, out_bfT: the weights' copies): columns from `live` on stay as they are
+  float *w, *m, *v;
+  int live;
+  float lr, b1, b2, eps, c1, c2;
+  int* err;  // set when a bounded wait expired
   int M, N, K;
-  int epi;
 };
 
-template <int BN>
+// One Adam update of a weight and its moments.  The fused multiply-adds are
+// written out: left to the compiler, the two places that inline this could
+// round the moments differently, and BF16 copies of weights a last bit apart
+// send a training run its own way.
+__device__ __forceinline__ float adam_step(float x, float& m, float& v, float g, const GemmArgs& a) {
+  m = __fmaf_rn(1.f - a.b1, g, __fmul_rn(a.b1, m));
+  v = __fmaf_rn((1.f - a.b2) * g, g, __fmul_rn(a.b2, v));
+  return x - a.lr * (m / a.c1) / (sqrtf(v / a.c2) + a.eps);
+}
+
+// One thread of a converged warp.  The loops of the copying and of the
+// issuing thread take this and not lane == 0: the tensor instructions' operands
+// are uniform registers, and where the compiler cannot see that one thread is
+// active it moves them there anew for each instruction (K-block of 64, tile of
+// 128 x 32: 0.29 -> 0.19 us).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(r));
+  return r != 0;
+}
+
+// A stage holds SUB K-blocks.
+template <int BN, int STAGES, int SUB, int EPI>
 struct Smem {
   static constexpr int A_BYTES = BM * BK * 2;  // 16 KB
   static constexpr int B_BYTES = BN * BK * 2;
-  static constexpr int STAGE = A_BYTES + B_BYTES;
-  static constexpr int TOTAL = 1024 + STAGES * STAGE;  // + 1024 alignment slack
+  static constexpr int BLOCK = A_BYTES + B_BYTES;
+  static constexpr int STAGE = SUB * BLOCK;
+  // EPI_ADAM, in the ring's place once the accumulator is complete: the tile
+  // in FP32 (pitch BN + 4 floats: 16-byte rows on shifted banks) and the new
+  // weights transposed in BF16 (pitch BM + 2: neighbouring columns on
+  // neighbouring banks)
+  static constexpr int PF = BN + 4, PT = BM + 2;
+  static constexpr int EPILOGUE = EPI == EPI_ADAM ? BM * PF * 4 + BN * PT * 2 : 0;
+  static constexpr int RING = STAGES * STAGE;
+  static constexpr int TOTAL = 1024 + (RING > EPILOGUE ? RING : EPILOGUE);  // + 1024 alignment slack
 };
 
-// C tile (blockIdx.y * 128, blockIdx.x * BN).  M, N, K: multiples of 128, BN, 64.
-template <int BN>
-__global__ void __launch_bounds__(128, 1) k_gemm(const __grid_constant__ CUtensorMap ta,
-                                                 const __grid_constant__ CUtensorMap tb, GemmArgs g) {
+__device__ __forceinline__ uint32_t bf16x2(float a, float b) {
+  const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&p);
+}
+
+// C tile (m0, n0) by the CTA's 128 threads.  M, N, K: multiples of 128, BN,
+// 64*SUB.
+template <int BN, int STAGES, int SUB, int EPI>
+__device__ __forceinline__ void gemm_tile(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, int m0,
+                                          int n0) {
   static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "MMA N");
+  using S = Smem<BN, STAGES, SUB, EPI>;
   extern __shared__ __align__(1024) unsigned char sm_raw[];
   __shared__ uint64_t full[STAGES], empty[STAGES], done;
   __shared__ uint32_t tmem_base;
   __shared__ int fail, issued, consumed;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  __shared__ double red[4];
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   unsigned char* base = sm_raw + ((1024u - (saddr(sm_raw) & 1023u)) & 1023u);
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int nk = g.K / BK;
+  const int nk = g.K / (BK * SUB);
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       bar_init(&full[s], 1);
@@ -179,37 +229,59 @@ __global__ void __launch_bounds__(128, 1) k_gemm(const __grid_constant__ CUtenso
   fence_after();
   const uint32_t tmem = tmem_base;
 
-  if (warp == 0 && lane == 0) {
-    // producer: K-block kb into stage kb % STAGES once the MMAs of
-    // kb - STAGES have released it
+  if (warp == 0 && elect_one()) {
+    // producer: stage s = kb % STAGES once the MMAs of kb - STAGES have
+    // released it (ph: parity of the round over the ring)
+    int s = 0;
+    uint32_t ph = 0;
     for (int kb = 0; kb < nk; ++kb) {
-      const int s = kb % STAGES;
-      if (kb >= STAGES && !bar_wait(&empty[s], ((kb / STAGES) - 1) & 1)) {
+      if (kb >= STAGES && !bar_wait(&empty[s], ph ^ 1u)) {
         fail = 1;
         break;
       }
-      unsigned char* st = base + s * Smem<BN>::STAGE;
-      bar_expect(&full[s], Smem<BN>::STAGE);
-      tma2d(st, &ta, kb * BK, m0, &full[s]);
-      tma2d(st + Smem<BN>::A_BYTES, &tb, kb * BK, n0, &full[s]);
+      unsigned char* st = base + s * S::STAGE;
+      bar_expect(&full[s], S::STAGE);
+#pragma unroll
+      for (int u = 0; u < SUB; ++u) {
+        tma2d(st + u * S::BLOCK, &ta, (kb * SUB + u) * BK, m0, &full[s]);
+        tma2d(st + u * S::BLOCK + S::A_BYTES, &tb, (kb * SUB + u) * BK, n0, &full[s]);
+      }
       issued = kb + 1;
+      if (++s == STAGES) {
+        s = 0;
+        ph ^= 1u;
+      }
     }
-  } else if (warp == 1 && lane == 0) {
-    // MMA issuer
+  } else if (warp == 1 && elect_one()) {
+    // MMA issuer; the descriptors' address fields (16-byte units) are advanced
+    // by additions.  A K-block of 64 took 0.32 us whatever the tile's width and
+    // the ring's depth, most of it this thread's; with both changes above and
+    // two K-blocks a stage 0.145 us (128 x 32 tile, 141 GB/s into the SM).
     constexpr uint32_t idesc = idesc_bf16(BM, BN);
+    const uint64_t ad0 = sdesc(base, 0), bd0 = sdesc(base + S::A_BYTES, 0);
+    uint64_t off = 0;
+    int s = 0;
+    uint32_t ph = 0;
     for (int kb = 0; kb < nk; ++kb) {
-      const int s = kb % STAGES;
-      if (!bar_wait(&full[s], (kb / STAGES) & 1)) {
+      if (!bar_wait(&full[s], ph)) {
         fail = 1;
         break;
       }
       fence_after();
-      const unsigned char* st = base + s * Smem<BN>::STAGE;
 #pragma unroll
-      for (int k = 0; k < BK / 16; ++k)
-        mma_bf16(tmem, sdesc(st, 32 * k), sdesc(st + Smem<BN>::A_BYTES, 32 * k), idesc, (kb | k) ? 1u : 0u);
+      for (int u = 0; u < SUB; ++u)
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k)
+          mma_bf16(tmem, ad0 + off + u * (S::BLOCK >> 4) + 2 * k, bd0 + off + u * (S::BLOCK >> 4) + 2 * k, idesc,
+                   (kb | u | k) ? 1u : 0u);
       mma_commit(&empty[s]);  // the stage is free once these MMAs have read it
       consumed = kb + 1;
+      off += S::STAGE >> 4;
+      if (++s == STAGES) {
+        s = 0;
+        off = 0;
+        ph ^= 1u;
+      }
     }
     mma_commit(&done);  // the accumulator is complete
   }
@@ -224,32 +296,123 @@ __global__ void __launch_bounds__(128, 1) k_gemm(const __grid_constant__ CUtenso
       // the box copies still in flight land before the CTA leaves (bounded)
       for (int kb = consumed; kb < issued; ++kb) bar_wait(&full[kb % STAGES], (kb / STAGES) & 1);
     }
+  } else if constexpr (EPI == EPI_ADAM) {
+    // the gradient tile to shared memory (rows of the accumulator are lanes),
+    // then whole rows of the weights and moments, BN/4 lanes a row
+    float* const sf = reinterpret_cast<float*>(base);
+    __nv_bfloat16* const stp = reinterpret_cast<__nv_bfloat16*>(base + BM * S::PF * 4);
+    {
+      const int row = 32 * warp + lane;
+      for (int c0 = 0; c0 < BN; c0 += 32) {
+        float v[32];
+        tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
+#pragma unroll
+        for (int i = 0; i < 32; i += 4)
+          *reinterpret_cast<float4*>(sf + row * S::PF + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+      }
+    }
+    __syncwarp();  // a warp reads the rows it has written
+    constexpr int LPR = BN / 4, RPI = 32 / LPR, UR = 4;  // lanes a row, rows an instruction, rows in flight / RPI
+    static_assert(32 % LPR == 0 && 32 % (RPI * UR) == 0, "rows of a warp");
+    const int cl = 4 * (lane % LPR), rl = lane / LPR;
+    for (int r0 = 0; r0 < 32; r0 += RPI * UR) {
+      float4 x[UR], mm[UR], vv[UR];
+#pragma unroll
+      for (int u = 0; u < UR; ++u) {
+        const size_t o = (size_t)(m0 + 32 * warp + r0 + u * RPI + rl) * g.N + n0 + cl;
+        x[u] = *reinterpret_cast<const float4*>(g.w + o);
+        mm[u] = *reinterpret_cast<const float4*>(g.m + o);
+        vv[u] = *reinterpret_cast<const float4*>(g.v + o);
+      }
+#pragma unroll
+      for (int u = 0; u < UR; ++u) {
+        const int row = 32 * warp + r0 + u * RPI + rl;
+        const float4 gr = *reinterpret_cast<const float4*>(sf + row * S::PF + cl);
+        if (n0 + cl + 3 < g.live) {
+          x[u].x = adam_step(x[u].x, mm[u].x, vv[u].x, gr.x, g);
+          x[u].y = adam_step(x[u].y, mm[u].y, vv[u].y, gr.y, g);
+          x[u].z = adam_step(x[u].z, mm[u].z, vv[u].z, gr.z, g);
+          x[u].w = adam_step(x[u].w, mm[u].w, vv[u].w, gr.w, g);
+        } else {
+          if (n0 + cl < g.live) x[u].x = adam_step(x[u].x, mm[u].x, vv[u].x, gr.x, g);
+          if (n0 + cl + 1 < g.live) x[u].y = adam_step(x[u].y, mm[u].y, vv[u].y, gr.y, g);
+          if (n0 + cl + 2 < g.live) x[u].z = adam_step(x[u].z, mm[u].z, vv[u].z, gr.z, g);
+        }
+        const size_t o = (size_t)(m0 + row) * g.N + n0 + cl;
+        *reinterpret_cast<float4*>(g.w + o) = x[u];
+        *reinterpret_cast<float4*>(g.m + o) = mm[u];
+        *reinterpret_cast<float4*>(g.v + o) = vv[u];
+        uint2 b;
+        b.x = bf16x2(x[u].x, x[u].y);
+        b.y = bf16x2(x[u].z, x[u].w);
+        *reinterpret_cast<uint2*>(g.out_bf + o) = b;
+        __nv_bfloat16* t = stp + cl * S::PT + row;
+        t[0] = __float2bfloat16_rn(x[u].x);
+        t[S::PT] = __float2bfloat16_rn(x[u].y);
+        t[2 * S::PT] = __float2bfloat16_rn(x[u].z);
+        t[3 * S::PT] = __float2bfloat16_rn(x[u].w);
+      }
+    }
+    __syncthreads();
+    // the transposed copy: a warp writes a column's 128 rows
+    for (int c = warp; c < BN; c += 4) {
+      const uint32_t* src = reinterpret_cast<const uint32_t*>(stp + c * S::PT);
+      uint32_t* dst = reinterpret_cast<uint32_t*>(g.out_bfT + (size_t)(n0 + c) * g.M + m0);
+      dst[lane] = src[lane];
+      dst[lane + 32] = src[lane + 32];
+    }
   } else {
     // epilogue: row m0 + 32*warp + lane, 32 columns at a time
     const int row = m0 + 32 * warp + lane;
+    double sq = 0.0;
+    const float* trow = EPI == EPI_LOSS ? g.ts + (size_t)g.idx[row] * g.N : nullptr;
     for (int c0 = 0; c0 < BN; c0 += 32) {
       float v[32];
-      tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
       const int col = n0 + c0;
-      if (g.epi == EPI_TANH || g.epi == EPI_LINEAR) {
+      float4 t4[8];
+      if (EPI == EPI_LOSS) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t4[i] = *reinterpret_cast<const float4*>(trow + col + 4 * i);
+      }
+      tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
+      if (EPI == EPI_TANH || EPI == EPI_LINEAR || EPI == EPI_LOSS) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] += g.bias[col + i];
       }
-      if (g.epi == EPI_TANH) {
+      if (EPI == EPI_TANH) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = tanhf(v[i]);
-      } else if (g.epi == EPI_DTANH) {
-        const __nv_bfloat16* y = g.aux + (size_t)row * g.N + col;
+      } else if (EPI == EPI_DTANH) {
+        const uint4* y = reinterpret_cast<const uint4*>(g.aux + (size_t)row * g.N + col);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float yy = __bfloat162float(y[i]);
-          v[i] *= 1.f - yy * yy;
+        for (int i = 0; i < 4; ++i) {
+          const uint4 q = y[i];
+          const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float lo = __uint_as_float(w[k] << 16), hi = __uint_as_float(w[k] & 0xffff0000u);
+            v[8 * i + 2 * k] *= 1.f - lo * lo;
+            v[8 * i + 2 * k + 1] *= 1.f - hi * hi;
+          }
+        }
+      } else if (EPI == EPI_LOSS) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float t[4] = {t4[i].x, t4[i].y, t4[i].z, t4[i].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float d = v[4 * i + k] - t[k];
+            sq += (double)d * d;
+            v[4 * i + k] = g.scale * d;
+          }
         }
       }
-      if (g.epi == EPI_TANH || g.epi == EPI_DTANH) {
-        __nv_bfloat16* o = g.out_bf + (size_t)row * g.N + col;
+      if (EPI == EPI_TANH || EPI == EPI_DTANH || EPI == EPI_LOSS) {
+        uint4* o = reinterpret_cast<uint4*>(g.out_bf + (size_t)row * g.N + col);
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) *reinterpret_cast<__nv_bfloat162*>(o + i) = __floats2bfloat162_rn(v[i], v[i + 1]);
+        for (int i = 0; i < 4; ++i)
+          o[i] = make_uint4(bf16x2(v[8 * i], v[8 * i + 1]), bf16x2(v[8 * i + 2], v[8 * i + 3]),
+                            bf16x2(v[8 * i + 4], v[8 * i + 5]), bf16x2(v[8 * i + 6], v[8 * i + 7]));
         // transposed copy: for a fixed column the 32 lanes write 32 consecutive rows
 #pragma unroll
         for (int i = 0; i < 32; ++i) g.out_bfT[(size_t)(col + i) * g.M + row] = __float2bfloat16_rn(v[i]);
@@ -259,10 +422,43 @@ __global__ void __launch_bounds__(128, 1) k_gemm(const __grid_constant__ CUtenso
         for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
       }
     }
+    if (EPI == EPI_LOSS) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      if (lane == 0) red[warp] = sq;
+      __syncthreads();
+      if (tid == 0) atomicAdd(g.loss, (red[0] + red[1] + red[2] + red[3]) / ((double)g.M * (double)g.N));
+    }
   }
   fence_before();
   __syncthreads();
   if (warp == 0) tmem_free(tmem, BN);
+}
+
+// one GEMM: tile (blockIdx.y, blockIdx.x)
+template <int BN, int STAGES, int SUB, int EPI>
+__global__ void __launch_bounds__(128, 1) k_gemm(const __grid_constant__ CUtensorMap ta,
+                                                 const __grid_constant__ CUtensorMap tb,
+                                                 const __grid_constant__ GemmArgs g) {
+  gemm_tile<BN, STAGES, SUB, EPI>(ta, tb, g, blockIdx.y * BM, blockIdx.x * BN);
+}
+
+// The weight gradients of up to GROUP layers with their Adam steps in one
+// launch, so that the few tiles of the hidden layers run beside the output
+// layer's.
+constexpr int GROUP = 8;
+struct GroupArgs {
+  CUtensorMap ta[GROUP], tb[GROUP];
+  GemmArgs g[GROUP];
+  int end[GROUP];  // running sum of the layers' tiles
+  int n;
+};
+template <int BN, int STAGES, int SUB>
+__global__ void __launch_bounds__(128, 4) k_gemm_adam(const __grid_constant__ GroupArgs a) {
+  int l = 0;
+  while ((int)blockIdx.x >= a.end[l]) ++l;
+  const int t = blockIdx.x - (l ? a.end[l - 1] : 0), nt = a.g[l].N / BN;
+  gemm_tile<BN, STAGES, SUB, EPI_ADAM>(a.ta[l], a.tb[l], a.g[l], t / nt * BM, t % nt * BN);
 }
 
 }  // namespace umma
