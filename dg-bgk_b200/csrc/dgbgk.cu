@@ -336,6 +336,7 @@ int build_launch_set(LaunchSet<T>& L, const std::vector<CaseDev<T>>& cs, int eb,
   L.args.wall_off = L.d_off + 2 * (n + 1);
   L.args.ctl = L.d_ctl;
   L.args.ncases = n;
+  L.args.fuse_resid = L.spec_cases.empty() ? 1 : 0;
   L.args.max_halo = max_halo;
   L.args.mom_rowbytes = maxrow;
   // moments: persistent grid
@@ -367,6 +368,26 @@ inline int launch_check(const char* what, int grid, int block, size_t smem) {
   return DGBGK_ECUDA;
 }
 
+// Launch with programmatic dependence on the kernel before it in the stream
+// (the kernel waits by itself, grid_wait): its launch and everything it does
+// before that wait pass while the other one ends.
+template <class... P, class... A>
+int launch_dependent(const char* what, void (*fn)(P...), int grid, int block, size_t smem, cudaStream_t st,
+                     const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, fn, args...);
+  return launch_check(what, grid, block, smem);
+}
+
 // One pseudo-time step of every case of the set: moments, wall flux, sweep,
 // residual bookkeeping.
 template <class T>
@@ -385,9 +406,8 @@ int enqueue_step(const LaunchSet<T>& L, cudaStream_t st, float* ms = nullptr, co
     TRY(launch_check("k_wall", L.total_walls, WALL_THREADS, 0));
     CK(cudaEventRecord(L.ev_join, L.st_wall));
   }
-  mom_fn<T>(L.mom_rows, L.one)<<<L.mom_grid, L.mom_warps * 32, L.mom_smem, st>>>(L.args, L.total_groups,
-                                                                                 L.one_case);
-  TRY(launch_check("k_moments", L.mom_grid, L.mom_warps * 32, L.mom_smem));
+  TRY(launch_dependent("k_moments", mom_fn<T>(L.mom_rows, L.one), L.mom_grid, L.mom_warps * 32, L.mom_smem, st,
+                       L.args, L.total_groups, L.one_case));
   if (out) {  // the previous step's GETMAC / GETFOR record, when due
     const int g = (out->nod.NP + 255) / 256;
     k_out_nodal<<<g, 256, 0, st>>>(*out);
@@ -404,8 +424,8 @@ int enqueue_step(const LaunchSet<T>& L, cudaStream_t st, float* ms = nullptr, co
   }
   if (ms) cudaEventRecord(ev[2], st);
   const int snt = SweepGeo<T>::threads(L.eb);
-  sweep_fn<T>(L.eb, L.immat, L.one)<<<L.sweep_grid, snt, L.sweep_smem, st>>>(L.args, L.total_units, L.one_case);
-  TRY(launch_check("k_sweep", L.sweep_grid, snt, L.sweep_smem));
+  TRY(launch_dependent("k_sweep", sweep_fn<T>(L.eb, L.immat, L.one), L.sweep_grid, snt, L.sweep_smem, st, L.args,
+                       L.total_units, L.one_case));
   // the specular part of ALPHA < 1 wall sides: the parallel items, then the
   // ones that wait on earlier deferred velocities
   for (const auto& c : L.spec_cases) {
@@ -421,8 +441,10 @@ int enqueue_step(const LaunchSet<T>& L, cudaStream_t st, float* ms = nullptr, co
     }
   }
   if (ms) cudaEventRecord(ev[3], st);
-  k_resid<T><<<L.n, 32, 0, st>>>(L.args);
-  TRY(launch_check("k_resid", L.n, 32, 0));
+  if (!L.args.fuse_resid) {
+    k_resid<T><<<L.n, 32, 0, st>>>(L.args);
+    TRY(launch_check("k_resid", L.n, 32, 0));
+  }
   if (ms) {
     cudaEventRecord(ev[4], st);
     cudaEventSynchronize(ev[4]);
@@ -431,6 +453,46 @@ int enqueue_step(const LaunchSet<T>& L, cudaStream_t st, float* ms = nullptr, co
   }
   return 0;
 }
+
+// Captured steps: a graph of GRAPH_STEPS pseudo-time steps and one of a
+// single step, each captured when it is first needed (the buffer swap is on
+// the device, so one graph serves every step).  Four steps a graph: the gap
+// between two graphs is longer than that between two steps of one, and a
+// shorter call does not run steps past its end.
+constexpr int GRAPH_STEPS = 4;
+constexpr int POLL_STEPS = 64;  // steps between two looks at the done flag
+struct StepGraphs {
+  cudaGraphExec_t exec[2] = {nullptr, nullptr};  // 1 step, GRAPH_STEPS steps
+  void drop() {
+    for (auto& e : exec) {
+      if (e) cudaGraphExecDestroy(e);
+      e = nullptr;
+    }
+  }
+  // the graphs that n steps need
+  template <class F> int prepare(cudaStream_t st, int n, F enqueue) {
+    for (int which = 0; which < 2; ++which) {
+      if (exec[which] || (which ? n < GRAPH_STEPS : n % GRAPH_STEPS == 0)) continue;
+      cudaGraph_t g;
+      CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+      int rc = 0;
+      for (int i = 0; i < (which ? GRAPH_STEPS : 1) && rc == 0; ++i) rc = enqueue();
+      const cudaError_t e = cudaStreamEndCapture(st, &g);
+      if (rc != 0) return rc;
+      CK(e);
+      const cudaError_t ei = cudaGraphInstantiate(&exec[which], g, 0);
+      cudaGraphDestroy(g);
+      if (ei != cudaSuccess) exec[which] = nullptr;
+      CK(ei);
+    }
+    return 0;
+  }
+  int run(cudaStream_t st, int n) const {
+    for (; n >= GRAPH_STEPS; n -= GRAPH_STEPS) CK(cudaGraphLaunch(exec[1], st));
+    for (; n > 0; --n) CK(cudaGraphLaunch(exec[0], st));
+    return 0;
+  }
+};
 
 // Reduced-rank extrapolation coefficients from the m x m Gram matrix G of
 // the snapshot differences (upper triangle accumulated by k_gram): solve
@@ -479,10 +541,9 @@ int rre_coeffs(std::vector<double>& G, int m, std::vector<double>& g) {
 }
 
 template <class T> struct Impl : ImplBase {
-  static constexpr int GRAPH_STEPS = 2;  // pseudo-time steps per graph launch
   cudaStream_t st = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, evpoll[2] = {nullptr, nullptr};
-  cudaGraphExec_t gexec = nullptr;
+  StepGraphs graphs;
   int cur = 0;  // host copy of Ctrl::cur
   int tpu = 1;  // velocity tiles per sweep work unit
   int Vp = 0;
@@ -828,29 +889,7 @@ template <class T> struct Impl : ImplBase {
     return 0;
   }
 
-  void drop_graphs() {
-    if (gexec) {
-      cudaGraphExecDestroy(gexec);
-      gexec = nullptr;
-    }
-  }
-  // GRAPH_STEPS pseudo-time steps as one graph (the buffer swap is on the
-  // device, so one graph serves every step)
-  int build_graph() {
-    if (gexec) return 0;
-    cudaGraph_t g;
-    CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    int rc = 0;
-    const OutArgs oa = out_args(-1, nullptr);
-    for (int k = 0; k < GRAPH_STEPS && rc == 0; ++k) rc = enqueue_step(single, st, nullptr, out_every > 0 ? &oa : nullptr);
-    cudaError_t e = cudaStreamEndCapture(st, &g);
-    if (rc != 0) return rc;
-    CK(e);
-    CK(cudaGraphInstantiate(&gexec, g, 0));
-    cudaGraphDestroy(g);
-    return 0;
-  }
-
+  void drop_graphs() { graphs.drop(); }
   void fill_ctrl(Ctrl& h, int max_steps, double tol) const {
     std::memset(&h, 0, sizeof(Ctrl));
     h.max_steps = max_steps;
@@ -920,12 +959,14 @@ template <class T> struct Impl : ImplBase {
     } else if (k == 3) {
       const int nt = std::max(n3, (int)pl.walls.size());
       k_shard_fin<T><<<(nt + 255) / 256, 256, 0, st>>>(C, sums1, sums2);
+      BatchArgs<T> args = single.args;
+      args.fuse_resid = 0;  // phase 4, with the residual of every shard
       sweep_fn<T>(single.eb, single.immat, true)<<<single.sweep_grid, SweepGeo<T>::threads(single.eb),
-                                                   single.sweep_smem, st>>>(single.args, single.total_units,
+                                                   single.sweep_smem, st>>>(args, single.total_units,
                                                                             single.one_case);
       k_shard_respart<T><<<1, 32, 0, st>>>(C, res);
     } else if (k == 4) {
-      k_shard_resid<T><<<1, 32, 0, st>>>(C, res, single.args.ctl);
+      k_shard_resid<T><<<1, 32, 0, st>>>(C, res);
     } else if (k == 0) {  // before phases 1, 2 and 5 outside a step: the kernels run
       TRY(aux_ctrl());
     } else if (k == 5) {  // the moments of the current state from the summed sums (no sweep)
@@ -967,16 +1008,15 @@ template <class T> struct Impl : ImplBase {
     if (max_steps == 0) return 0;
     CK(cudaSetDevice(device));
     TRY(ensure_hist(max_steps));
-    TRY(build_graph());
+    const OutArgs oa = out_args(-1, nullptr);
+    TRY(graphs.prepare(st, max_steps, [&] { return enqueue_step(single, st, nullptr, out_every > 0 ? &oa : nullptr); }));
     TRY(upload_ctrl(max_steps, tol));
     CK(cudaEventRecord(ev0, st));
-    const int launches = (max_steps + GRAPH_STEPS - 1) / GRAPH_STEPS;
-    const int chunk = 32;
     int issued = 0, chunks = 0;
     bool stop = false;
-    while (issued < launches && !stop) {
-      const int n = std::min(chunk, launches - issued);
-      for (int i = 0; i < n; ++i) CK(cudaGraphLaunch(gexec, st));
+    while (issued < max_steps && !stop) {
+      const int n = std::min(POLL_STEPS, max_steps - issued);
+      TRY(graphs.run(st, n));
       issued += n;
       const int slot = 1 + (chunks & 1);
       CK(cudaMemcpyAsync(&hctrl[slot], ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, st));
@@ -1700,13 +1740,12 @@ struct BatchBase {
 };
 
 template <class T> struct BatchImpl : BatchBase {
-  static constexpr int GRAPH_STEPS = 2;
   std::vector<Impl<T>*> cs;
   LaunchSet<T> L;
   int device = 0, nsm = 148, eb = 128, upc = 8, immat = 1, max_halo = 0;
   cudaStream_t st = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, evp[2] = {nullptr, nullptr};
-  cudaGraphExec_t gexec = nullptr;
+  StepGraphs graphs;
   int* d_done = nullptr;
   int* h_done = nullptr;  // pinned [2]
   double* h_l2 = nullptr;  // pinned [ncases]: the cases' last L2 residuals
@@ -1729,7 +1768,7 @@ template <class T> struct BatchImpl : BatchBase {
   ~BatchImpl() override {
     cudaSetDevice(device);
     if (st) cudaStreamSynchronize(st);
-    if (gexec) cudaGraphExecDestroy(gexec);
+    graphs.drop();
     L.release();
     dfree(d_done);
     if (h_done) cudaFreeHost(h_done);
@@ -1808,10 +1847,7 @@ template <class T> struct BatchImpl : BatchBase {
     for (auto* c : cs) gens.push_back(c->gen);
     eb = e;
     upc = u;
-    if (gexec) {
-      cudaGraphExecDestroy(gexec);
-      gexec = nullptr;
-    }
+    graphs.drop();
     return 0;
   }
 
@@ -1912,20 +1948,6 @@ template <class T> struct BatchImpl : BatchBase {
     return configure(beb, bupc);
   }
 
-  int build_graph() {
-    if (gexec) return 0;
-    cudaGraph_t g;
-    CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    int rc = 0;
-    for (int k = 0; k < GRAPH_STEPS && rc == 0; ++k) rc = enqueue_step(L, st);
-    cudaError_t e = cudaStreamEndCapture(st, &g);
-    if (rc != 0) return rc;
-    CK(e);
-    CK(cudaGraphInstantiate(&gexec, g, 0));
-    cudaGraphDestroy(g);
-    return 0;
-  }
-
   int advance(int max_steps, double tol, int* steps, double* l2) override {
     if (max_steps < 0) {
       set_error("max_steps < 0");
@@ -1941,16 +1963,14 @@ template <class T> struct BatchImpl : BatchBase {
     for (size_t i = 0; i < cs.size() && !stale; ++i) stale = gens[i] != cs[i]->gen;
     if (stale) TRY(configure(eb, upc));
     for (auto* c : cs) CK(cudaStreamSynchronize(c->st));
-    TRY(build_graph());
+    TRY(graphs.prepare(st, max_steps, [&] { return enqueue_step(L, st); }));
     TRY(upload_ctrls(max_steps, tol));
     CK(cudaEventRecord(ev0, st));
-    const int launches = max_steps > 0 ? (max_steps + GRAPH_STEPS - 1) / GRAPH_STEPS : 0;
-    const int chunk = 32;
     int issued = 0, chunks = 0;
     bool stop = false;
-    while (issued < launches && !stop) {
-      const int n = std::min(chunk, launches - issued);
-      for (int i = 0; i < n; ++i) CK(cudaGraphLaunch(gexec, st));
+    while (issued < max_steps && !stop) {
+      const int n = std::min(POLL_STEPS, max_steps - issued);
+      TRY(graphs.run(st, n));
       issued += n;
       k_all_done<T><<<1, 256, 0, st>>>(L.args, d_done);
       CK(cudaGetLastError());

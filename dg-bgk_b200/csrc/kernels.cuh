@@ -1,7 +1,7 @@
 // sm_100a kernels of the DG-BGK pseudo-time step.
 //
-// One step (src/advnce.f90:220-400) is four launches on one stream (five
-// with ALPHA < 1: k_wspec after the sweep):
+// One step (src/advnce.f90:220-400) is three launches (with ALPHA < 1 also
+// k_wspec and k_resid after the sweep):
 //   k_moments : MACROS passes 1+2 (src/macros.f90:80-154) fused with COMPMU
 //               (src/compmu.f90:36-97) and the GTEQNF parameters
 //               (src/gteqnf.f90:26-40).  Persistent warps take R whole
@@ -18,8 +18,9 @@
 //               once per unit, the tiles' f rows arrive by cp.async,
 //               double-buffered, and eight lanes share an element, each at 4
 //               (FP32, packed pairs) or 2 (FP64) velocities.
-//   k_resid   : GETRES + the residual bookkeeping (src/advnce.f90:385,
-//               422-429), the convergence test and the step counter.
+//               Its last CTA does GETRES + the residual bookkeeping
+//               (src/advnce.f90:385, 422-429), the convergence test and the
+//               step counter.
 // Every device-side wait on an mbarrier is bounded: on expiry the kernel
 // sets Ctrl::timeout, drains its own copies with a second bounded wait and
 // returns; the host reports DGBGK_ECUDA.
@@ -37,6 +38,16 @@ constexpr double PI_D = 3.1416;  // the reference's PI
 constexpr double TINY_D = 1e-20;
 constexpr double LOG2E_D = 1.4426950408889634;  // log2(e)
 constexpr unsigned WAIT_TRIES = 1u << 22;  // x ~256 ns sleep: ~1 s
+
+// Programmatic dependent launch: the next kernel of the stream may start (its
+// CTAs as this one's leave their SMs) once every CTA has called this or left;
+// what it then does before grid_wait must not touch anything an earlier kernel
+// writes.
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// ... and waits here until the kernels before it are complete
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -192,6 +203,7 @@ template <class T> struct BatchArgs {
   int ncases;
   int max_halo;             // over the cases (sweep tile layout)
   int sweep_bufs;           // sweep tile buffers, 2 or (a wide halo) 1
+  int fuse_resid;           // the sweep's last CTA does the step's bookkeeping (else k_resid)
   int mom_stages;           // moment ring stages per warp
   unsigned mom_rowbytes;    // moment ring row size (max over the cases)
 };
@@ -575,6 +587,8 @@ __global__ void __launch_bounds__(ONE ? 640 : 512, 1)
     fence_mbar_init();
   }
   __syncthreads();
+  grid_launch_dependents();
+  grid_wait();  // the state, the control blocks
   // lane 0: the rows of group g into stage s (none when the case is done)
   auto fill = [&](int s, int g) {
     const int c = ONE ? 0 : find_case(a.grp_off, a.ncases, g);
@@ -765,6 +779,33 @@ __device__ __forceinline__ double step_dt(const Ctrl* c) {
   return fmin(dtb, dtc);
 }
 
+// ----------------------------------------------------------- residual ----
+// GETRES + the residual bookkeeping (src/advnce.f90:385, 422-429) per case,
+// one thread per case: the step's max and L2 residual into the history, the
+// non-finite and convergence tests, the step counter and the buffer swap;
+// the step's accumulators are cleared for the next step.  The sweep's last
+// CTA runs it (or k_resid).
+template <class T> __device__ __forceinline__ void resid_book(const CaseDev<T>& C, double mm, double sq) {
+  Ctrl* c = C.ctrl;
+  const int st = c->step;
+  const double l2 = sqrt(sq);
+  C.hist_linf[st] = mm;
+  C.hist_l2[st] = l2;
+  C.hist_dt[st] = step_dt(c);
+  if (!isfinite(l2) || !isfinite(mm)) {
+    c->nonfinite = 1;
+    c->done = 1;
+  }
+  if (c->timeout) c->done = 1;
+  if (c->ref == 0.0 && l2 > 0.0) c->ref = l2;
+  c->acc_sq = 0.0;
+  c->acc_max = 0.0;
+  c->maxmu = 0.0;
+  c->cur ^= 1;
+  c->step = st + 1;
+  if (c->step >= c->max_steps) c->done = 1;
+  if (c->tol > 0.0 && l2 <= c->tol * c->ref) c->done = 1;
+}
 // Sweep geometry.  LPE = 8 lanes share an element, each with one 16-byte
 // vector of velocities (4 FP32 or 2 FP64), so a warp works on EPW = 4
 // elements at 32 (16) velocities and every row access -- global or shared --
@@ -1048,7 +1089,7 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
   // (a unit of a finished case has no barrier of its own: with one slot,
   // thread 0 could loop round and replace the value before a slow warp read
   // it, and the warps would then disagree on the unit and on the barriers)
-  __shared__ int s_unit[2];
+  __shared__ int s_unit[2], s_last;
   __shared__ double red_m[NW], red_s[NW];
   // FP64: the 2^(j/64) table of the NFO exp (one entry for FP32, unused)
   __shared__ double etab[sizeof(T) == 8 ? EXP_TAB : 1];
@@ -1081,6 +1122,8 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
     cur = ctl->cur;
     dtd = step_dt(ctl);
   };
+  grid_launch_dependents();
+  grid_wait();  // the moments and walls, the control blocks, the unit counter
   if (ONE) control(one.ctrl);
   // the unit after this one, drawn ahead so the atomic's latency is hidden
   int next = (tid == 0 && unit < total_units) ? (int)gridDim.x + atomicAdd(&a.ctl->sweep_next, 1) : 0;
@@ -1449,6 +1492,31 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
     __syncthreads();
     if (tid == 0) resid_add<NW>(one.ctrl, red_m, red_s);
   }
+  // the last CTA to get here: every residual has been added and every unit
+  // drawn, so the counters go back to zero and (fuse_resid) the cases' step is
+  // booked here; as a launch of its own that took 2.5 us of each step
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(&a.ctl->sweep_done, 1) == (int)gridDim.x - 1;
+    if (s_last) {
+      __threadfence();
+      a.ctl->sweep_next = 0;
+      a.ctl->sweep_done = 0;
+    }
+  }
+  if (!a.fuse_resid) return;
+  if (ONE) {
+    if (tid != 0 || !s_last || one.ctrl->done) return;
+    resid_book(one, __ldcg(&one.ctrl->acc_max), __ldcg(&one.ctrl->acc_sq));
+  } else {
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int k = tid; k < a.ncases; k += NT) {
+      const CaseDev<T>& C = a.cases[k];
+      if (!C.ctrl->done) resid_book(C, __ldcg(&C.ctrl->acc_max), __ldcg(&C.ctrl->acc_sq));
+    }
+  }
 }
 
 // ------------------------------------------------ specular wall part ----
@@ -1541,35 +1609,10 @@ template <class T> __global__ void __launch_bounds__(256) k_wspec(const __grid_c
   }
 }
 
-// ----------------------------------------------------------- residual ----
-// GETRES + the residual bookkeeping (src/advnce.f90:385, 422-429) per case,
-// one thread per case: the step's max and L2 residual into the history, the
-// non-finite and convergence tests, the step counter and the buffer swap;
-// the step's accumulators are cleared for the next step.
-template <class T> __device__ __forceinline__ void resid_book(const CaseDev<T>& C, double mm, double sq) {
-  Ctrl* c = C.ctrl;
-  const int st = c->step;
-  const double l2 = sqrt(sq);
-  C.hist_linf[st] = mm;
-  C.hist_l2[st] = l2;
-  C.hist_dt[st] = step_dt(c);
-  if (!isfinite(l2) || !isfinite(mm)) {
-    c->nonfinite = 1;
-    c->done = 1;
-  }
-  if (c->timeout) c->done = 1;
-  if (c->ref == 0.0 && l2 > 0.0) c->ref = l2;
-  c->acc_sq = 0.0;
-  c->acc_max = 0.0;
-  c->maxmu = 0.0;
-  c->cur ^= 1;
-  c->step = st + 1;
-  if (c->step >= c->max_steps) c->done = 1;
-  if (c->tol > 0.0 && l2 <= c->tol * c->ref) c->done = 1;
-}
+// The bookkeeping as a launch of its own, one CTA per case: for sets with
+// ALPHA < 1 cases, whose residual is complete after k_wspec.
 template <class T> __global__ void k_resid(BatchArgs<T> a) {
   if (threadIdx.x != 0) return;
-  if (blockIdx.x == 0) a.ctl->sweep_next = 0;
   const CaseDev<T>& C = a.cases[blockIdx.x];
   if (C.ctrl->done) return;
   resid_book(C, C.ctrl->acc_max, C.ctrl->acc_sq);
@@ -1691,9 +1734,8 @@ template <class T> __global__ void k_shard_respart(const __grid_constant__ CaseD
   res[1] = C.ctrl->acc_sq;
 }
 template <class T>
-__global__ void k_shard_resid(const __grid_constant__ CaseDev<T> C, const double* __restrict__ res, BatchCtl* ctl) {
+__global__ void k_shard_resid(const __grid_constant__ CaseDev<T> C, const double* __restrict__ res) {
   if (threadIdx.x != 0) return;
-  ctl->sweep_next = 0;
   if (C.ctrl->done) return;
   resid_book(C, res[0], res[1]);
 }

@@ -116,11 +116,11 @@ struct Ctrl {
   int nonfinite;  // set when a residual was NaN/Inf
   double tol;     // relative L2 tolerance (<= 0: none)
   double ref;     // reference L2 residual (0: take the first step's)
-  double maxmu;   // max MU of the current step (atomicMax on the bits; reset by k_resid)
+  double maxmu;   // max MU of the current step (atomicMax on the bits; reset by resid_book)
   double dtc;     // Courant limit DTEc (src/alotim.f90)
-  double acc_sq;  // sum of squared changes of the current step (sweep atomics; reset by k_resid)
-  double acc_max; // max residual of the current step (atomicMax on the bits; reset by k_resid)
-  int cur;        // which f buffer holds the current state (k_resid swaps it)
+  double acc_sq;  // sum of squared changes of the current step (sweep atomics; reset by resid_book)
+  double acc_max; // max residual of the current step (atomicMax on the bits; reset by resid_book)
+  int cur;        // which f buffer holds the current state (resid_book swaps it)
   int timeout;    // set when a bounded device wait gave up
   int itime0;     // steps the handle ran before this advance call (the reference's ITIME - step - 1)
   int pad0;
@@ -128,8 +128,9 @@ struct Ctrl {
 
 // Device-side control of one launch set (a case alone or a batch).
 struct BatchCtl {
-  int sweep_next;  // sweep work units handed out beyond the first wave (reset by k_resid)
-  int pad[15];
+  int sweep_next;  // sweep work units handed out beyond the first wave
+  int sweep_done;  // sweep CTAs that have finished (both reset by the last one)
+  int pad[14];
   double etab[EXP_TAB];  // 2^(j/64) of the FP64 sweep's exp
 };
 
