@@ -153,7 +153,7 @@ template <class T, bool ONE> MomFn<T> mom_fn1(int R) {
 }
 template <class T> MomFn<T> mom_fn(int R, bool one) { return one ? mom_fn1<T, true>(R) : mom_fn1<T, false>(R); }
 // dynamic shared memory of a sweep CTA: 227 KB less its static arrays
-constexpr size_t SWEEP_SMEM_MAX = 227 * 1024 - 1024;
+constexpr size_t SWEEP_SMEM_MAX = 227 * 1024 - 3072;
 template <class T> using SweepFn = void (*)(BatchArgs<T>, int, const CaseDev<T>);
 template <class T, bool ONE> SweepFn<T> sweep_fn1(int eb, int immat) {
   if (eb == 64) return immat == 1 ? k_sweep<T, 64, 1, ONE> : k_sweep<T, 64, 0, ONE>;

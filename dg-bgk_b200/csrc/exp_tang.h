@@ -2,16 +2,19 @@
 // implementation of the exponential function in IEEE floating-point
 // arithmetic", ACM Trans. Math. Softw. 15(2), 1989), for the sweep's
 // Maxwellian values (x <= 0), from the mathematics:
-//   x = (64 m + j) ln2/64 + r,  j = 0..63,  |r| <= ln2/128,
-//   exp(x) = 2^m * 2^(j/64) * exp(r),
-// with k = 64 m + j the integer nearest x*64/ln2 (rounded by adding and
-// subtracting 1.5*2^52), r = x - k*ln2/64 by two fused multiply-adds with
-// ln2/64 split into a 32-bit head and its remainder, and exp(r) - 1 by the
-// Taylor polynomial of degree 5 (truncation error |r|^6/720 < 4e-17
-// relative).  The table tab[j] = 2^(j/64) is the caller's (filled once per
-// CTA); 2^m is applied by an integer add to the exponent field.  Below
-// x = -707 (results under 1e-307) the value is flushed to +0; NaN stays NaN.
-// Measured against long-double exp on the host (tests/test_exp_tang.py).
+//   x = (256 m + j) ln2/256 + r,  j = 0..255,  |r| <= ln2/512,
+//   exp(x) = 2^m * 2^(j/256) * exp(r),
+// with k = 256 m + j the integer nearest x*256/ln2 (rounded by adding and
+// subtracting 1.5*2^52), r = x - k*ln2/256 by two fused multiply-adds with
+// ln2/256 split into a 32-bit head and its remainder, and exp(r) - 1 by the
+// Taylor polynomial of degree 4 (truncation error |r|^5/120 < 4e-17
+// relative).  The table tab[j] = 2^(j/256) is the caller's (in shared memory,
+// 2 KB; with 64 entries the polynomial took a degree more); 2^m is applied by
+// an integer add to the exponent field.  From x = -707 down (results under
+// 1e-307) the value is flushed to +0, by an integer comparison of the high
+// word, which keeps the FP64 pipe free and lets a NaN, whatever its sign,
+// through.  Measured against long-double exp on the host
+// (tests/test_exp_tang.py).
 #pragma once
 #include <cstdint>
 #include <cstring>
@@ -24,7 +27,7 @@
 
 namespace dgbgk {
 
-constexpr int EXP_TAB = 64;
+constexpr int EXP_BITS = 8, EXP_TAB = 1 << EXP_BITS;
 
 DGBGK_HD double dbl_from_bits(int64_t b) {
 #if defined(__CUDA_ARCH__)
@@ -46,26 +49,27 @@ DGBGK_HD int64_t dbl_bits(double d) {
 }
 
 DGBGK_HD double exp_tang(double x, const double* __restrict__ tab) {
-  const double inv_step = 92.33248261689366;        // 64 / ln2
-  const double step_hi = 0.01083042469326756;       // ln2/64, leading 32 bits
-  const double step_lo = 2.9815858269852933e-12;    // ln2/64 - step_hi
+  const double inv_step = 369.3299304675746;        // 256 / ln2
+  const double step_hi = 0.00270760617331689;      // ln2/256, leading 32 bits
+  const double step_lo = 7.453964567463233e-13;     // ln2/256 - step_hi
   const double shift = 6755399441055744.0;          // 1.5 * 2^52
   const double ks = fma(x, inv_step, shift);        // k in the low word
   const double kd = ks - shift;
   const int k = (int)(uint32_t)dbl_bits(ks);
   double r = fma(-kd, step_hi, x);
   r = fma(-kd, step_lo, r);
-  double p = fma(r, 1.0 / 120.0, 1.0 / 24.0);
-  p = fma(r, p, 1.0 / 6.0);
+  double p = fma(r, 1.0 / 24.0, 1.0 / 6.0);
   p = fma(r, p, 0.5);
   p = fma(r, p, 1.0);
   p = r * p;  // exp(r) - 1
   const double t = tab[k & (EXP_TAB - 1)];
   const double y = fma(t, p, t);
-  const int64_t m = (int64_t)(k >> 6);  // floor(k / 64)
+  const int64_t m = (int64_t)(k >> EXP_BITS);  // floor(k / 256)
   // 2^m: m added to the exponent field (two's complement, shifted unsigned)
   const double v = dbl_from_bits((int64_t)((uint64_t)dbl_bits(y) + ((uint64_t)m << 52)));
-  return x > -707.0 ? v : (x != x ? x : 0.0);
+  // high words from -707 to -infinity, NaNs not among them
+  const uint32_t h = (uint32_t)((uint64_t)dbl_bits(x) >> 32);
+  return h - 0xC0861800u <= 0xFFF00000u - 0xC0861800u ? 0.0 : v;
 }
 
 }  // namespace dgbgk

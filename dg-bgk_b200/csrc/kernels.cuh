@@ -880,7 +880,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 }
 
 // exp of the NFO exponent: FP64 by Tang's table-driven method (exp_tang.h,
-// about one ulp, `tab` the CTA's 2^(j/64) table); FP32 2^x from the SFU
+// about one ulp, `tab` the CTA's 2^(j/256) table); FP32 2^x from the SFU
 // (ex2.approx, relative error ~2^-22; the FP32 coefficient carries the
 // log2(e) factor, applied in FP64 by the moment kernel; no table).
 template <class T> __device__ __forceinline__ T nfo_exp(T x, const double* tab);
@@ -1091,11 +1091,12 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
   // it, and the warps would then disagree on the unit and on the barriers)
   __shared__ int s_unit[2], s_last;
   __shared__ double red_m[NW], red_s[NW];
-  // FP64: the 2^(j/64) table of the NFO exp (one entry for FP32, unused)
+  // FP64: the 2^(j/256) table of the NFO exp (one entry for FP32, unused)
   __shared__ double etab[sizeof(T) == 8 ? EXP_TAB : 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int sub = lane / G::LPE, l8 = tid & (G::LPE - 1);
-  if (sizeof(T) == 8 && tid < EXP_TAB) etab[tid] = a.ctl->etab[tid];
+  if (sizeof(T) == 8)
+    for (int i = tid; i < EXP_TAB; i += NT) etab[i] = a.ctl->etab[i];
   const unsigned tile_bytes = G::tile_bytes(EB, a.max_halo);
   const bool two = a.sweep_bufs > 1;
   unsigned char* const recs = sm_raw + (two ? 2 : 1) * tile_bytes;  // pitch RP

@@ -131,7 +131,7 @@ struct BatchCtl {
   int sweep_next;  // sweep work units handed out beyond the first wave
   int sweep_done;  // sweep CTAs that have finished (both reset by the last one)
   int pad[14];
-  double etab[EXP_TAB];  // 2^(j/64) of the FP64 sweep's exp
+  double etab[EXP_TAB];  // 2^(j/256) of the FP64 sweep's exp
 };
 
 }  // namespace dgbgk
