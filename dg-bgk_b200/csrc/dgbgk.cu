@@ -562,7 +562,10 @@ template <class T> struct Impl : ImplBase {
   WallSide* walls = nullptr;
   int *node_off = nullptr, *node_dg = nullptr;
   double* node_ae = nullptr;
-  double *hist_linf = nullptr, *hist_l2 = nullptr, *hist_dt = nullptr;
+  double *hist_linf = nullptr, *hist_l2 = nullptr, *hist_dt = nullptr;  // one allocation, pitch hist_cap
+  double* init_buf = nullptr;  // inputs of the init kernels, kept between calls
+  size_t init_cap = 0;
+  double* nodal = nullptr;     // [6*NP] nodal fields of macros()
   int hist_cap = 0;
   Ctrl* ctrl = nullptr;
   Ctrl* hctrl = nullptr;  // pinned: [0] upload, [1..2] polls
@@ -617,8 +620,8 @@ template <class T> struct Impl : ImplBase {
     dfree(node_dg);
     dfree(node_ae);
     dfree(hist_linf);
-    dfree(hist_l2);
-    dfree(hist_dt);
+    dfree(init_buf);
+    dfree(nodal);
     dfree(ctrl);
     dfree(rside);
     dfree(rf_i);
@@ -879,11 +882,9 @@ template <class T> struct Impl : ImplBase {
   int ensure_hist(int n) {
     if (n <= hist_cap) return 0;
     dfree(hist_linf);
-    dfree(hist_l2);
-    dfree(hist_dt);
-    TRY(dalloc(&hist_linf, n));
-    TRY(dalloc(&hist_l2, n));
-    TRY(dalloc(&hist_dt, n));
+    TRY(dalloc(&hist_linf, 3 * (size_t)n));
+    hist_l2 = hist_linf + n;
+    hist_dt = hist_l2 + n;
     hist_cap = n;
     if (halo) TRY(refresh());
     return 0;
@@ -924,10 +925,13 @@ template <class T> struct Impl : ImplBase {
     ref_host = c.ref;
     cur = c.cur;
     itime_total += ns;
-    if (ns > 0) {
-      if (linf) CK(cudaMemcpy(linf, hist_linf, ns * sizeof(double), cudaMemcpyDeviceToHost));
-      if (l2) CK(cudaMemcpy(l2, hist_l2, ns * sizeof(double), cudaMemcpyDeviceToHost));
-      if (dt) CK(cudaMemcpy(dt, hist_dt, ns * sizeof(double), cudaMemcpyDeviceToHost));
+    if (ns > 0 && (linf || l2 || dt)) {  // the three histories in one copy
+      const size_t w = (size_t)ns * sizeof(double);
+      std::vector<double> h(3 * (size_t)ns);
+      CK(cudaMemcpy2D(h.data(), w, hist_linf, (size_t)hist_cap * sizeof(double), w, 3, cudaMemcpyDeviceToHost));
+      double* dsts[3] = {linf, l2, dt};
+      for (int k = 0; k < 3; ++k)
+        if (dsts[k]) std::memcpy(dsts[k], h.data() + (size_t)k * ns, w);
     }
     return finish_status(c);
   }
@@ -1073,9 +1077,9 @@ template <class T> struct Impl : ImplBase {
     TRY(moments_now());
     TRY(record(out_args((int)itime_total, out_direct)));
     double hdr[4];
+    CK(cudaMemcpyAsync(&hctrl[1], ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(hdr, out_direct, sizeof hdr, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    CK(cudaMemcpy(&hctrl[1], ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost));
     TRY(finish_status(hctrl[1]));
     if (lift) *lift = hdr[1];
     if (drag) *drag = hdr[2];
@@ -1288,6 +1292,17 @@ template <class T> struct Impl : ImplBase {
     return 0;
   }
 
+  // room for n values of the init kernels' inputs (allocating and freeing them
+  // on each call waits for the device twice)
+  int ensure_init(size_t n) {
+    if (n <= init_cap) return 0;
+    dfree(init_buf);
+    init_cap = 0;
+    TRY(dalloc(&init_buf, n));
+    init_cap = n;
+    return 0;
+  }
+
   int init_uniform(double t1, double p1, double u0, double v0, const double* scale) override {
     CK(cudaSetDevice(device));
     // INICON2 (src/inicon2.f90:120-174) evaluated per velocity in double
@@ -1314,16 +1329,14 @@ template <class T> struct Impl : ImplBase {
       for (int en = 0; en < pl.E; ++en)
         for (int i = 0; i < 3; ++i) sc[3 * (size_t)en + i] = scale[3 * (size_t)pl.perm[en] + i];
     }
-    double *dg = nullptr, *dsc = nullptr;
-    TRY(upload(&dg, g, st));
-    if (scale) TRY(upload(&dsc, sc, st));
+    TRY(ensure_init(g.size() + sc.size()));
+    double* dsc = scale ? init_buf + g.size() : nullptr;
+    CK(cudaMemcpyAsync(init_buf, g.data(), g.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+    if (scale) CK(cudaMemcpyAsync(dsc, sc.data(), sc.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     const size_t ndg = (size_t)3 * pl.E;
-    k_init_uniform<T><<<(unsigned)ndg, 128, 0, st>>>(f[0], dg, dsc, vacuum ? 0.0 : n1, pl.V, Vp, ndg);
-    cudaError_t e = cudaGetLastError();
-    cudaStreamSynchronize(st);
-    cudaFree(dg);
-    if (dsc) cudaFree(dsc);
-    CK(e);
+    k_init_uniform<T><<<(unsigned)ndg, 128, 0, st>>>(f[0], init_buf, dsc, vacuum ? 0.0 : n1, pl.V, Vp, ndg);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(st));
     cur = 0;
     ++epoch;
     itime_total = 0;  // a new state: ITIME starts again
@@ -1341,15 +1354,13 @@ template <class T> struct Impl : ImplBase {
         prm[4 * d + 2] = v[o];
         prm[4 * d + 3] = t[o];
       }
-    double* dp = nullptr;
-    TRY(upload(&dp, prm, st));
+    TRY(ensure_init(prm.size()));
+    CK(cudaMemcpyAsync(init_buf, prm.data(), prm.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     const size_t ndg = (size_t)3 * pl.E;
-    k_init_maxwellian<T><<<(unsigned)ndg, 128, 0, st>>>(f[0], dp, cxD, cyD, pl.M / 6.022e26, pl.rgas, pl.V, Vp,
+    k_init_maxwellian<T><<<(unsigned)ndg, 128, 0, st>>>(f[0], init_buf, cxD, cyD, pl.M / 6.022e26, pl.rgas, pl.V, Vp,
                                                          ndg);
-    cudaError_t e = cudaGetLastError();
-    cudaStreamSynchronize(st);
-    cudaFree(dp);
-    CK(e);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(st));
     cur = 0;
     ++epoch;
     itime_total = 0;  // a new state: ITIME starts again
@@ -1370,19 +1381,16 @@ template <class T> struct Impl : ImplBase {
   int macros(double* nd, double* rho, double* u, double* v, double* ps, double* temp) override {
     CK(cudaSetDevice(device));
     TRY(moments_now());
-    double* out = nullptr;
-    TRY(dalloc(&out, 6 * (size_t)pl.NP));
+    if (!nodal) TRY(dalloc(&nodal, 6 * (size_t)pl.NP));
+    double* out = nodal;
     NodalArgs a{node_off, node_dg, node_ae, nraw, disux, disuy, disps, out, out + pl.NP, out + 2 * pl.NP,
                 out + 3 * pl.NP, out + 4 * pl.NP, out + 5 * pl.NP, pl.NP, pl.M / 6.022e26, pl.rgas};
     k_nodal<<<(pl.NP + 255) / 256, 256, 0, st>>>(a);
-    cudaError_t e = cudaGetLastError();
+    CK(cudaGetLastError());
     std::vector<double> h(6 * (size_t)pl.NP);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(h.data(), out, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
-    cudaFree(out);
-    CK(e);
-    CK(cudaMemcpy(&hctrl[1], ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(&hctrl[1], ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(h.data(), out, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
     TRY(finish_status(hctrl[1]));
     double* dsts[6] = {nd, rho, u, v, ps, temp};
     for (int k = 0; k < 6; ++k)
