@@ -494,6 +494,22 @@ struct StepGraphs {
   }
 };
 
+// The Gram matrix of the m differences of m + 1 snapshots of N values.
+template <class T, int M = RRE_MAX - 1>
+int gram(const T* snaps, size_t N, int m, double* G, int nsm, cudaStream_t st) {
+  if constexpr (M > 1) {
+    if (m < M) return gram<T, M - 1>(snaps, N, m, G, nsm, st);
+  }
+  // one resident wave: every block ends with its own sums
+  int per_sm = 0;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_gram<T, M>, 256, 0));
+  const size_t nv = N * sizeof(T) / 16;
+  const int grid = (int)std::min<size_t>((size_t)std::max(per_sm, 1) * nsm, (nv + 255) / 256);
+  k_gram<T, M><<<grid, 256, 0, st>>>(snaps, N, N, G);
+  CK(cudaGetLastError());
+  return 0;
+}
+
 // Reduced-rank extrapolation coefficients from the m x m Gram matrix G of
 // the snapshot differences (upper triangle accumulated by k_gram): solve
 // G gamma = 1 and scale to sum(gamma) = 1.  G is overwritten.
@@ -1260,9 +1276,8 @@ template <class T> struct Impl : ImplBase {
     if (!d_gram) TRY(dalloc(&d_gram, (size_t)RRE_MAX * RRE_MAX));
     if (!d_gamma) TRY(dalloc(&d_gamma, (size_t)RRE_MAX));
     CK(cudaMemsetAsync(d_gram, 0, (size_t)m * m * sizeof(double), st));
+    TRY(gram<T>(snaps, N, m, d_gram, nsm, st));
     const int grid = (int)std::min<size_t>((size_t)4 * nsm, (N + 255) / 256);
-    k_gram<T><<<grid, 256, 0, st>>>(snaps, N, n, N, d_gram);
-    CK(cudaGetLastError());
     std::vector<double> G((size_t)m * m), g;
     CK(cudaMemcpyAsync(G.data(), d_gram, G.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -2096,9 +2111,7 @@ template <class T> struct BatchImpl : BatchBase {
       if (!c->d_gamma) TRY(dalloc(&c->d_gamma, (size_t)RRE_MAX));
       const size_t N = (size_t)3 * c->pl.E * c->Vp;
       CK(cudaMemsetAsync(c->d_gram, 0, (size_t)m * m * sizeof(double), st));
-      const int grid = (int)std::min<size_t>((size_t)4 * nsm, (N + 255) / 256);
-      k_gram<T><<<grid, 256, 0, st>>>(c->snaps, N, n, N, c->d_gram);
-      CK(cudaGetLastError());
+      TRY(gram<T>(c->snaps, N, m, c->d_gram, nsm, st));
       CK(cudaMemcpyAsync(h_gram + i * GS, c->d_gram, (size_t)m * m * sizeof(double), cudaMemcpyDeviceToHost, st));
     }
     CK(cudaStreamSynchronize(st));
