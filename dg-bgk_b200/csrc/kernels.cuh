@@ -567,7 +567,8 @@ __global__ void __launch_bounds__(ONE ? 640 : 512, 1)
   constexpr bool ELEM = R == 3;
   constexpr int L = ELEM ? 32 : 32 / R;
   extern __shared__ __align__(128) unsigned char sm_raw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // uniform: the ring's addresses too
   const int grp = ELEM ? 0 : lane / L, sub = lane % L;
   const int nstage = a.mom_stages;
   // layout: [barriers][tables [mom_tables][Vp] (ONE)][rings: warp, stage, R rows]
