@@ -376,7 +376,8 @@ def run_ours(a, d):
                         "kernel_ms": dict(zip(names, [float(x) for x in kms])),
                         "step_frac": step_gbs / peak},
            "clocks": ck,
-           "gpu_launches": a.steps * (4 if (case.mesh.bsido[:, 3] == 4).any() else 3)}
+           # moments, sweep (with the residual bookkeeping), wall flux
+           "gpu_launches": a.steps * (3 if (case.mesh.bsido[:, 3] == 4).any() else 2)}
     del s
     # plain FP64 path on the same workload
     if not a.no_fp64 and a.precision == 32:

@@ -1,5 +1,5 @@
 // C ABI of the DG-BGK sweep on B200 (sm_100a): handle management, device
-// memory, the captured two-step CUDA graph and the state transfers.
+// memory, the captured CUDA graphs of the steps and the state transfers.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -388,8 +388,9 @@ int launch_dependent(const char* what, void (*fn)(P...), int grid, int block, si
   return launch_check(what, grid, block, smem);
 }
 
-// One pseudo-time step of every case of the set: moments, wall flux, sweep,
-// residual bookkeeping.
+// One pseudo-time step of every case of the set: moments, wall flux, sweep
+// (its last CTA does the residual bookkeeping; a launch of its own only
+// where k_wspec follows the sweep).
 template <class T>
 int enqueue_step(const LaunchSet<T>& L, cudaStream_t st, float* ms = nullptr, const OutArgs* out = nullptr) {
   cudaEvent_t ev[5];

@@ -824,35 +824,12 @@ template <class T> struct SweepGeo {
   static constexpr int LPE = 8;                  // lanes per element
   static constexpr int VT = W * LPE;             // velocities per tile
   static constexpr int EPW = 32 / LPE;           // elements of a warp at a time
-#ifndef DGBGK_IT32_64
-#define DGBGK_IT32_64 2
-#endif
-#ifndef DGBGK_IT32_128
-#define DGBGK_IT32_128 2
-#endif
-#ifndef DGBGK_IT64_64
-#define DGBGK_IT64_64 2
-#endif
-#ifndef DGBGK_IT64_128
-#define DGBGK_IT64_128 2
-#endif
-#ifndef DGBGK_SWEEP_REGS32
-#define DGBGK_SWEEP_REGS32 128
-#endif
-#ifndef DGBGK_SWEEP_REGS64
-#define DGBGK_SWEEP_REGS64 128
-#endif
   // block elements per lane group: their NFO and UMEAN stay in registers
   // between the phases (16 registers an element)
-  static constexpr int iters(int EB) {
-    return sizeof(T) == 4 ? (EB == 64 ? DGBGK_IT32_64 : DGBGK_IT32_128) : (EB == 64 ? DGBGK_IT64_64 : DGBGK_IT64_128);
-  }
-  static constexpr int threads(int EB) { return EB / (EPW * iters(EB)) * 32; }
-  // resident CTAs per SM the register budget is set for
-  static constexpr int min_ctas(int EB) {
-    const int c = 65536 / ((sizeof(T) == 4 ? DGBGK_SWEEP_REGS32 : DGBGK_SWEEP_REGS64) * threads(EB));
-    return c < 1 ? 1 : c;
-  }
+  static constexpr int ITERS = 2;
+  static constexpr int threads(int EB) { return EB / (EPW * ITERS) * 32; }
+  // resident CTAs per SM at 128 registers a thread (16 warps)
+  static constexpr int min_ctas(int EB) { return 65536 / (128 * threads(EB)); }
   static constexpr int RW = (int)(sizeof(ElemRec<T>) / 16);                // record words
   static constexpr int HW = (REC_HEAD_VALUES * (int)sizeof(typename CoefOf<T>::type) + 15) / 16;  // head words
   // pitches in shared memory: odd numbers of 16-byte words, so that the four
@@ -1069,14 +1046,16 @@ __device__ __forceinline__ void resid_add(Ctrl* ctrl, const double* red_m, const
 // (the records hold them as pairs) and the swizzle's index arithmetic, the
 // staging of the new rows through the tile, and the neighbour gather's bank
 // conflicts (2.0e7 -> 0.3e7 per launch).  200x100 channel, 24x48 velocities
-// (1.375e8 DOFs): FP32 0.394 -> 0.304 ms, FP64 0.945 -> 0.770.  Bound (FP32,
+// (1.375e8 DOFs): FP32 0.394 -> 0.293 ms, FP64 0.945 -> 0.742.  Bound (FP32,
 // ncu): latency at 16 warps per SM (128 registers), issue active 0.52, stalls
 // per issue wait 1.2, short-scoreboard and barrier 0.9 each, math-pipe 0.9;
 // FMA pipe 0.41 and shared-memory wavefronts 0.62 of their peaks.  Measured
 // and not kept: one element per lane group and 16 warps per 64 elements
 // (FP32 0.372, FP64 0.817), four per group in FP64 (1.04), FP64 at 168
 // registers (0.840), coefficients duplicated in registers (0.387), f loaded
-// straight into registers at the start of phase 1 (0.387).
+// straight into registers at the start of phase 1 (0.387), one tile buffer
+// and three CTAs at 80 registers (FP32 0.358), the wall records staged in
+// shared memory (FP32 0.295, FP64 0.788: it spills).
 template <class T, int EB, int IMMAT, bool ONE>
 __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_ctas(EB))
     k_sweep(BatchArgs<T> a, int total_units, const __grid_constant__ CaseDev<T> one) {
@@ -1084,7 +1063,7 @@ __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_cta
   using P = typename Pair<T>::type;
   using VecT = typename Pair<T>::vec;
   constexpr int W = G::W, NP = G::NP, VT = G::VT, RW = G::RW, RP = G::RP, HW = G::HW, HR = G::HR;
-  constexpr int ITERS = G::iters(EB), EPW = G::EPW;
+  constexpr int ITERS = G::ITERS, EPW = G::EPW;
   constexpr int NT = G::threads(EB), NW = NT / 32;
   static_assert(NW * EPW * ITERS == EB, "whole warps");
   extern __shared__ __align__(128) unsigned char sm_raw[];

@@ -3,7 +3,7 @@
 // HBM layout of the distribution function: f[(e*3 + i)*Vp + v] -- element e
 // (in the plan's locality order), DG node i (0..2), discrete velocity v
 // fastest, rows padded to a pitch Vp (a multiple of 32 velocities, so every
-// row starts on a 128-byte boundary and splits into whole 64-byte sweep
+// row starts on a 128-byte boundary and splits into whole 128-byte sweep
 // segments).  The padding velocities hold zeros forever (the buffers are
 // cleared at allocation and the kernels write zeros there), so kernels may
 // read whole 16-byte vectors past V without bounds checks.  Two such buffers are

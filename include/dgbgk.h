@@ -223,7 +223,9 @@ int dgbgk_last_timing(dgbgk_handle* h, double* total_ms);
 /* Runs nsteps time steps launch by launch (no graph) with CUDA events
  * between the kernels on the library's stream; kernel_ms[4] receives the
  * mean device time per step of [moments, wall flux, sweep, residual]. The
- * state advances by nsteps steps exactly as under dgbgk_advance(). */
+ * state advances by nsteps steps exactly as under dgbgk_advance().  The
+ * residual bookkeeping is part of the sweep, and the last entry the gap
+ * between two events, except where ALPHA < 1 puts it in a launch of its own. */
 int dgbgk_profile_steps(dgbgk_handle* h, int nsteps, double* kernel_ms);
 
 /* No counterpart in the reference.  dgbgk_get_macros() without any device
