@@ -666,10 +666,17 @@ template <class T> struct Impl : ImplBase {
   }
 
   int nvt() const { return (pl.V + SweepGeo<T>::VT - 1) / SweepGeo<T>::VT; }
-  // measured on B200: FP32 sweep of the 200x100 channel at 24x48 velocities
+  // Measured on B200: FP32 sweep of the 200x100 channel at 24x48 velocities
   // 0.304 ms with 64 elements (two CTAs of 8 warps per SM), 0.312 with 128
-  // (one of 16); FP64 0.805 with 64, 0.770 with 128
-  static int default_eb() { return sizeof(T) == 8 ? 128 : 64; }
+  // (one of 16).  FP64: 128, except where that leaves SMs without a tile:
+  // 8x8 cavity at 16x16 velocities (16 tiles) 16.1 us with 128, 14.5 with 64;
+  // 32x32 at 16x32 (512 tiles) 33.4 against 35.8; the channel 0.743 against
+  // 0.741.
+  static int default_eb(long nelem, long nvel, int nsm) {
+    if (sizeof(T) == 4) return 64;
+    const long tiles = (nelem + 127) / 128 * ((nvel + SweepGeo<T>::VT - 1) / SweepGeo<T>::VT);
+    return tiles <= nsm ? 64 : 128;
+  }
 
   int init(int tile_elems) {
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
@@ -829,7 +836,7 @@ template <class T> struct Impl : ImplBase {
 
   // Sweep tile: EB elements per CTA x one 128-byte velocity segment.
   int set_tile(int tile_elems) {
-    int eb = tile_elems > 0 ? tile_elems : default_eb();
+    int eb = tile_elems > 0 ? tile_elems : default_eb(pl.E, pl.V, nsm);
     if (eb != 64 && eb != 128) {
       set_error("tile_elems must be 64 or 128");
       return DGBGK_EINVAL;
@@ -1547,8 +1554,8 @@ int dgbgk_create(const dgbgk_mesh* mesh, const dgbgk_vspace* vs, const dgbgk_par
   }
   std::string err;
   const int eb0 = prm->tile_elems > 0      ? prm->tile_elems
-                  : prm->precision == 64 ? Impl<double>::default_eb()
-                                         : Impl<float>::default_eb();
+                  : prm->precision == 64 ? Impl<double>::default_eb(mesh->nelem, (long)vs->rorder * vs->torder, prop.multiProcessorCount)
+                                         : Impl<float>::default_eb(mesh->nelem, (long)vs->rorder * vs->torder, prop.multiProcessorCount);
   int rc = build_plan(*mesh, *vs, *prm, eb0, impl->pl, &err);
   if (rc != 0) {
     set_error(err);

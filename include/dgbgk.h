@@ -83,7 +83,8 @@ typedef struct dgbgk_params {
                          in FP32 with FP64 moments and residual norms      */
   const double* wall_velocity; /* (2,NBOUN) moving-wall velocity per
                                   boundary side, or NULL (all at rest)    */
-  int tile_elems;     /* sweep tile: elements per CTA, 64 or 128 (0: 64 for FP32, 128 for FP64;
+  int tile_elems;     /* sweep tile: elements per CTA, 64 or 128 (0: 64 for FP32; FP64 128, or
+                         64 where 128 would leave SMs without a tile;
                          a halo too wide for a 128-element tile takes 64) */
   int moment_rows;    /* moment kernel: velocity rows per warp step -- 1, 2 or 4
                          rows of any elements (32/R lanes per row), or 3: the

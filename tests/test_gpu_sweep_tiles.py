@@ -72,3 +72,16 @@ def test_wide_halos(k, prec, tile):
     # the halo does grow; past what a 128-element tile can hold, 64 are taken
     assert s.info()["max_halo"] >= min(2 * k, 100)
     assert s.info()["tile_elems"] in (64, 128)
+
+
+@pytest.mark.parametrize("nt", [8, 9, 10, 13])
+def test_default_fp64_tile_follows_the_tile_count(nt):
+    # 2048 elements: 16 blocks of 128 at V = 16 * nt, so 128, 144, 160 and 208
+    # tiles; a chip with more SMs than tiles takes 64 elements
+    import torch
+
+    s, o, _ = pair(cavity_case(32, 16, nt, mach=0.3, kn=0.1))
+    nsm = torch.cuda.get_device_properties(0).multi_processor_count
+    assert s.info()["tile_elems"] == (64 if 16 * nt <= nsm else 128)
+    s.advance(2), o.advance(2)
+    assert rel_l2(s.get_state(), o.get_state()) <= TOL64
