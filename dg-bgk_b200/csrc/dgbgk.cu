@@ -368,23 +368,11 @@ inline int launch_check(const char* what, int grid, int block, size_t smem) {
   return DGBGK_ECUDA;
 }
 
-// Launch with programmatic dependence on the kernel before it in the stream
-// (the kernel waits by itself, grid_wait): its launch and everything it does
-// before that wait pass while the other one ends.
+// launch_pdl, and the launch's error
 template <class... P, class... A>
 int launch_dependent(const char* what, void (*fn)(P...), int grid, int block, size_t smem, cudaStream_t st,
                      const A&... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, fn, args...);
+  launch_pdl(fn, dim3((unsigned)grid), dim3((unsigned)block), smem, st, args...);
   return launch_check(what, grid, block, smem);
 }
 

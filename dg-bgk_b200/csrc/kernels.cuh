@@ -30,6 +30,7 @@
 #include <type_traits>
 
 #include "exp_tang.h"
+#include "pdl.cuh"
 #include "types.h"
 
 namespace dgbgk {
@@ -38,16 +39,6 @@ constexpr double PI_D = 3.1416;  // the reference's PI
 constexpr double TINY_D = 1e-20;
 constexpr double LOG2E_D = 1.4426950408889634;  // log2(e)
 constexpr unsigned WAIT_TRIES = 1u << 22;  // x ~256 ns sleep: ~1 s
-
-// Programmatic dependent launch: the next kernel of the stream may start (its
-// CTAs as this one's leave their SMs) once every CTA has called this or left;
-// what it then does before grid_wait must not touch anything an earlier kernel
-// writes.
-__device__ __forceinline__ void grid_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-// ... and waits here until the kernels before it are complete
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll

@@ -121,7 +121,7 @@ template <int BN, int STAGES, int SUB, int EPI> int launch_gemm(const Gemm& G, c
   auto fn = k_gemm<BN, STAGES, SUB, EPI>;
   constexpr int bytes = Smem<BN, STAGES, SUB, EPI>::TOTAL;
   MCK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  fn<<<dim3(g.N / BN, g.M / BM), 128, bytes, st>>>(G.ta, G.tb, g);
+  launch_pdl(fn, dim3(g.N / BN, g.M / BM), dim3(128), bytes, st, G.ta, G.tb, g);
   MCK(cudaGetLastError());
   return 0;
 }
@@ -148,6 +148,8 @@ int run_gemm(const Gemm& G, cudaStream_t st) { return run_gemm(G, G.g, st); }
 __global__ void k_gather(const float* __restrict__ xs, const int* __restrict__ idx, int n_in, int B,
                          __nv_bfloat16* x0, __nv_bfloat16* x0T) {
   const int r = blockIdx.x * blockDim.y + threadIdx.y, c = threadIdx.x;
+  grid_launch_dependents();
+  grid_wait();
   const __nv_bfloat16 v = __float2bfloat16_rn(c < n_in ? xs[(size_t)idx[r] * n_in + c] : 0.f);
   x0[(size_t)r * KPAD + c] = v;
   x0T[(size_t)c * B + r] = v;
@@ -177,6 +179,8 @@ struct BiasArgs {
 __global__ void k_bias_adam(const __grid_constant__ BiasArgs a, const __grid_constant__ GemmArgs p) {
   int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
+  grid_launch_dependents();
+  grid_wait();
   if (j >= a.end[a.n - 1]) return;
   int l = 0;
   while (j >= a.end[l]) ++l;
@@ -383,8 +387,9 @@ struct dgbgk_mlp {
 
   // forward, and the loss (into *lslot) and its gradient at the output, of
   // the minibatch whose inputs are in H[0] and whose targets are rows id of t
+  // (*lslot is zero before: a memset between two kernels would keep the second
+  // from starting early)
   int forward_loss(const float* t, const int* id, double* lslot) {
-    MCK(cudaMemsetAsync(lslot, 0, sizeof(double), st));
     for (int l = 0; l < depth; ++l) MTRY(run_gemm(fwd[l], st));
     GemmArgs g = out_loss.g;
     g.ts = t;
@@ -434,7 +439,7 @@ struct dgbgk_mlp {
         g.c2 = p.c2;
         a.end[a.n] = tiles += (g.M / BM) * (g.N / 64);
       }
-      k_gemm_adam<64, STAGES_ADAM, 1><<<tiles, 128, bytes, st>>>(a);
+      launch_pdl(k_gemm_adam<64, STAGES_ADAM, 1>, dim3(tiles), dim3(128), bytes, st, a);
       MCK(cudaGetLastError());
     }
     for (int l0 = 0; l0 <= depth; l0 += BIAS_LAYERS) {
@@ -448,14 +453,14 @@ struct dgbgk_mlp {
         a.v[a.n] = L[l].vb;
         a.end[a.n] = rows += L[l].out;
       }
-      k_bias_adam<<<(rows + 7) / 8, 256, 0, st>>>(a, p);
+      launch_pdl(k_bias_adam, dim3((rows + 7) / 8), dim3(256), 0, st, a, p);
       MCK(cudaGetLastError());
     }
     return 0;
   }
 
   int gather(const float* x, const int* id) {
-    k_gather<<<B / 4, dim3(KPAD, 4), 0, st>>>(x, id, n_in, B, H[0], HT[0]);
+    launch_pdl(k_gather, dim3(B / 4), dim3(KPAD, 4), 0, st, x, id, n_in, B, H[0], HT[0]);
     MCK(cudaGetLastError());
     return 0;
   }
@@ -577,6 +582,7 @@ int dgbgk_mlp_gradient(dgbgk_mlp* m, const float* x, const float* t, int n, doub
   if (!m || !x || !t || n != m->B) return set_error("dgbgk_mlp_gradient: n must equal the batch size"), DGBGK_EINVAL;
   MCK(cudaSetDevice(m->device));
   MTRY(m->load_batch_host(x, t, n));
+  MCK(cudaMemsetAsync(m->loss, 0, sizeof(double), m->st));
   MTRY(m->forward_loss(m->tin, m->iin, m->loss));
   MTRY(m->backward());
   MTRY(m->check_err());
@@ -644,6 +650,7 @@ int dgbgk_mlp_train(dgbgk_mlp* m, int iters, float lr, unsigned long long seed, 
     id[k] = perm[pos++];
   }
   MCK(cudaMemcpyAsync(m->idx, id.data(), id.size() * sizeof(int), cudaMemcpyHostToDevice, m->st));
+  MCK(cudaMemsetAsync(m->loss, 0, iters * sizeof(double), m->st));
   for (int it = 0; it < iters; ++it) {
     const int* id = m->idx + (size_t)it * B;
     MTRY(m->gather(m->xs, id));

@@ -22,6 +22,8 @@
 
 #include <cstdint>
 
+#include "pdl.cuh"
+
 namespace dgbgk {
 namespace umma {
 
@@ -228,6 +230,10 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap& ta, const CUtensorM
   __syncthreads();
   fence_after();
   const uint32_t tmem = tmem_base;
+  // the tensor memory is held: a CTA of the next kernel that waits for some
+  // waits for CTAs that need nothing more
+  grid_launch_dependents();
+  grid_wait();  // the operands, and the readers of what the epilogue writes
 
   if (warp == 0 && elect_one()) {
     // producer: stage s = kb % STAGES once the MMAs of kb - STAGES have
