@@ -424,7 +424,7 @@ int enqueue_step(const LaunchSet<T>& L, cudaStream_t st, float* ms = nullptr, co
       TRY(launch_check("k_wspec", g, 256, 0));
     }
     if (c.spec_seq) {
-      const int g = (c.n_spec_slots + 255) / 256;
+      const int g = (c.n_spec_slots + 7) / 8;
       k_wspec<T><<<g, 256, 0, st>>>(c, 1);
       TRY(launch_check("k_wspec", g, 256, 0));
     }

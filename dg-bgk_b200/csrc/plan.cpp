@@ -172,28 +172,40 @@ static int build_specular(const dgbgk_mesh& m, const dgbgk_vspace& vs, Plan& pl,
   pl.spec_par.clear();
   pl.spec_seq.clear();
   pl.spec_seq_off.assign(ns + 1, 0);
+  std::vector<int> level(V);
+  std::vector<std::vector<int>> at;  // a slot's sequential items by level - 1
   for (int s = 0; s < ns; ++s) {
     const int e = pl.welem[s];
+    at.clear();
     for (int v = 0; v < V; ++v) {
       if (!mask[(size_t)s * V + v]) continue;
-      bool dep = false;
-      for (int k = 0; k < 3 && !dep; ++k) {
+      level[v] = 0;
+      for (int k = 0; k < 3; ++k) {
         const PlanEdge& ed = pl.edge[3 * (size_t)e + k];
         if ((ed.low & 3) != 3) continue;
         const size_t o = ((size_t)pl.rside[ed.bside] * V + v) * 2;
         if (pl.rf_i[o] < 0) continue;
-        for (int j = 0; j < 2 && !dep; ++j) {
+        for (int j = 0; j < 2; ++j) {
           const int I = pl.rf_i[o + j];
           const unsigned char mI = mask[(size_t)s * V + I];
-          if (I < v && (((mI >> k) & 1) || ((mI >> ((k + 1) % 3)) & 1))) dep = true;
+          if (I < v && (((mI >> k) & 1) || ((mI >> ((k + 1) % 3)) & 1))) level[v] = std::max(level[v], level[I] + 1);
         }
       }
-      if (dep)
-        pl.spec_seq.push_back(s * V + v);
-      else
+      if (level[v] == 0) {
         pl.spec_par.push_back(s * V + v);
+        continue;
+      }
+      if ((int)at.size() < level[v]) at.resize(level[v]);
+      at[level[v] - 1].push_back(s * V + v);
     }
-    pl.spec_seq_off[s + 1] = (int)pl.spec_seq.size();
+    for (const auto& l : at) {
+      const int end = (int)(pl.spec_seq.size() / 2 + l.size());
+      for (int it : l) {
+        pl.spec_seq.push_back(it);
+        pl.spec_seq.push_back(end);
+      }
+    }
+    pl.spec_seq_off[s + 1] = (int)(pl.spec_seq.size() / 2);
   }
   pl.spec = true;
   return 0;

@@ -59,7 +59,8 @@ struct Plan {
   // velocity loop updates it in place, so velocities I < v contribute their
   // new values.  Items are (wall element slot, v) pairs with some node
   // deferred; an item whose mirrored velocities include an earlier deferred
-  // one is "sequential" (processed per element in velocity order).
+  // one is "sequential" (processed per element, by the length of the chain of
+  // such items before it: its level).
   bool spec = false;
   std::vector<int> welem;         // wall elements (plan order) by slot
   std::vector<int> wslot;         // [E] slot of each element, -1 without a wall side
@@ -68,7 +69,7 @@ struct Plan {
   std::vector<double> rf_z;       // [rows][V][2] ZD1, ZD2
   std::vector<int> spec_par;      // items slot*V + v processed in parallel
   std::vector<int> spec_seq_off;  // [slots + 1]
-  std::vector<int> spec_seq;      // sequential items, per slot in velocity order
+  std::vector<int> spec_seq;      // sequential items, per slot by level: (item, where its level ends) pairs
 };
 
 // Device edge word of edge i = 3*e + k (ElemEdge::info): the kind, the

@@ -85,3 +85,16 @@ def test_default_fp64_tile_follows_the_tile_count(nt):
     assert s.info()["tile_elems"] == (64 if 16 * nt <= nsm else 128)
     s.advance(2), o.advance(2)
     assert rel_l2(s.get_state(), o.get_state()) <= TOL64
+
+
+@pytest.mark.parametrize("immat", [1, 0])
+@pytest.mark.parametrize("prec,n", [(64, 12), (64, 17), (32, 18)])
+def test_specular_chains_of_corner_elements(prec, n, immat):
+    # ALPHA < 1: a corner element's velocities wait on one another in chains of
+    # several levels, taken level by level
+    c = cavity_case(6, n, n, mach=0.4, kn=0.5)
+    c.immat, c.alpha = immat, 0.9
+    s, o, _ = pair(c, prec=prec)
+    r, q = s.advance(4), o.advance(4)
+    assert rel_l2(s.get_state(), o.get_state()) <= tol(prec)
+    assert rel_l2(r["res_l2"], q["res_l2"]) <= (1e-9 if prec == 64 else 1e-4)
