@@ -891,14 +891,20 @@ template <class T> struct Impl : ImplBase {
     return refresh();
   }
 
+  // Room for the histories of n steps.  The old ones go first, so that longer
+  // ones need no room beside them; until the new ones and the launch set that
+  // names them are there, hist_cap is 0 and every path to a sweep comes back
+  // here (an allocation that failed left the launch set with freed addresses).
   int ensure_hist(int n) {
     if (n <= hist_cap) return 0;
+    hist_cap = 0;
     dfree(hist_linf);
+    hist_l2 = hist_dt = nullptr;
     TRY(dalloc(&hist_linf, 3 * (size_t)n));
     hist_l2 = hist_linf + n;
     hist_dt = hist_l2 + n;
-    hist_cap = n;
     if (halo) TRY(refresh());
+    hist_cap = n;
     return 0;
   }
 
@@ -967,6 +973,10 @@ template <class T> struct Impl : ImplBase {
     const int n3 = 3 * pl.E;
     const int gw = (n3 * 32 + 255) / 256;  // a warp per DG node
     const CaseDev<T>& C = single.one_case;
+    if ((k == 3 || k == 4) && hist_cap == 0) {
+      set_error("dgbgk_shard_phase: no step history (the last dgbgk_shard_begin failed)");
+      return DGBGK_ECUDA;
+    }
     if (k == 1) {
       k_shard_sums1<T><<<gw, 256, 0, st>>>(C, sums1);
     } else if (k == 2) {

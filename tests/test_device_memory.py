@@ -1,0 +1,107 @@
+"""The library's host code where device memory runs short or sizes are extreme,
+against a CUDA runtime in host memory (tests/host_runtime.cpp; CPU): kernels do
+nothing there, and a launch that is given a freed address is counted."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import PKG, ROOT
+
+PRELUDE = """
+import ctypes, sys
+sys.path.insert(0, {pkg!r})
+from dgbgk import _lib
+_lib.use_library({lib!r})
+import numpy as np
+from dgbgk import Batch, Solver, cavity_case
+from dgbgk.warmstart import MLP
+hr = _lib.lib()
+for f in (hr.hr_limit, hr.hr_largest):
+    f.argtypes = [ctypes.c_size_t]
+hr.hr_largest.restype = ctypes.c_size_t
+hr.hr_fail_at.argtypes = [ctypes.c_long]
+hr.hr_last_bad.restype = ctypes.c_char_p
+def fails(f, limit):
+    # f runs out of device memory in an allocation of more than limit bytes
+    hr.hr_limit(limit)
+    try:
+        f()
+    except _lib.DgbgkError as e:
+        assert "out of memory" in str(e), e
+    else:
+        raise AssertionError("did not fail")
+    finally:
+        hr.hr_limit(0)
+def solver(n=4, prec=64, **more):
+    s = Solver.from_case(cavity_case(n, 4, 8, mach=0.3, kn=0.1), precision=prec, **more)
+    s.init_case()
+    return s
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    objs = [os.path.join(PKG, "_build", f"{n}.o") for n in ("dgbgk", "mlp", "plan", "setup_host")]
+    cuda = "/usr/local/cuda/include"
+    if not all(os.path.exists(p) for p in objs + [os.path.join(cuda, "cuda_runtime_api.h")]):
+        pytest.skip("the library's objects and CUDA's headers are needed")
+    lib = str(tmp_path_factory.mktemp("hr") / "libhr.so")
+    gxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
+    r = subprocess.run([gxx, "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", cuda, "-I",
+                        os.path.join(PKG, "csrc"), "-o", lib, os.path.join(ROOT, "tests", "host_runtime.cpp")] + objs,
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+    def go(body):
+        code = PRELUDE.format(pkg=PKG, lib=lib) + body + "\nassert hr.hr_bad() == 0, hr.hr_last_bad()\n"
+        r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stderr
+
+    return go
+
+
+@pytest.mark.parametrize("prec", [64, 32])
+def test_a_history_that_does_not_fit_leaves_no_freed_one_behind(run, prec):
+    run(f"""
+s = solver(prec={prec})
+assert s.advance(1500)["steps"] == 3
+for again in (1200, 1500, 4):           # within what the handle held before
+    fails(lambda: s.advance(1_000_000), 4_000_000)
+    assert s.advance(again)["steps"] == 3
+fails(lambda: s.profile(1_000_000), 4_000_000)
+s.profile(2)
+assert s.macros()["rho"].size == s.NP
+""")
+
+
+def test_a_history_that_does_not_fit_and_a_batch(run):
+    run("""
+a, b = solver(), solver(5)
+t = Batch([a, b])
+t.advance(10)
+fails(lambda: a.advance(1_000_000), 4_000_000)
+t.advance(10)                           # the batch's table named the old history
+fails(lambda: t.advance(1_000_000), 4_000_000)
+t.advance(10)
+assert a.advance(10)["steps"] == 3
+""")
+
+
+def test_a_shard_without_its_history_is_refused(run):
+    run("""
+from dgbgk.cases import gll
+from dgbgk.solver import setup_mesh, vspace
+c = cavity_case(4, 4, 8, mach=0.3, kn=0.1)
+m = c.mesh
+vc, sw = vspace(c.rorder, c.torder, *gll(c.rorder))
+s = Solver(m.intma, m.coord, m.bsido, setup_mesh(m.intma, m.coord, m.bsido), vc, sw, c.rorder, c.torder, c.rv,
+           rgas=c.rgas, molar_mass=c.molar_mass, diameter=c.diameter, wall_velocity=m.wall_velocity, shard=1)
+L, p = _lib.lib(), ctypes.c_void_p(256)
+assert L.dgbgk_shard_begin(s.h, 4, 0.0) == 0 and L.dgbgk_shard_phase(s.h, 4, p, p, p) == 0
+fails(lambda: _lib.check(L.dgbgk_shard_begin(s.h, 1_000_000, 0.0)), 4_000_000)
+assert L.dgbgk_shard_phase(s.h, 3, p, p, p) == _lib.DGBGK_ECUDA
+assert L.dgbgk_shard_phase(s.h, 4, p, p, p) == _lib.DGBGK_ECUDA
+assert L.dgbgk_shard_begin(s.h, 4, 0.0) == 0 and L.dgbgk_shard_phase(s.h, 3, p, p, p) == 0
+""")
