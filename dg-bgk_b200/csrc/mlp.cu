@@ -219,6 +219,17 @@ template <class X> void mfree(X*& p) {
   p = nullptr;
 }
 
+// room for n values, the old ones freed first; none (cap 0) when the new
+// allocation fails
+template <class X> int room(X*& p, size_t& cap, size_t n) {
+  if (n <= cap) return 0;
+  cap = 0;
+  mfree(p);
+  MTRY(mall(&p, n));
+  cap = n;
+  return 0;
+}
+
 struct Layer {
   int in = 0, in_live = 0, out = 0;
   float *w = nullptr, *b = nullptr, *gw = nullptr, *gb = nullptr;
@@ -236,12 +247,12 @@ struct dgbgk_mlp {
   std::vector<__nv_bfloat16*> G, GT;     // dZ of layers 1..depth, and dP (index depth+1)
   float* P = nullptr;
   double* loss = nullptr;                // one slot per training step (slot 0 otherwise)
-  int loss_cap = 1;
+  size_t loss_cap = 0;
   int* err = nullptr;
   float *xs = nullptr, *ts = nullptr;    // training set
   int nset = 0;
   int* idx = nullptr;
-  int idx_cap = 0;
+  size_t idx_cap = 0;
   float *xin = nullptr, *tin = nullptr;  // staging of one host batch
   int* iin = nullptr;
   long long adam_t = 0;
@@ -310,7 +321,7 @@ struct dgbgk_mlp {
       MTRY(mall(&GT[l], (size_t)B * c));
     }
     MTRY(mall(&P, (size_t)B * n_out));
-    MTRY(mall(&loss, 1));
+    MTRY(room(loss, loss_cap, 1));
     MTRY(mall(&err, 1));
     MTRY(mall(&xin, (size_t)B * n_in));
     MTRY(mall(&tin, (size_t)B * n_out));
@@ -582,6 +593,7 @@ int dgbgk_mlp_gradient(dgbgk_mlp* m, const float* x, const float* t, int n, doub
   if (!m || !x || !t || n != m->B) return set_error("dgbgk_mlp_gradient: n must equal the batch size"), DGBGK_EINVAL;
   MCK(cudaSetDevice(m->device));
   MTRY(m->load_batch_host(x, t, n));
+  MTRY(room(m->loss, m->loss_cap, 1));
   MCK(cudaMemsetAsync(m->loss, 0, sizeof(double), m->st));
   MTRY(m->forward_loss(m->tin, m->iin, m->loss));
   MTRY(m->backward());
@@ -627,16 +639,8 @@ int dgbgk_mlp_train(dgbgk_mlp* m, int iters, float lr, unsigned long long seed, 
   const int B = m->B;
   if (iters == 0) return 0;
   MCK(cudaStreamSynchronize(m->st));
-  if (m->idx_cap < iters * B) {
-    mfree(m->idx);
-    MTRY(mall(&m->idx, (size_t)iters * B));
-    m->idx_cap = iters * B;
-  }
-  if (m->loss_cap < iters) {
-    mfree(m->loss);
-    MTRY(mall(&m->loss, iters));
-    m->loss_cap = iters;
-  }
+  MTRY(room(m->idx, m->idx_cap, (size_t)iters * B));
+  MTRY(room(m->loss, m->loss_cap, (size_t)iters));
   std::vector<int> id((size_t)iters * B);
   std::mt19937_64 rng(seed);
   std::vector<int> perm(m->nset);

@@ -105,3 +105,26 @@ assert L.dgbgk_shard_phase(s.h, 3, p, p, p) == _lib.DGBGK_ECUDA
 assert L.dgbgk_shard_phase(s.h, 4, p, p, p) == _lib.DGBGK_ECUDA
 assert L.dgbgk_shard_begin(s.h, 4, 0.0) == 0 and L.dgbgk_shard_phase(s.h, 3, p, p, p) == 0
 """)
+
+
+@pytest.mark.parametrize("k", [1, 2])
+def test_a_training_call_that_does_not_fit_leaves_the_network_usable(run, k):
+    # the k-th buffer that a longer call needs (the rows' indices, the losses)
+    run(f"""
+m = MLP(3, 128, 1, 128, 128, seed=1)
+x, t = np.zeros((128, 3), np.float32), np.zeros((128, 128), np.float32)
+m.set_data(x, t)
+m.train(4)
+for longer in (40, 80):
+    hr.hr_fail_at({k})
+    try:
+        m.train(longer)
+    except _lib.DgbgkError as e:
+        assert "out of memory" in str(e), e
+    else:
+        raise AssertionError("did not fail")
+    m.gradient(x, t)
+    assert m.train(4).size == 4
+    hr.hr_fail_at(-1)
+assert m.train(40).size == 40
+""")
