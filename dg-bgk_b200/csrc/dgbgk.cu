@@ -567,7 +567,7 @@ template <class T> struct Impl : ImplBase {
   WallSide* walls = nullptr;
   int *node_off = nullptr, *node_dg = nullptr;
   double* node_ae = nullptr;
-  double *hist_linf = nullptr, *hist_l2 = nullptr, *hist_dt = nullptr;  // one allocation, pitch hist_cap
+  double* hist = nullptr;  // [hist_cap][3] per step of an advance call: max residual, L2 residual, DTE
   double* init_buf = nullptr;  // inputs of the init kernels, kept between calls
   size_t init_cap = 0;
   double* nodal = nullptr;     // [6*NP] nodal fields of macros()
@@ -624,7 +624,7 @@ template <class T> struct Impl : ImplBase {
     dfree(node_off);
     dfree(node_dg);
     dfree(node_ae);
-    dfree(hist_linf);
+    dfree(hist);
     dfree(init_buf);
     dfree(nodal);
     dfree(ctrl);
@@ -782,9 +782,7 @@ template <class T> struct Impl : ImplBase {
     hc.disuy = disuy;
     hc.disps = disps;
     hc.mu = mu;
-    hc.hist_linf = hist_linf;
-    hc.hist_l2 = hist_l2;
-    hc.hist_dt = hist_dt;
+    hc.hist = hist;
     hc.ctrl = ctrl;
     hc.MM = pl.M / 6.022e26;
     hc.sigt = 3.1416 * pl.d * pl.d;
@@ -898,11 +896,8 @@ template <class T> struct Impl : ImplBase {
   int ensure_hist(int n) {
     if (n <= hist_cap) return 0;
     hist_cap = 0;
-    dfree(hist_linf);
-    hist_l2 = hist_dt = nullptr;
-    TRY(dalloc(&hist_linf, 3 * (size_t)n));
-    hist_l2 = hist_linf + n;
-    hist_dt = hist_l2 + n;
+    dfree(hist);
+    TRY(dalloc(&hist, 3 * (size_t)n));
     if (halo) TRY(refresh());
     hist_cap = n;
     return 0;
@@ -943,13 +938,17 @@ template <class T> struct Impl : ImplBase {
     ref_host = c.ref;
     cur = c.cur;
     itime_total += ns;
-    if (ns > 0 && (linf || l2 || dt)) {  // the three histories in one copy
-      const size_t w = (size_t)ns * sizeof(double);
-      std::vector<double> h(3 * (size_t)ns);
-      CK(cudaMemcpy2D(h.data(), w, hist_linf, (size_t)hist_cap * sizeof(double), w, 3, cudaMemcpyDeviceToHost));
+    if (linf || l2 || dt) {  // a step's three values lie together: one copy (HIST_CHUNK steps) for all
+      constexpr int HIST_CHUNK = 1 << 16;
       double* dsts[3] = {linf, l2, dt};
-      for (int k = 0; k < 3; ++k)
-        if (dsts[k]) std::memcpy(dsts[k], h.data() + (size_t)k * ns, w);
+      std::vector<double> h(3 * (size_t)std::min(ns, HIST_CHUNK));
+      for (int s0 = 0; s0 < ns; s0 += HIST_CHUNK) {
+        const int n = std::min(HIST_CHUNK, ns - s0);
+        CK(cudaMemcpy(h.data(), hist + 3 * (size_t)s0, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost));
+        for (int k = 0; k < 3; ++k)
+          if (dsts[k])
+            for (int i = 0; i < n; ++i) dsts[k][s0 + i] = h[3 * (size_t)i + k];
+      }
     }
     return finish_status(c);
   }
@@ -2042,7 +2041,7 @@ template <class T> struct BatchImpl : BatchBase {
       }
       if (steps) steps[i] = ns[i];
       if (l2 && ns[i] > 0)
-        CK(cudaMemcpyAsync(&h_l2[i], c->hist_l2 + ns[i] - 1, sizeof(double), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(&h_l2[i], c->hist + 3 * (size_t)(ns[i] - 1) + 1, sizeof(double), cudaMemcpyDeviceToHost, st));
     }
     if (l2) {
       CK(cudaStreamSynchronize(st));

@@ -124,9 +124,7 @@ template <class T> struct alignas(64) CaseDev {
   double* disuy;
   double* disps;
   double* mu;
-  double* hist_linf;  // per step of an advance call
-  double* hist_l2;
-  double* hist_dt;
+  double* hist;  // [step][3] of an advance call: max residual, L2 residual, DTE
   Ctrl* ctrl;
   double MM, sigt;  // M/NA, PI*d*d
   T alpha;
@@ -782,9 +780,10 @@ template <class T> __device__ __forceinline__ void resid_book(const CaseDev<T>& 
   Ctrl* c = C.ctrl;
   const int st = c->step;
   const double l2 = sqrt(sq);
-  C.hist_linf[st] = mm;
-  C.hist_l2[st] = l2;
-  C.hist_dt[st] = step_dt(c);
+  double* h = C.hist + 3 * (size_t)st;
+  h[0] = mm;
+  h[1] = l2;
+  h[2] = step_dt(c);
   if (!isfinite(l2) || !isfinite(mm)) {
     c->nonfinite = 1;
     c->done = 1;

@@ -8,7 +8,8 @@
 // allocation.  Freed memory is kept, so an address never comes back.
 // hr_limit(n): allocations of more than n bytes fail (0: none do); hr_fail_at(k):
 // the k-th allocation from now on fails.
-// A read of a case's control block says that the march ended after three steps.
+// A read of a case's control block says that the march ended after hr_steps
+// (three) steps.  hr_block(size): the live allocation of that size.
 #include <cuda.h>
 #include <cuda_runtime_api.h>
 
@@ -31,7 +32,7 @@ struct Block {
 std::map<uintptr_t, Block> blocks;
 size_t limit_bytes = 0;
 long fail_at = -1;
-int bad = 0;
+int march_steps = 3, bad = 0;
 std::string last_bad;
 // (a function's static: the objects register their kernels before this file's are made)
 std::map<const void*, std::string>& kernels() {
@@ -113,7 +114,7 @@ cudaError_t copy(void* d, const void* s, size_t n, cudaMemcpyKind k) {
   if ((to && !device_range(d, n, "copy to")) || (from && !device_range(s, n, "copy from"))) return cudaErrorInvalidValue;
   if (k == cudaMemcpyDeviceToHost && n == sizeof(dgbgk::Ctrl)) {
     auto* c = (dgbgk::Ctrl*)s;
-    c->step = std::min(c->max_steps, 3);
+    c->step = std::min(c->max_steps, march_steps);
     c->done = 1;
   }
   std::memmove(d, s, n);
@@ -124,14 +125,13 @@ cudaError_t copy(void* d, const void* s, size_t n, cudaMemcpyKind k) {
 extern "C" {
 void hr_limit(size_t n) { limit_bytes = n; }
 void hr_fail_at(long k) { fail_at = k; }
+void hr_steps(int n) { march_steps = n; }
 int hr_bad() { return bad; }
 const char* hr_last_bad() { return last_bad.c_str(); }
-// the largest live allocation of at most `most` bytes
-size_t hr_largest(size_t most) {
-  size_t n = 0;
+void* hr_block(size_t size) {
   for (const auto& b : blocks)
-    if (b.second.live && b.second.size <= most) n = std::max(n, b.second.size);
-  return n;
+    if (b.second.live && b.second.size == size) return (void*)b.first;
+  return nullptr;
 }
 
 cudaError_t cudaMalloc(void** p, size_t n) {

@@ -18,9 +18,8 @@ import numpy as np
 from dgbgk import Batch, Solver, cavity_case
 from dgbgk.warmstart import MLP
 hr = _lib.lib()
-for f in (hr.hr_limit, hr.hr_largest):
-    f.argtypes = [ctypes.c_size_t]
-hr.hr_largest.restype = ctypes.c_size_t
+hr.hr_limit.argtypes = hr.hr_block.argtypes = [ctypes.c_size_t]
+hr.hr_block.restype = ctypes.c_void_p
 hr.hr_fail_at.argtypes = [ctypes.c_long]
 hr.hr_last_bad.restype = ctypes.c_char_p
 def fails(f, limit):
@@ -127,4 +126,30 @@ for longer in (40, 80):
     assert m.train(4).size == 4
     hr.hr_fail_at(-1)
 assert m.train(40).size == 40
+""")
+
+
+def test_histories_of_a_call_with_a_very_large_step_limit(run):
+    # rows of 8 B a step would be further apart than a 2-D copy's pitch may be
+    run("""
+s = solver()
+r = s.advance(2 ** 28 + 1, tol=0.5)
+assert r["steps"] == 3 and r["res_l2"].size == 3
+assert s.advance(5)["steps"] == 3       # the handle keeps the room
+""")
+
+
+@pytest.mark.parametrize("n", [1, 65535, 65536, 65537, 200_000])
+def test_histories_come_back_by_kind_and_step(run, n):
+    # written where the sweep writes them: three values a step
+    run(f"""
+s = solver()
+hr.hr_steps({n})
+s.advance(300_000)
+want = np.arange(3.0 * 300_000).reshape(-1, 3)
+ctypes.memmove(hr.hr_block(want.nbytes), want.ctypes.data, want.nbytes)
+r = s.advance(300_000)
+assert r["steps"] == {n}
+for k, name in enumerate(("res_linf", "res_l2", "dte")):
+    assert np.array_equal(r[name], want[:{n}, k]), name
 """)
