@@ -1895,6 +1895,7 @@ template <class T> struct BatchImpl : BatchBase {
   // tile shape on the cases' current states, restoring the states after
   // each, and keeps the fastest.
   int autotune(int fixed_eb, int fixed_upc, int fixed_rows, int steps) {
+    for (auto* c : cs) TRY(c->ensure_hist(steps + 1));
     std::vector<T*> backup(cs.size(), nullptr);
     int rc = 0;
     for (size_t i = 0; i < cs.size() && rc == 0; ++i) {

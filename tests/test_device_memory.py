@@ -153,3 +153,14 @@ assert r["steps"] == {n}
 for k, name in enumerate(("res_linf", "res_l2", "dte")):
     assert np.array_equal(r[name], want[:{n}, k]), name
 """)
+
+
+@pytest.mark.parametrize("tune_steps", [4, 1022, 1023, 1024, 5000])
+def test_the_autotuner_has_a_history_for_its_steps(run, tune_steps):
+    # tune_steps timed steps after an untimed one, 24 B of history each (room
+    # for 1024 steps from the start)
+    run(f"""
+s = solver()
+Batch([s], tune_steps={tune_steps})
+assert hr.hr_block(24 * max(1024, {tune_steps} + 1))
+""")
