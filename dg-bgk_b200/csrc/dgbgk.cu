@@ -1113,17 +1113,18 @@ template <class T> struct Impl : ImplBase {
       return DGBGK_EINVAL;
     }
     CK(cudaStreamSynchronize(st));
+    drop_graphs();  // the step graph takes the record kernels or leaves them out
     dfree(out_ring);
     dfree(out_count);
-    out_every = every;
-    out_cap = every > 0 ? cap : 0;
+    out_every = out_cap = 0;  // off until the new ring is there
     if (every > 0) {
       TRY(dalloc(&out_ring, (size_t)cap * rec_len()));
       TRY(dalloc(&out_count, 1));
       CK(cudaMemsetAsync(out_count, 0, sizeof(int), st));
       CK(cudaStreamSynchronize(st));
+      out_every = every;
+      out_cap = cap;
     }
-    drop_graphs();  // the step graph takes the record kernels or leaves them out
     return 0;
   }
   int output_count(int* n) override {

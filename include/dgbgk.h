@@ -189,7 +189,8 @@ int dgbgk_get_forces(dgbgk_handle* h, double* lift, double* drag);
  * set (dgbgk_set_state*, dgbgk_init_*), counted across advance calls and
  * carried over by dgbgk_copy_state -- is a multiple of `every`, into a
  * device ring of `capacity` records (the oldest is overwritten).  Each call
- * replaces the ring; every = 0 stops recording.  Batches do not record. */
+ * replaces the ring; every = 0 stops recording, as does a call that finds no
+ * room for its ring.  Batches do not record. */
 int dgbgk_set_output(dgbgk_handle* h, int every, int capacity);
 /* Records taken since dgbgk_set_output (the ring holds the last
  * min(count, capacity)). */

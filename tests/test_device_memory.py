@@ -164,3 +164,19 @@ s = solver()
 Batch([s], tune_steps={tune_steps})
 assert hr.hr_block(24 * max(1024, {tune_steps} + 1))
 """)
+
+
+@pytest.mark.parametrize("held", [True, False])
+def test_an_output_ring_that_does_not_fit_is_off(run, held):
+    run(f"""
+s = solver()
+if {held}:
+    s.set_output(2, capacity=4)
+s.advance(8)
+fails(lambda: s.set_output(2, capacity=1_000_000), 4_000_000)
+s.advance(8)
+s.advance(2000)                         # the step graphs are captured anew
+assert s.outputs() == []
+s.set_output(2, capacity=4)
+s.advance(8)
+""")
