@@ -557,6 +557,7 @@ template <class T> struct Impl : ImplBase {
   ElemRec<T>* rec = nullptr;
   int* halo = nullptr;  // [nblocks][hp]
   int hp = 0;
+  bool tiled = false;  // halo, rec and the launch set are those of pl's blocks
   T *cmax = nullptr, *cmin = nullptr;
   T* tabs = nullptr;  // moment tables [MOM_TABS][Vp]
   double *nraw = nullptr, *disux = nullptr, *disuy = nullptr, *disps = nullptr, *mu = nullptr;
@@ -827,7 +828,10 @@ template <class T> struct Impl : ImplBase {
       set_error("tile_elems must be 64 or 128");
       return DGBGK_EINVAL;
     }
-    if (pl.EB != eb || halo == nullptr) {
+    const bool same = tiled && pl.EB == eb;
+    tiled = false;
+    if (!same) {
+      ++gen;
       build_blocks(pl, eb);
       if (eb == 128 && SweepGeo<T>::smem(eb, pl.max_halo, 1) > SWEEP_SMEM_MAX) {
         // a halo too wide for this tile (an element order without locality):
@@ -886,8 +890,13 @@ template <class T> struct Impl : ImplBase {
       return DGBGK_EUNSUP;
     }
     tpu = tiles_per_unit_alone((long)pl.nblocks * nvt(), sps * nsm, nvt());
-    return refresh();
+    TRY(refresh());
+    tiled = true;
+    return 0;
   }
+  // Before any kernel on the records: a re-blocking that failed on the way (a
+  // batch's, out of memory) has freed the old ones.
+  int ensure_tile() { return tiled ? 0 : set_tile(pl.EB); }
 
   // Room for the histories of n steps.  The old ones go first, so that longer
   // ones need no room beside them; until the new ones and the launch set that
@@ -898,7 +907,7 @@ template <class T> struct Impl : ImplBase {
     hist_cap = 0;
     dfree(hist);
     TRY(dalloc(&hist, 3 * (size_t)n));
-    if (halo) TRY(refresh());
+    if (tiled) TRY(refresh());
     hist_cap = n;
     return 0;
   }
@@ -963,6 +972,7 @@ template <class T> struct Impl : ImplBase {
   // (res[1]) over the shards between them, on this stream.
   int shard_begin(int max_steps, double tol) override {
     CK(cudaSetDevice(device));
+    TRY(ensure_tile());
     TRY(ensure_hist(std::max(max_steps, 1)));
     TRY(upload_ctrl(max_steps, tol));
     CK(cudaEventRecord(ev0, st));
@@ -993,6 +1003,7 @@ template <class T> struct Impl : ImplBase {
     } else if (k == 4) {
       k_shard_resid<T><<<1, 32, 0, st>>>(C, res);
     } else if (k == 0) {  // before phases 1, 2 and 5 outside a step: the kernels run
+      TRY(ensure_tile());
       TRY(aux_ctrl());
     } else if (k == 5) {  // the moments of the current state from the summed sums (no sweep)
       const int nt = std::max(n3, (int)pl.walls.size());
@@ -1032,6 +1043,7 @@ template <class T> struct Impl : ImplBase {
     if (steps) *steps = 0;
     if (max_steps == 0) return 0;
     CK(cudaSetDevice(device));
+    TRY(ensure_tile());
     TRY(ensure_hist(max_steps));
     const OutArgs oa = out_args(-1, nullptr);
     TRY(graphs.prepare(st, max_steps, [&] { return enqueue_step(single, st, nullptr, out_every > 0 ? &oa : nullptr); }));
@@ -1161,6 +1173,7 @@ template <class T> struct Impl : ImplBase {
 
   int profile(int nsteps, double* ms) override {
     CK(cudaSetDevice(device));
+    TRY(ensure_tile());
     TRY(ensure_hist(std::max(nsteps, 1)));
     TRY(upload_ctrl(nsteps, 0.0));
     double acc[4] = {0, 0, 0, 0};
@@ -1392,6 +1405,7 @@ template <class T> struct Impl : ImplBase {
   // last phase 3 or 5: the sums are over every shard)
   int moments_now() {
     if (shard) return 0;
+    TRY(ensure_tile());
     TRY(aux_ctrl());
     mom_fn<T>(single.mom_rows, true)<<<single.mom_grid, single.mom_warps * 32, single.mom_smem, st>>>(
         single.args, single.total_groups, single.one_case);

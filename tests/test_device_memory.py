@@ -180,3 +180,26 @@ assert s.outputs() == []
 s.set_output(2, capacity=4)
 s.advance(8)
 """)
+
+
+@pytest.mark.parametrize("prec", [64, 32])
+def test_a_re_blocking_that_does_not_fit_is_made_up_for(run, prec):
+    # every allocation of a batch that re-blocks its case fails in turn; the
+    # case alone and the batch that held it before go on
+    run(f"""
+s = solver(prec={prec})
+t = Batch([s], tile_elems=64)
+for k in range(1, 9):
+    hr.hr_fail_at(k)
+    try:
+        Batch([s], tile_elems=128)
+    except _lib.DgbgkError:
+        pass
+    hr.hr_fail_at(-1)
+    if k % 2:
+        s.advance(4)
+        s.macros()
+    t.advance(4)
+    s.macros()
+    s.profile(2)
+""")
