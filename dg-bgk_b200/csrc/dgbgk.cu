@@ -113,7 +113,7 @@ template <class T> struct LaunchSet {
   int* d_off = nullptr;  // [3][n + 1]: sweep units, moment row groups, wall sides
   BatchCtl* d_ctl = nullptr;
   BatchArgs<T> args{};
-  int n = 0, cap = 0, total_units = 0, total_groups = 0, total_walls = 0;
+  int n = 0, cap = 0, total_units = 0, total_groups = 0, total_walls = 0, nsm = 0;
   int eb = 128, immat = 1;
   bool one = false;       // a single case: the kernels take it as a parameter
   CaseDev<T> one_case{};  // that case (zeros for a batch)
@@ -322,6 +322,7 @@ int build_launch_set(LaunchSet<T>& L, const std::vector<CaseDev<T>>& cs, int eb,
   for (int j = 0; j < EXP_TAB; ++j) ctl.etab[j] = std::exp2((double)j / EXP_TAB);
   CK(cudaMemcpyAsync(L.d_ctl, &ctl, sizeof(BatchCtl), cudaMemcpyHostToDevice, st));
   L.n = n;
+  L.nsm = nsm;
   L.one = one;
   L.one_case = one ? cs[0] : CaseDev<T>{};
   L.eb = eb;
@@ -419,7 +420,7 @@ int enqueue_step(const LaunchSet<T>& L, cudaStream_t st, float* ms = nullptr, co
   // ones that wait on earlier deferred velocities
   for (const auto& c : L.spec_cases) {
     if (c.n_spec_par > 0) {
-      const int g = std::min(4 * 148, (c.n_spec_par + 255) / 256);
+      const int g = std::min(4 * L.nsm, (c.n_spec_par + 255) / 256);
       k_wspec<T><<<g, 256, 0, st>>>(c, 0);
       TRY(launch_check("k_wspec", g, 256, 0));
     }

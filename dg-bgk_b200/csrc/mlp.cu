@@ -101,13 +101,14 @@ struct Gemm {
 // CTAs of 128 x 128 tiles, 75 with 16 of 128 x 32.
 constexpr int STAGES32 = 5, STAGES64 = 2, STAGES_ADAM = 2;
 
-int plan_gemm(Gemm& G, const __nv_bfloat16* A, const __nv_bfloat16* B, int M, int N, int K, int epi, GemmArgs g) {
+int plan_gemm(Gemm& G, const __nv_bfloat16* A, const __nv_bfloat16* B, int M, int N, int K, int epi, GemmArgs g,
+              int nsm) {
   if (M % BM || N % 64 || (K % (2 * BK) && !(K == BK && epi == EPI_TANH))) {
     set_error("MLP GEMM shape not a multiple of the tile");
     return DGBGK_EINVAL;
   }
   G.epi = epi;
-  G.bn = epi != EPI_ADAM && epi != EPI_F32 && (long)(M / BM) * (N / 64) < 148 ? 32 : 64;
+  G.bn = epi != EPI_ADAM && epi != EPI_F32 && (long)(M / BM) * (N / 64) < nsm ? 32 : 64;
   MTRY(bf16_map(&G.ta, A, M, K, BM));
   MTRY(bf16_map(&G.tb, B, N, K, G.bn));
   G.g = g;
@@ -240,7 +241,7 @@ struct Layer {
 }  // namespace
 
 struct dgbgk_mlp {
-  int device = 0, n_in = 0, width = 0, depth = 0, n_out = 0, B = 0;
+  int device = 0, nsm = 0, n_in = 0, width = 0, depth = 0, n_out = 0, B = 0;
   cudaStream_t st = nullptr;
   std::vector<Layer> L;                  // depth + 1 layers
   std::vector<__nv_bfloat16*> H, HT;     // activations 0..depth (0 = input), [B][in] and [in][B]
@@ -357,27 +358,27 @@ struct dgbgk_mlp {
       if (l < depth) {
         g.out_bf = H[l + 1];
         g.out_bfT = HT[l + 1];
-        MTRY(plan_gemm(fwd[l], H[l], y.wb, B, y.out, y.in, EPI_TANH, g));
+        MTRY(plan_gemm(fwd[l], H[l], y.wb, B, y.out, y.in, EPI_TANH, g, nsm));
       } else {
         g.out_f = P;
-        MTRY(plan_gemm(fwd[l], H[l], y.wb, B, y.out, y.in, EPI_LINEAR, g));
+        MTRY(plan_gemm(fwd[l], H[l], y.wb, B, y.out, y.in, EPI_LINEAR, g, nsm));
         g.out_bf = G[nl];
         g.out_bfT = GT[nl];
         g.scale = 2.f / (float)((size_t)B * n_out);
-        MTRY(plan_gemm(out_loss, H[l], y.wb, B, y.out, y.in, EPI_LOSS, g));
+        MTRY(plan_gemm(out_loss, H[l], y.wb, B, y.out, y.in, EPI_LOSS, g, nsm));
       }
       // dW_l = G_{l+1}^T H_l: [out][in], K = B
       GemmArgs gw{};
       gw.err = err;
       gw.out_f = y.gw;
-      MTRY(plan_gemm(bwd_dw[l], GT[l + 1], HT[l], y.out, y.in, B, EPI_F32, gw));
+      MTRY(plan_gemm(bwd_dw[l], GT[l + 1], HT[l], y.out, y.in, B, EPI_F32, gw, nsm));
       gw.w = y.w;
       gw.m = y.mw;
       gw.v = y.vw;
       gw.out_bf = y.wb;
       gw.out_bfT = y.wbT;
       gw.live = y.in_live;
-      MTRY(plan_gemm(adam_dw[l], GT[l + 1], HT[l], y.out, y.in, B, EPI_ADAM, gw));
+      MTRY(plan_gemm(adam_dw[l], GT[l + 1], HT[l], y.out, y.in, B, EPI_ADAM, gw, nsm));
       // G_l = (G_{l+1} W_l) (1 - H_l^2): [B][in], K = out (not for the input layer)
       if (l > 0) {
         GemmArgs gx{};
@@ -385,7 +386,7 @@ struct dgbgk_mlp {
         gx.aux = H[l];
         gx.out_bf = G[l];
         gx.out_bfT = GT[l];
-        MTRY(plan_gemm(bwd_dx[l], G[l + 1], y.wbT, B, y.in, y.out, EPI_DTANH, gx));
+        MTRY(plan_gemm(bwd_dx[l], G[l + 1], y.wbT, B, y.in, y.out, EPI_DTANH, gx, nsm));
       }
     }
     return 0;
@@ -521,6 +522,7 @@ int dgbgk_mlp_create(int n_in, int width, int depth, int n_out, int batch, unsig
   }
   std::unique_ptr<dgbgk_mlp> m(new dgbgk_mlp());
   m->device = device;
+  m->nsm = prop.multiProcessorCount;
   m->n_in = n_in;
   m->width = width;
   m->depth = depth;

@@ -9,7 +9,9 @@
 // hr_limit(n): allocations of more than n bytes fail (0: none do); hr_fail_at(k):
 // the k-th allocation from now on fails.
 // A read of a case's control block says that the march ended after hr_steps
-// (three) steps.  hr_block(size): the live allocation of that size.
+// (three) steps.  hr_block(size): the live allocation of that size.  hr_sms(n): the
+// device has n SMs.  hr_blocks_of(kernel): the blocks of the largest launch
+// of a kernel whose mangled name has this text.
 #include <cuda.h>
 #include <cuda_runtime_api.h>
 
@@ -32,7 +34,7 @@ struct Block {
 std::map<uintptr_t, Block> blocks;
 size_t limit_bytes = 0;
 long fail_at = -1;
-int march_steps = 3, bad = 0;
+int march_steps = 3, sms = 148, bad = 0;
 std::string last_bad;
 // (a function's static: the objects register their kernels before this file's are made)
 std::map<const void*, std::string>& kernels() {
@@ -81,8 +83,10 @@ void execute(const Launch& l) {
   }
   check_words(l.words.data(), l.words.size(), l.what);
 }
-cudaError_t launch(const void* fn, void** args) {
+std::map<std::string, unsigned> grids;
+cudaError_t launch(const void* fn, dim3 grid, void** args) {
   const std::string& name = kernels()[fn];
+  grids[name] = std::max(grids[name], grid.x * grid.y);
   Launch l;
   if (name.find("k_sweep") != std::string::npos) {
     // (BatchArgs, whose first word is the case table; total units; the case,
@@ -126,6 +130,12 @@ extern "C" {
 void hr_limit(size_t n) { limit_bytes = n; }
 void hr_fail_at(long k) { fail_at = k; }
 void hr_steps(int n) { march_steps = n; }
+void hr_sms(int n) { sms = n; }
+unsigned hr_blocks_of(const char* kernel) {
+  for (const auto& g : grids)
+    if (g.first.find(kernel) != std::string::npos) return g.second;
+  return 0;
+}
 int hr_bad() { return bad; }
 const char* hr_last_bad() { return last_bad.c_str(); }
 void* hr_block(size_t size) {
@@ -172,8 +182,10 @@ cudaError_t cudaMemset(void* d, int v, size_t n) {
 }
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return cudaMemset(d, v, n); }
 
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cudaStream_t) { return launch(f, args); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void* f, void** args) { return launch(f, args); }
+cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3, void** args, size_t, cudaStream_t) { return launch(f, g, args); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) {
+  return launch(f, c->gridDim, args);
+}
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
   capturing = new Graph;
   return cudaSuccess;
@@ -200,12 +212,12 @@ cudaError_t cudaGetDeviceCount(int* n) { return *n = 1, cudaSuccess; }
 cudaError_t cudaGetDeviceProperties(cudaDeviceProp* p, int) {
   std::memset((void*)p, 0, sizeof *p);
   p->major = 10;
-  p->multiProcessorCount = 148;
+  p->multiProcessorCount = sms;
   p->memPitch = 0x7fffffff;
   return cudaSuccess;
 }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
-  *v = a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 227 * 1024 : 148;
+  *v = a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 227 * 1024 : sms;
   return cudaSuccess;
 }
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }

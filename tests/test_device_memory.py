@@ -203,3 +203,23 @@ for k in range(1, 9):
     s.macros()
     s.profile(2)
 """)
+
+
+@pytest.mark.parametrize("sms", [8, 16, 148])
+def test_launch_shapes_follow_the_device(run, sms):
+    run(f"""
+hr.hr_sms({sms})
+# 1024 rows and 128 outputs: 16 tiles of 64 columns, or 32 of 32 where they leave SMs without one
+m = MLP(3, 128, 1, 128, 1024, seed=1)
+m.forward(np.zeros((1024, 3), np.float32))
+narrow, wide = (hr.hr_blocks_of(b"k_gemmILi%dELi%dELi2ELi1E" % t) for t in ((32, 5), (64, 2)))
+assert (narrow, wide) == ((32, 0) if 16 < {sms} else (0, 16)), (narrow, wide)
+# ALPHA < 1: at most four blocks of k_wspec per SM
+c = cavity_case(40, 16, 16, mach=0.3, kn=0.1)
+c.alpha = 0.9
+s = Solver.from_case(c)
+s.init_case()
+s.advance(1)
+blocks = hr.hr_blocks_of(b"k_wspec")
+assert 32 <= blocks <= 4 * {sms} and (blocks == 32) == ({sms} == 8), blocks
+""")
