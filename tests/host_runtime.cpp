@@ -11,7 +11,8 @@
 // A read of a case's control block says that the march ended after hr_steps
 // (three) steps.  hr_block(size): the live allocation of that size.  hr_sms(n): the
 // device has n SMs.  hr_blocks_of(kernel): the blocks of the largest launch
-// of a kernel whose mangled name has this text.
+// of a kernel whose mangled name has this text.  hr_sweep_bufs(): the tile buffers
+// of the last sweep launched.
 #include <cuda.h>
 #include <cuda_runtime_api.h>
 
@@ -34,7 +35,7 @@ struct Block {
 std::map<uintptr_t, Block> blocks;
 size_t limit_bytes = 0;
 long fail_at = -1;
-int march_steps = 3, sms = 148, bad = 0;
+int march_steps = 3, sms = 148, sweep_bufs = 0, bad = 0;
 std::string last_bad;
 // (a function's static: the objects register their kernels before this file's are made)
 std::map<const void*, std::string>& kernels() {
@@ -94,7 +95,9 @@ cudaError_t launch(const void* fn, dim3 grid, void** args) {
     l.table = *(const uintptr_t*)args[0];
     l.what = "the sweep's case";
     const auto it = find(l.table);
-    const int ncases = ((const int*)args[0])[10];  // after the table, three offsets and the control block
+    const int* ints = (const int*)args[0] + 10;  // after the table, three offsets and the control block
+    const int ncases = ints[0];
+    sweep_bufs = ints[2];  // after the widest halo
     if (it != blocks.end() && ncases == 1)
       l.words.assign((const uintptr_t*)args[2], (const uintptr_t*)args[2] + it->second.size / 8);
   } else if (name.find("k_out_") != std::string::npos) {
@@ -131,6 +134,7 @@ void hr_limit(size_t n) { limit_bytes = n; }
 void hr_fail_at(long k) { fail_at = k; }
 void hr_steps(int n) { march_steps = n; }
 void hr_sms(int n) { sms = n; }
+int hr_sweep_bufs() { return sweep_bufs; }
 unsigned hr_blocks_of(const char* kernel) {
   for (const auto& g : grids)
     if (g.first.find(kernel) != std::string::npos) return g.second;

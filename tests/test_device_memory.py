@@ -223,3 +223,21 @@ s.advance(1)
 blocks = hr.hr_blocks_of(b"k_wspec")
 assert 32 <= blocks <= 4 * {sms} and (blocks == 32) == ({sms} == 8), blocks
 """)
+
+
+@pytest.mark.parametrize("prec", [64, 32])
+@pytest.mark.parametrize("k,asked,tile,bufs", [(6, 64, 64, 2), (24, 64, 64, 2), (64, 64, 64, 1), (6, 128, 128, 2),
+                                               (24, 128, 128, 1), (64, 128, 64, 1)])
+def test_wide_halos_take_the_paths_they_are_run_for(run, k, asked, tile, bufs, prec):
+    # the meshes of test_gpu_sweep_tiles.py::test_wide_halos: a 64-element tile
+    # has two buffers up to a halo of 160 (162 in FP32), a 128-element one up to
+    # 86 (88) and one up to 232 (235); past that 64 elements are taken
+    run(f"""
+sys.path[:0] = [{os.path.join(ROOT, "tests")!r}, {os.path.join(ROOT, "oracle")!r}]
+from test_gpu_sweep_tiles import sheets
+s = Solver.from_case(sheets(cavity_case(6, 4, 9, mach=0.3, kn=0.1), {k}), precision={prec}, tile_elems={asked})
+s.init_case()
+s.advance(1)
+i = s.info()
+assert (i["tile_elems"], hr.hr_sweep_bufs()) == ({tile}, {bufs}), (i, hr.hr_sweep_bufs())
+""")
