@@ -278,8 +278,9 @@ def large_leg(device, steps=10, warmup=3):
     achieved bandwidth at FP32 and FP64 (the time to steady state of this
     workload is recorded by dgbgk.steady, not here)."""
     from dgbgk import Solver, config5
+    from dgbgk.profile import step_parts
     case = config5()
-    names = ["k_moments", "k_wall", "k_sweep", "k_resid"]
+    names = step_parts(case)
     peak, _ = peaks()
     out = {"workload": workload(case, 32).replace(", f in FP32", ""), "dofs": case.dofs}
     for prec in (32, 64):
@@ -335,6 +336,7 @@ def run_ours(a, d):
     import numpy as np
     import torch
     from dgbgk import Solver
+    from dgbgk.profile import step_parts
 
     torch.cuda.set_device(d.local)
     case = make_case(a.config)
@@ -356,7 +358,7 @@ def run_ours(a, d):
 
     # dominant kernel, timed live with CUDA events on the library's stream
     kms = s.profile(5)
-    names = ["k_moments", "k_wall", "k_sweep", "k_resid"]
+    names = step_parts(case)
     sf = 4 if a.precision == 32 else 8
     alg_bytes = 2 * sf * case.dofs  # one read + one write of f per DOF-update
     peak, peak_src = peaks()

@@ -210,7 +210,8 @@ class Solver:
         return t.value
 
     def profile(self, nsteps):
-        """Mean device ms per step of [moments, wall, sweep, residual]."""
+        """Mean device ms per step of [moments, wall, sweep, what follows it]
+        (named by dgbgk.profile.step_parts)."""
         ms = np.zeros(4)
         check(lib().dgbgk_profile_steps(self.h, nsteps, ptr(ms)))
         return ms

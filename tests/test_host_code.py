@@ -1,6 +1,7 @@
-"""The library's host code where device memory runs short or sizes are extreme,
-against a CUDA runtime in host memory (tests/host_runtime.cpp; CPU): kernels do
-nothing there, and a launch that is given a freed address is counted."""
+"""The library's host code without a GPU, against a CUDA runtime in host memory
+(tests/host_runtime.cpp; CPU): where device memory runs short, where sizes are
+extreme, and which launches a call makes.  Kernels do nothing there; a launch that
+is given a freed address is counted."""
 import os
 import subprocess
 import sys
@@ -240,4 +241,22 @@ s.init_case()
 s.advance(1)
 i = s.info()
 assert (i["tile_elems"], hr.hr_sweep_bufs()) == ({tile}, {bufs}), (i, hr.hr_sweep_bufs())
+""")
+
+
+@pytest.mark.parametrize("alpha", [1.0, 0.9])
+@pytest.mark.parametrize("walls", [True, False])
+def test_the_profile_names_the_launches_there_are(run, alpha, walls):
+    run(f"""
+from dgbgk import channel_case
+from dgbgk.profile import step_parts
+c = channel_case(-2.0, 4.0, -2.0, 2.0, 12, 8, 8, 8, mach=2.0, kn=0.05)
+c.alpha = {alpha}
+if not {walls}:
+    c.mesh.bsido[c.mesh.bsido[:, 3] == 4, 3] = 2
+s = Solver.from_case(c)
+s.init_case()
+s.profile(1)
+assert step_parts(c)[:3] == ["k_moments", "k_wall", "k_sweep"]
+assert step_parts(c)[3] == ("k_resid" if hr.hr_blocks_of(b"7k_resid") else "gap")
 """)
