@@ -245,8 +245,8 @@ inline int tiles_per_unit_alone(long total_tiles, int grid, int nvt) {
 // Uploads the case table and picks the launch shapes.  Moments: per-warp
 // rings of R-row stages; picks (R, warps per CTA, ring stages) with the most
 // resident warps per SM (shared memory and registers), then the most rows in
-// flight, then the fewest rows per warp step (FP32 takes the element mode
-// first, below).  Measured on B200 at 24x48 velocities, one row per warp
+// flight, then the fewest rows per warp step (the element mode first while
+// eight warps of it fit, below).  Measured on B200 at 24x48 velocities, one row per warp
 // step against two or four: warps count for more than stages (FP64: 20 warps
 // with one-stage rings 0.344 ms, 16 with one 0.372, 10 with two 0.486; FP32:
 // 20 with one 0.204, 16 with two 0.207).

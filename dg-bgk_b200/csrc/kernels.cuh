@@ -877,11 +877,6 @@ __device__ __forceinline__ double2 pfma(double2 a, double2 b, double2 c) {
   return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
 }
 __device__ __forceinline__ double2 pdup(double a) { return make_double2(a, a); }
-template <class P> __device__ __forceinline__ P pneg(P a) {
-  a.x = -a.x;
-  a.y = -a.y;
-  return a;
-}
 // a - b; FP32 as one packed fma(b, -1, a), the same rounding (negating a
 // packed operand takes two instructions)
 __device__ __forceinline__ float2 psub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
@@ -983,9 +978,6 @@ __device__ __forceinline__ float fmax_nan(float a, float b) {
   float r;
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
-}
-__device__ __forceinline__ double fmax_nan(double a, double b) {
-  return (a != a || b != b) ? a + b : fmax(a, b);
 }
 
 // Adds the per-warp residual partials (max |d|, sum of squares) to a case's

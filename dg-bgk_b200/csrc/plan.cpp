@@ -300,7 +300,6 @@ int build_plan(const dgbgk_mesh& m, const dgbgk_vspace& vs, const dgbgk_params& 
       g.gx[k] = G[k];
       g.gy[k] = G[k + 3];
     }
-    g.area = 0.5 * G[6];
     g.inflow = 0;
     for (int k = 0; k < 3; ++k) {
       if (inflow_pt[m.intma[3 * eo + k]]) g.inflow |= 1 << k;

@@ -9,11 +9,12 @@
 
 namespace dgbgk {
 
-// Element edge before blocking: the device record ElemEdge<T> packs `low`
-// with the neighbour's tile slot (interior) or `bside` (boundary) into info.
+// Element edge before blocking.  The device record (ElemRec) takes its normal
+// times its length, the tile rows of the flux source that edge_info gives for
+// a blocking, and a wall's boundary side.
 struct PlanEdge {
   double nx = 0, ny = 0, alen = 0;
-  int low = -1;   // info bits [0,7): kind, left flag, neighbour local nodes
+  int low = -1;   // bits [0,7) of edge_info: kind, left flag, neighbour local nodes
   int nbr = -1;   // neighbour element (plan order) or -1
   int bside = -1; // boundary side index or -1
 };
@@ -21,7 +22,6 @@ struct PlanEdge {
 // Velocity-independent data of one element (FP64 master copy).
 struct PlanGeo {
   double gx[3] = {0, 0, 0}, gy[3] = {0, 0, 0};  // GEOME(1:3), GEOME(4:6)
-  double area = 0;                              // 0.5 * GEOME(7)
   double mm[3] = {0, 0, 0};  // MMAT (IMMAT = 1) or CMMAT row sums (IMMAT = 0)
   int inflow = 0;            // bit i: DG node i sits on an inflow-side node
 };
@@ -51,7 +51,7 @@ struct Plan {
   // nodal gather (MACROS tail / GETMAC): CSR over mesh nodes
   std::vector<int> node_off, node_dg;  // DG node index (plan order) per entry
   std::vector<double> node_ae;         // GEOME(7) of its element
-  // Wall accommodation ALPHA < 1 (IMMAT = 1): the specular part of GETBOU.
+  // Wall accommodation ALPHA < 1: the specular part of GETBOU.
   // A molecule leaving a wall side at velocity v (TEST < 0) carries
   // (1-ALPHA) times the element's own f at the mirrored velocity, read as
   // the two grid velocities I1, I2 around it and interpolated with ZD1, ZD2
@@ -72,10 +72,10 @@ struct Plan {
   std::vector<int> spec_seq;      // sequential items, per slot by level: (item, where its level ends) pairs
 };
 
-// Device edge word of edge i = 3*e + k (ElemEdge::info): the kind, the
-// flux source's local nodes and its tile slot -- the neighbour across an
-// interior side, the element itself (slot own_slot, nodes k and k+1) on a
-// boundary side.
+// Edge i = 3*e + k under the present blocking: the kind (bits 0, 1), the flux
+// source's local nodes (bits 3, 4 and 5, 6) and its tile slot (from bit 8) --
+// the neighbour across an interior side, the element itself (slot own_slot,
+// nodes k and k+1) on a boundary side.
 inline int edge_info(const Plan& pl, size_t i, int own_slot) {
   const PlanEdge& e = pl.edge[i];
   const int kind = e.low & 3;

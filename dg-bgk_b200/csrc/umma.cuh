@@ -4,11 +4,11 @@
 // tensor memory.
 //
 // One CTA computes one 128 x BN tile of C with 128 threads:
-//   * warp 0, lane 0 loads 128 x 64 (A) and BN x 64 (B) BF16 boxes per
-//     K-block with TMA (128-byte swizzle) into a ring of stages;
-//   * warp 1, lane 0 issues tcgen05.mma (kind::f16, M = 128, N = BN, K = 16
-//     per instruction, four per K-block) and frees each stage with
-//     tcgen05.commit on the stage's "empty" mbarrier;
+//   * an elected thread of warp 0 loads 128 x 64 (A) and BN x 64 (B) BF16
+//     boxes per K-block with TMA (128-byte swizzle) into a ring of stages;
+//   * an elected thread of warp 1 issues tcgen05.mma (kind::f16, M = 128,
+//     N = BN, K = 16 per instruction, four per K-block) and frees each stage
+//     with tcgen05.commit on the stage's "empty" mbarrier;
 //   * all four warps read the accumulator with tcgen05.ld (warp w owns TMEM
 //     lanes 32w..32w+31, i.e. rows 32w..32w+31 of the tile) and run the
 //     epilogue.
