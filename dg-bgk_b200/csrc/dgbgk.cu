@@ -661,7 +661,8 @@ template <class T> struct Impl : ImplBase {
   // (one of 16).  FP64: 128, except where that leaves SMs without a tile:
   // 8x8 cavity at 16x16 velocities (16 tiles) 16.1 us with 128, 14.5 with 64;
   // 32x32 at 16x32 (512 tiles) 33.4 against 35.8; the channel 0.743 against
-  // 0.741.
+  // 0.741.  In between it is not always the faster one: 64x64 at 16x32 (2048
+  // tiles), a step of 131 us with 128 and 123 with 64.
   static int default_eb(long nelem, long nvel, int nsm) {
     if (sizeof(T) == 4) return 64;
     const long tiles = (nelem + 127) / 128 * ((nvel + SweepGeo<T>::VT - 1) / SweepGeo<T>::VT);

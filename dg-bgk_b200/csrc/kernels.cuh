@@ -1037,7 +1037,10 @@ __device__ __forceinline__ void resid_add(Ctrl* ctrl, const double* red_m, const
 // registers (0.840), coefficients duplicated in registers (0.387), f loaded
 // straight into registers at the start of phase 1 (0.387), one tile buffer
 // and three CTAs at 80 registers (FP32 0.358), the wall records staged in
-// shared memory (FP32 0.295, FP64 0.788: it spills).
+// shared memory (FP32 0.295, FP64 0.788).  At 128 registers FP32 with IMMAT =
+// 1 does not spill; the others do (bytes of stores per thread, a single case /
+// a batch: FP64 76 to 80 / 124, FP64 with IMMAT = 0 112 / 120, FP32 with
+// IMMAT = 0, which reads the residual tables in the update, 168 / 84).
 template <class T, int EB, int IMMAT, bool ONE>
 __global__ void __launch_bounds__(SweepGeo<T>::threads(EB), SweepGeo<T>::min_ctas(EB))
     k_sweep(BatchArgs<T> a, int total_units, const __grid_constant__ CaseDev<T> one) {
