@@ -174,7 +174,8 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, 
   return copy(d, s, n, k);
 }
 cudaError_t cudaMemcpy2D(void* d, size_t dp, const void* s, size_t sp, size_t w, size_t h, cudaMemcpyKind k) {
-  if (dp > 0x7fffffff || sp > 0x7fffffff) return cudaErrorInvalidPitchValue;  // cudaDeviceProp::memPitch
+  // cudaDeviceProp::memPitch, the range stated (a driver may let larger ones through)
+  if (dp > 0x7fffffff || sp > 0x7fffffff) return cudaErrorInvalidPitchValue;
   for (size_t i = 0; i < h; ++i)
     if (const cudaError_t e = copy((char*)d + i * dp, (const char*)s + i * sp, w, k)) return e;
   return cudaSuccess;

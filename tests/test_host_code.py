@@ -131,7 +131,8 @@ assert m.train(40).size == 40
 
 
 def test_histories_of_a_call_with_a_very_large_step_limit(run):
-    # rows of 8 B a step would be further apart than a 2-D copy's pitch may be
+    # rows of 8 B a step would be further apart than the largest pitch that the
+    # device states for a 2-D copy
     run("""
 s = solver()
 r = s.advance(2 ** 28 + 1, tol=0.5)
